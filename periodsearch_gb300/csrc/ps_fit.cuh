@@ -215,22 +215,6 @@ __device__ inline T warp_sum(T v)
     return v;
 }
 
-// Sum over the block; every thread gets the result.  red holds >= NT/32 doubles.
-template <int NT>
-__device__ inline double block_sum(double v, double *red)
-{
-    v = warp_sum(v);
-    int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    double t = 0;
-#pragma unroll
-    for (int i = 0; i < NT / 32; i++) t += red[i];
-    __syncthreads();
-    return t;
-}
-
 // Asynchronous global -> shared copies (cp.async, 8 or 16 bytes, both
 // addresses aligned to the size), completed by cp_async_wait_all of the
 // issuing thread.
@@ -361,22 +345,12 @@ __device__ inline void warp_sum9(const double (&v)[9], double *out, int lane)
     out[iz] = z + __shfl_xor_sync(0xffffffffu, z, 1);
 }
 
-// FP64 facet stage of point p of the tile (bright.c:59-120), one warp.  A
-// first pass lists the point's lit facets in increasing order (s.lidx,
-// s.nlit); the law and the facet sums then run over that list with every
-// lane busy (an FP64 instruction holds its sub-partition's FP64 unit for
-// the whole warp, however few lanes are active), lane l taking the list's
-// entries l, l + 32, ...  W is left in the W row at the list positions.
-// The facet sums go to s.red[p * kRedStride + 0..5]: brightness, the three
-// rotation derivatives, the Lambert and the scattering-weight derivatives.
-__device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> &s, int p, int wcols, double cl,
-                                        double cls)
+// Lists the lit facets of a point with Earth and Sun directions e, f in
+// increasing order into idx (one warp); returns their count.
+__device__ inline int list_lit_fp64(const DevObject &ob, double e1, double e2, double e3, double f1, double f2,
+                                    double f3, uint16_t *idx)
 {
     const int lane = threadIdx.x & 31, F = ob.nfac;
-    const double *pt = s.pt + p * kPointStride;
-    const double e1 = pt[0], e2 = pt[1], e3 = pt[2];
-    const double f1 = pt[3], f2 = pt[4], f3 = pt[5];
-    uint16_t *idx = s.lidx + static_cast<size_t>(p) * wcols;
     // The lit test in FP32 where it is decided beyond its rounding: the FP32
     // dot products of the FP32-rounded unit vectors are within ~4e-7 of the
     // FP64 ones, so outside a 1e-4 band (scaled by the direction's 1-norm)
@@ -408,6 +382,27 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
         n += __popc(m);
     }
     __syncwarp();
+    return n;
+}
+
+// FP64 facet stage of point p of the tile (bright.c:59-120), one warp.  A
+// first pass lists the point's lit facets in increasing order (s.lidx,
+// s.nlit); the law and the facet sums then run over that list with every
+// lane busy (an FP64 instruction holds its sub-partition's FP64 unit for
+// the whole warp, however few lanes are active), lane l taking the list's
+// entries l, l + 32, ...  W is left in the W row at the list positions.
+// The facet sums go to s.red[p * kRedStride + 0..5]: brightness, the three
+// rotation derivatives, the Lambert and the scattering-weight derivatives.
+// count: add the point's lit facets to the CTA's counter.
+__device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> &s, int p, int wcols, double cl,
+                                        double cls, bool count)
+{
+    const int lane = threadIdx.x & 31;
+    const double *pt = s.pt + p * kPointStride;
+    const double e1 = pt[0], e2 = pt[1], e3 = pt[2];
+    const double f1 = pt[3], f2 = pt[4], f3 = pt[5];
+    uint16_t *idx = s.lidx + static_cast<size_t>(p) * wcols;
+    const int n = list_lit_fp64(ob, e1, e2, e3, f1, f2, f3, idx);
     // The rotation derivatives sum_i Area_i (dsmu_i (n_i . D_k) + dsmu0_i
     // (n_i . E_k)) (bright.c:87-104; D_k, E_k: the derivative directions of
     // the Earth and Sun vectors) are D_k . U + E_k . V with U = sum Area
@@ -452,7 +447,7 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
         rd[4] = sums[7];
         rd[5] = sums[8];
         s.nlit[p] = n;
-        atomicAdd(lit_counter(s.misc), static_cast<unsigned long long>(n));
+        if (count) atomicAdd(lit_counter(s.misc), static_cast<unsigned long long>(n));
     }
 }
 
@@ -706,9 +701,10 @@ __device__ inline void setup_mixed_geo(float4 g0, float4 g1, const float *bm, fl
         const float php0 = bm[27], php1 = bm[28], php2 = bm[29];
         const float inv_w = 1.f / php1;
         const float ex = expf(-alpha * inv_w);
-        pt[24] = 1 + php0 * ex + php2 * alpha;
+        const float pe = __fmul_rn(php0, ex);
+        pt[24] = fmaf(php2, alpha, __fadd_rn(1.f, pe));   // one rounding wherever it is formed
         pt[25] = ex;
-        pt[26] = php0 * ex * alpha * (inv_w * inv_w);
+        pt[26] = pe * alpha * (inv_w * inv_w);
         pt[27] = alpha;
     }
     if (part != 0) pt[30] = g1.w;
@@ -761,6 +757,12 @@ __device__ inline void setup_mixed_rotate(float *pt)
     }
 }
 
+// 1 + a exp(-alpha / d) + k alpha (phasec.c), one rounding wherever it is formed.
+__device__ inline double phase_scale_fp64(double a, double k, double ex, double alpha)
+{
+    return fma(k, alpha, __dadd_rn(1.0, __dmul_rn(a, ex)));
+}
+
 // Point set-up of observation q (bright.c:27-57, phasec.c, matrix.c): the
 // rotated Earth and Sun directions with their beta/lambda/omega derivatives,
 // the phase function and its derivatives, into pt[0..27].
@@ -799,15 +801,16 @@ __device__ inline void setup_point(const DevObject &ob, const FitConfig &cfg, in
     }
     const double td = ob.tim[q];
     const R t = R(td);
-    R ex;
+    R ex, scale;
     R inv_w = 0;
     if constexpr (kFP64) {
         ex = exp(-alpha / php1);
+        scale = phase_scale_fp64(php0, php2, ex, alpha);
     } else {
         inv_w = 1.f / php1;
         ex = expf(-alpha * inv_w);
+        scale = 1 + php0 * ex + php2 * alpha;
     }
-    const R scale = 1 + php0 * ex + php2 * alpha;
     const double f = rotation_phase_fp64(omg, td, cfg.phi0);
     const R cf = cos(f), sf = sin(f);
     const R fm[9] = {cf, sf, R(0), -sf, cf, R(0), R(0), R(0), R(1)};
@@ -861,6 +864,34 @@ __device__ inline void setup_point(const DevObject &ob, const FitConfig &cfg, in
     if constexpr (kFP64) pt[26] = php0 * ex * alpha / (php1 * php1);
     else pt[26] = php0 * ex * alpha * (inv_w * inv_w);
     pt[27] = alpha;
+}
+
+// The part of the FP64 form's set-up that the model value needs: the rotated
+// Earth and Sun directions into e[0..5] and the phase function (returned),
+// by setup_point's operations.
+__device__ inline double setup_point_light(const DevObject &ob, const FitConfig &cfg, int q, double omg,
+                                           const double *bm, double (&e)[6])
+{
+    const double ee[3] = {ob.eex[q], ob.eey[q], ob.eez[q]}, e0v[3] = {ob.e0x[q], ob.e0y[q], ob.e0z[q]};
+    const double alpha = ob.alpha_pt[q];
+    const double f = rotation_phase_fp64(omg, ob.tim[q], cfg.phi0);
+    const double cf = cos(f), sf = sin(f);
+    const double fm[9] = {cf, sf, 0.0, -sf, cf, 0.0, 0.0, 0.0, 1.0};
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        double x = 0, y = 0;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            double m = 0;
+#pragma unroll
+            for (int k = 0; k < 3; k++) m = m + fm[i * 3 + k] * bm[k * 3 + j];
+            x = x + m * ee[j];
+            y = y + m * e0v[j];
+        }
+        e[i] = x;
+        e[3 + i] = y;
+    }
+    return phase_scale_fp64(bm[27], bm[29], exp(-alpha / bm[28]), alpha);
 }
 
 // ---------------------------------------------------------------------------
@@ -1089,6 +1120,55 @@ __device__ void contract_tc_issue(Smem<PS_FORM_MIXED> &s, int F, TcState &t)
     }
 }
 
+// Earth and Sun directions of a point record (setup_mixed_phase,
+// setup_mixed_geo) rotated about the spin axis.
+__device__ inline void rotate_directions(const float *pt, float (&e)[6])
+{
+    const float cf = pt[28], sf = pt[29];
+    e[0] = cf * pt[0] + sf * pt[1];
+    e[1] = cf * pt[1] - sf * pt[0];
+    e[2] = pt[2];
+    e[3] = cf * pt[3] + sf * pt[4];
+    e[4] = cf * pt[4] - sf * pt[3];
+    e[5] = pt[5];
+}
+
+// The Lommel-Seeliger + Lambert law on a pair of facets (fac_at's two float4
+// of the pair) as FP32x2 operations, one paired instruction each.
+// Branch-free: the 8 points of a warp see different lit facets, so a branch
+// would diverge on almost every step (and a warp-uniform skip of groups
+// unlit for all 8 points measured slower, twice); unlit and padding facets
+// get zero area (every term vanishes) and a safe denominator.
+struct LitPair {
+    float2 ax, m, m0, r, mm;   // area (0 when unlit), mu, mu0, 1 / (mu + mu0), mu mu0
+    __device__ inline LitPair(const float4 &fa, const float4 &fb, const float2 &E1, const float2 &E2, const float2 &E3,
+                              const float2 &F1, const float2 &F2, const float2 &F3)
+    {
+        const float2 nx = make_float2(fa.x, fa.y), ny = make_float2(fa.z, fa.w), nz = make_float2(fb.x, fb.y);
+        float2 mu = __fmul2_rn(E1, nx), mu0 = __fmul2_rn(F1, nx);
+        mu = __ffma2_rn(E2, ny, mu);
+        mu0 = __ffma2_rn(F2, ny, mu0);
+        mu = __ffma2_rn(E3, nz, mu);
+        mu0 = __ffma2_rn(F3, nz, mu0);
+        const bool lit0 = mu.x > float(kTinyMu) && mu0.x > float(kTinyMu);
+        const bool lit1 = mu.y > float(kTinyMu) && mu0.y > float(kTinyMu);
+        // Area (= Darea g, also the weight of W: the Lambert and
+        // Lommel-Seeliger terms share it)
+        ax = make_float2(lit0 ? fb.z : 0.f, lit1 ? fb.w : 0.f);
+        m = make_float2(lit0 ? mu.x : 1.f, lit1 ? mu.y : 1.f);
+        m0 = make_float2(lit0 ? mu0.x : 1.f, lit1 ? mu0.y : 1.f);
+        const float2 dnom = __fadd2_rn(m, m0);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(dnom.x));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(dnom.y));
+        mm = __fmul2_rn(m, m0);
+    }
+    // s = mu mu0 (cl + cls / (mu + mu0))
+    __device__ inline float2 law(const float2 &CL, const float2 &CLS) const
+    {
+        return __fmul2_rn(mm, __ffma2_rn(CLS, r, CL));
+    }
+};
+
 // Facet stage of the tensor-core path (bright.c:59-120).  Warp w takes
 // points 8 (w % 4) .. +7 (lane / 4) and the facet quarter w / 4, each lane
 // of a point taking two adjacent facets of every 8 (lane % 4), so that one
@@ -1112,14 +1192,14 @@ __device__ void facet_stage_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int 
     // (setup_mixed_phase): Earth and Sun directions rotated here.
     float e1 = 0, e2 = 0, e3 = 0, f1 = 0, f2 = 0, f3 = 0;
     if (p < np) {
-        const float *pt = s.pt + p * kPointStride;
-        const float cf = pt[28], sf = pt[29];
-        e1 = cf * pt[0] + sf * pt[1];
-        e2 = cf * pt[1] - sf * pt[0];
-        e3 = pt[2];
-        f1 = cf * pt[3] + sf * pt[4];
-        f2 = cf * pt[4] - sf * pt[3];
-        f3 = pt[5];
+        float e[6];
+        rotate_directions(s.pt + p * kPointStride, e);
+        e1 = e[0];
+        e2 = e[1];
+        e3 = e[2];
+        f1 = e[3];
+        f2 = e[4];
+        f3 = e[5];
     }
     // The rotation derivatives sum_i Area_i (dsmu (n_i . D_k) + dsmu0 (n_i .
     // E_k)) over the lit facets are D_k . U + E_k . V with U = sum Area dsmu
@@ -1139,30 +1219,10 @@ __device__ void facet_stage_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int 
         const int cm = g * kcs + kc;    // core matrix (8-point group, 8-facet group)
         const float4 fa = s.fac[i], fb = s.fac[i + 1];
         const float2 nx = make_float2(fa.x, fa.y), ny = make_float2(fa.z, fa.w), nz = make_float2(fb.x, fb.y);
-        float2 mu = __fmul2_rn(E1, nx), mu0 = __fmul2_rn(F1, nx);
-        mu = __ffma2_rn(E2, ny, mu);
-        mu0 = __ffma2_rn(F2, ny, mu0);
-        mu = __ffma2_rn(E3, nz, mu);
-        mu0 = __ffma2_rn(F3, nz, mu0);
-        // Branch-free: the 8 points of a warp see different lit facets,
-        // so a branch would diverge on almost every step (and a
-        // warp-uniform skip of groups unlit for all 8 points measured
-        // slower, twice); unlit and padding facets get zero area (every
-        // term vanishes) and a safe denominator.
-        const bool lit0 = mu.x > float(kTinyMu) && mu0.x > float(kTinyMu);
-        const bool lit1 = mu.y > float(kTinyMu) && mu0.y > float(kTinyMu);
-        // Area (= Darea g, also the weight of W: the Lambert and
-        // Lommel-Seeliger terms share it)
-        const float2 ax = make_float2(lit0 ? fb.z : 0.f, lit1 ? fb.w : 0.f);
-        const float2 m = make_float2(lit0 ? mu.x : 1.f, lit1 ? mu.y : 1.f);
-        const float2 m0 = make_float2(lit0 ? mu0.x : 1.f, lit1 ? mu0.y : 1.f);
-        // LitTerms<float, PS_FORM_MIXED> on both halves
-        const float2 dnom = __fadd2_rn(m, m0);
-        float2 r;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(dnom.x));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(dnom.y));
-        const float2 mm = __fmul2_rn(m, m0);
-        const float2 sv = __fmul2_rn(mm, __ffma2_rn(CLS, r, CL));
+        // (unlit facets carry zero area: no branch, see LitPair)
+        const LitPair lp(fa, fb, E1, E2, E3, F1, F2, F3);
+        const float2 ax = lp.ax, m = lp.m, m0 = lp.m0, r = lp.r, mm = lp.mm;
+        const float2 sv = lp.law(CL, CLS);
         const float2 q0 = __fmul2_rn(m0, r), q1 = __fmul2_rn(m, r);
         const float2 dsmu = __ffma2_rn(CLS, __fmul2_rn(q0, q0), __fmul2_rn(CL, m0));
         const float2 dsmu0 = __ffma2_rn(CLS, __fmul2_rn(q1, q1), __fmul2_rn(CL, m));
@@ -1459,45 +1519,32 @@ __device__ void tc_alpha_flush(const DevObject &ob, Smem<PS_FORM_MIXED> &s, doub
     __syncthreads();
 }
 
-// ---------------------------------------------------------------------------
-// Model evaluation (mrqcof) at parameters a[] into matrix M (mfit x mfit,
-// lower triangle accumulated then mirrored) and vector bv.  Leaves chi^2,
-// the facet-area sum and the convexity residuals in misc.
-// ---------------------------------------------------------------------------
+// The parts of an evaluation at parameters a[] that do not depend on the
+// points: facet areas (s.area, s.gv), their sum, the rotation matrices and
+// the phase and scattering parameters (s.bmat), the scale of the tensor-core
+// operand; clears chi^2.  Ends with a barrier.
 template <int FORM, int KU>
-__device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<FORM> &s,
-                         const double *a, double *M, double *bv, typename RealOf<FORM>::T *scratch, TcState &tcs)
+__device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double *a)
 {
     using R = typename RealOf<FORM>::T;
     constexpr bool kFP64 = FORM == PS_FORM_FP64;
-    // tensor-core path: the point set-up of the next tile runs on warps 1..15
-    // while thread 0 issues the current tile's MMAs
     constexpr bool kPipe = !kFP64 && (KU == 0 || KU == 3);
-    // alpha/beta on the tensor cores (KU 0), or on the SIMT pipes behind the
-    // wide tensor-core contraction (KU 3: 65..96 coefficients)
-    constexpr bool kTcAlpha = !kFP64 && KU == 0;
-    constexpr bool kWide = !kFP64 && KU == 3;
     constexpr int NT = threads_of<FORM>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int F = ob.nfac, C = ob.ncoef, ma = ob.ma, mf = ob.mfit, P = L.P;
-    const int wcols = L.wcols;
-    const int RW = rel_row_stride(ma);   // parked row of a relative lightcurve
-    const R *nxR, *nyR, *nzR, *dareaR;
-    const R *dsphR;
-    if constexpr (kFP64) {
-        nxR = ob.nx;
-        nyR = ob.ny;
-        nzR = ob.nz;
-        dareaR = ob.darea;
-        dsphR = ob.dsph;
-    } else {
-        nxR = ob.nx_f;
-        nyR = ob.ny_f;
-        nzR = ob.nz_f;
-        dareaR = ob.darea_f;
-        dsphR = ob.dsph_f;
+    const int F = ob.nfac, C = ob.ncoef, ma = ob.ma;
+    // The scalars' exp, cos and sin on the last warp (the pole angles on two
+    // lanes at once), which has no facets on the usual grids, while the
+    // other warps compute the curvature.
+    if (warp == NT / 32 - 1) {
+        if (lane < 2) {
+            const double x = a[C + lane];
+            s.misc[M_TRIG + 2 * lane] = cos(x);
+            s.misc[M_TRIG + 2 * lane + 1] = sin(x);
+        } else if (lane == 2) {
+            s.misc[M_CL] = exp(a[ma - 2]);
+            s.misc[M_CHISQ] = 0;
+        }
     }
-
     // curv.c:10-39 -- g_i = exp(sum over (m,l) of P_l^m (c cos + c' sin)), FP64.
     double asum = 0;
     for (int i = tid; i < F; i += NT) {
@@ -1530,25 +1577,19 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
         }
         asum += ar;
     }
-    double tot = block_sum<NT>(asum, s.misc + M_RED);
-    if (tid == 0) {
-        s.misc[M_AREA] = tot;
-        s.misc[M_CHISQ] = 0;
-        s.misc[M_CL] = exp(a[ma - 2]);
-        s.misc[M_TRIG] = cos(a[C]);
-        s.misc[M_TRIG + 1] = sin(a[C]);
-        s.misc[M_TRIG + 2] = cos(a[C + 1]);
-        s.misc[M_TRIG + 3] = sin(a[C + 1]);
-    }
-    for (int e = tid; e < mf * mf; e += NT) M[e] = 0;
-    for (int j = tid; j < mf; j += NT) bv[j] = 0;
-
-    // blmatrix.c:9-46 in FP64 from the angles' cos/sin of thread 0, one
-    // entry per lane of warp 0 (every FP64 instruction holds the FP64 unit
-    // for the whole warp, so each scalar is computed once), stored in the
-    // facet-stage type with the phase and scattering parameters.
+    asum = warp_sum(asum);
+    if (lane == 0) s.misc[M_RED + warp] = asum;
     __syncthreads();
-    if (warp == 0) {
+    // Every scalar once, on a warp of its own (an FP64 instruction holds the
+    // FP64 unit for the whole warp): the area sum, blmatrix.c:9-46 in FP64
+    // from the angles' cos/sin, one entry per lane, stored in the
+    // facet-stage type with the phase and scattering parameters.
+    if (tid == 0) {
+        double t = 0;
+#pragma unroll
+        for (int i = 0; i < NT / 32; i++) t += s.misc[M_RED + i];
+        s.misc[M_AREA] = t;
+    } else if (warp == 2) {
         R v;
         if (lane < 27) {
             const int code = c_bl_code[lane];
@@ -1574,6 +1615,55 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
             mx * fmaxf(1.f, fabsf(static_cast<float>(s.misc[M_CL])) + 0.5f * fabsf(static_cast<float>(a[C + 7])));
         if (lane == 0) s.misc[M_WEXP] = (wmax > 0.f && wmax < 1e30f) ? static_cast<double>(13 - ilogbf(wmax)) : 0.0;
     }
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// Model evaluation (mrqcof) at parameters a[] into matrix M (mfit x mfit,
+// lower triangle accumulated then mirrored) and vector bv.  Leaves chi^2,
+// the facet-area sum and the convexity residuals in misc.  fresh = false:
+// shape_prologue has run at the same parameters already (the chi^2 of an
+// accepted step), and the FP64 form's lit facets have been counted.
+// ---------------------------------------------------------------------------
+template <int FORM, int KU>
+__device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<FORM> &s,
+                         const double *a, double *M, double *bv, typename RealOf<FORM>::T *scratch, TcState &tcs,
+                         bool fresh = true)
+{
+    using R = typename RealOf<FORM>::T;
+    constexpr bool kFP64 = FORM == PS_FORM_FP64;
+    // tensor-core path: the point set-up of the next tile runs on warps 1..15
+    // while thread 0 issues the current tile's MMAs
+    constexpr bool kPipe = !kFP64 && (KU == 0 || KU == 3);
+    // alpha/beta on the tensor cores (KU 0), or on the SIMT pipes behind the
+    // wide tensor-core contraction (KU 3: 65..96 coefficients)
+    constexpr bool kTcAlpha = !kFP64 && KU == 0;
+    constexpr bool kWide = !kFP64 && KU == 3;
+    constexpr int NT = threads_of<FORM>();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int F = ob.nfac, C = ob.ncoef, ma = ob.ma, mf = ob.mfit, P = L.P;
+    const int wcols = L.wcols;
+    const int RW = rel_row_stride(ma);   // parked row of a relative lightcurve
+    const R *nxR, *nyR, *nzR, *dareaR;
+    const R *dsphR;
+    if constexpr (kFP64) {
+        nxR = ob.nx;
+        nyR = ob.ny;
+        nzR = ob.nz;
+        dareaR = ob.darea;
+        dsphR = ob.dsph;
+    } else {
+        nxR = ob.nx_f;
+        nyR = ob.ny_f;
+        nzR = ob.nz_f;
+        dareaR = ob.darea_f;
+        dsphR = ob.dsph_f;
+    }
+
+    if (fresh) shape_prologue<FORM, KU>(ob, s, a);
+    else if (tid == 0) s.misc[M_CHISQ] = 0;
+    for (int e = tid; e < mf * mf; e += NT) M[e] = 0;
+    for (int j = tid; j < mf; j += NT) bv[j] = 0;
     const double omg = a[C + 2];
     __syncthreads();
     const R cls = s.bmat[30], cl = s.bmat[31];
@@ -1665,7 +1755,7 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
                     facet_stage_tc<NT>(ob, s, np, cl, cls, wscale);
                 }
                 else if constexpr (kFP64) {
-                    for (int p = warp; p < np; p += NT / 32) facet_point_fp64(ob, s, p, wcols, cl, cls);
+                    for (int p = warp; p < np; p += NT / 32) facet_point_fp64(ob, s, p, wcols, cl, cls, fresh);
                 }
                 else
                 for (int p = warp; p < np; p += NT / 32) {
@@ -2044,7 +2134,7 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
 constexpr int kMaxSplit = 8;
 
 __device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<PS_FORM_FP64> &s,
-                               const double *a, double *M, double *bv, double *scratch)
+                               const double *a, double *M, double *bv, double *scratch, bool fresh)
 {
     namespace cgr = cooperative_groups;
     constexpr int NT = threads_of<PS_FORM_FP64>();
@@ -2056,48 +2146,10 @@ __device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const 
     const int RW = rel_row_stride(ma);
 
     // curv.c:10-39 and blmatrix.c:9-46 on every CTA (as in evaluate)
-    double asum = 0;
-    for (int i = tid; i < F; i += NT) {
-        double g = 0;
-        for (int q = 0; q < ob.npairs; q++) {
-            int m = ob.pair_m[q], n = ob.pair_n[q];
-            double fsum = a[n] * ob.fc[m * F + i];
-            if (m != 0) fsum = fsum + a[n + 1] * ob.fs[m * F + i];
-            g = g + ob.pleg[q * F + i] * fsum;
-        }
-        g = exp(g);
-        double ar = ob.darea[i] * g;
-        s.area[i] = ar;
-        s.gv[i] = g;
-        asum += ar;
-    }
-    double tot = block_sum<NT>(asum, s.misc + M_RED);
-    if (tid == 0) {
-        s.misc[M_AREA] = tot;
-        s.misc[M_CHISQ] = 0;
-        s.misc[M_CL] = exp(a[ma - 2]);
-        s.misc[M_TRIG] = cos(a[C]);
-        s.misc[M_TRIG + 1] = sin(a[C]);
-        s.misc[M_TRIG + 2] = cos(a[C + 1]);
-        s.misc[M_TRIG + 3] = sin(a[C + 1]);
-    }
+    if (fresh) shape_prologue<PS_FORM_FP64, 1>(ob, s, a);
+    else if (tid == 0) s.misc[M_CHISQ] = 0;
     for (int e = tid; e < mf * mf; e += NT) M[e] = 0;
     for (int j = tid; j < mf; j += NT) bv[j] = 0;
-    __syncthreads();
-    if (warp == 0) {
-        double v;
-        if (lane < 27) {
-            const int code = c_bl_code[lane];
-            const int fa = code & 3, fb = (code >> 2) & 3;
-            const double va = fa == 1 ? s.misc[M_TRIG] : fa == 2 ? s.misc[M_TRIG + 1] : fa == 3 ? 1.0 : 0.0;
-            const double vb = fb == 1 ? s.misc[M_TRIG + 2] : fb == 2 ? s.misc[M_TRIG + 3] : 1.0;
-            const double p = va * vb;
-            v = (code & 16) ? -p : p;
-        } else {
-            v = lane == 31 ? s.misc[M_CL] : a[lane == 30 ? C + 7 : C + 3 + (lane - 27)];
-        }
-        s.bmat[lane] = v;
-    }
     const double omg = a[C + 2];
     __syncthreads();
     const double cls = s.bmat[30], cl_w = s.bmat[31];
@@ -2114,7 +2166,7 @@ __device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const 
             if (sp >= 0 && sp < np)
                 setup_point<PS_FORM_FP64>(ob, cfg, start + t0 + sp, omg, s.bmat, s.pt + sp * kPointStride);
             __syncthreads();
-            for (int p = warp; p < np; p += NT / 32) facet_point_fp64(ob, s, p, wcols, cl_w, cls);
+            for (int p = warp; p < np; p += NT / 32) facet_point_fp64(ob, s, p, wcols, cl_w, cls, fresh);
         } else {
             for (int p = warp; p < np; p += NT / 32) {
                 const double *nc = (p == 0) ? ob.nx : (p == 1) ? ob.ny : ob.nz;
@@ -2288,6 +2340,405 @@ __device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const 
     for (int e = tid; e < mf * mf; e += NT) {
         const int j = e / mf, k = e - j * mf;
         if (k > j) M[e] = M[k * mf + j];
+    }
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// chi^2 alone at parameters a[], FP64 form: of mrqcof.c what decides whether
+// a step is accepted.  About half of an LM fit's steps are rejected, and a
+// rejected step's alpha and beta are never used, so run_fit takes the trial's
+// chi^2 from here and evaluates the derivatives of accepted steps only.
+//
+// Every value is formed by the operations of evaluate in their order: a
+// point's brightness by lane l over the entries l, l + 32, ... of its lit
+// list and the same butterfly, the relative lightcurves' sums and chi^2 over
+// the points in data order, so chi^2, the area sum and the convexity
+// residuals are evaluate's bit for bit.
+//
+// The points go through in chunks: set-up with a thread per point; a warp
+// per pair of points (taken from a counter, lit counts differ) for the
+// brightness; residuals.  No barrier inside a chunk's facet work.  The chain
+// of chi^2 additions over a chunk runs on the last warp during the next
+// chunk's facet work.  Buffers in the W region (unused here).  In a cluster
+// every CTA computes its share of the pairs, sends the model values to the
+// others and runs the sums itself.
+// ---------------------------------------------------------------------------
+struct Chi2Plan {
+    double *rec;      // [7][cap]: Earth and Sun directions, phase function
+    double *ym;       // [2][cap]: model values, then weighted squared residuals
+    uint16_t *idx;    // [warps][wcols]: lit lists
+    int cap;          // points
+};
+
+__device__ inline Chi2Plan chi2_plan(const SlotLayout &L, const Smem<PS_FORM_FP64> &s)
+{
+    constexpr int NW = threads_of<PS_FORM_FP64>() / 32;
+    Chi2Plan c;
+    const int lists = (NW * L.wcols * 2 + 15) & ~15;
+    c.cap = (static_cast<int>(L.J - L.W) - lists) / (9 * static_cast<int>(sizeof(double)));
+    c.rec = s.W;
+    c.ym = s.W + static_cast<size_t>(7) * c.cap;
+    c.idx = reinterpret_cast<uint16_t *>(s.W + static_cast<size_t>(9) * c.cap);
+    return c;
+}
+
+// A chunk ends on a tile-independent boundary: kChi2Chunk points, but a
+// relative lightcurve is never cut (its sum comes before its residuals).
+constexpr int kChi2Chunk = 384;
+
+// Whether the object's longest relative lightcurve fits in a chunk.
+__device__ inline bool chi2_fits(const DevObject &ob, const SlotLayout &L, const Smem<PS_FORM_FP64> &s)
+{
+    const int cap = chi2_plan(L, s).cap;
+    return cap >= 32 && ob.max_rel_points <= cap;
+}
+
+template <bool SPLIT>
+__device__ void chi2_fp64(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<PS_FORM_FP64> &s,
+                          const double *a)
+{
+    namespace cgr = cooperative_groups;
+    constexpr int NT = threads_of<PS_FORM_FP64>(), NW = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int rank = 0, cs = 1;
+    if constexpr (SPLIT) {
+        rank = static_cast<int>(cgr::this_cluster().block_rank());
+        cs = static_cast<int>(cgr::this_cluster().num_blocks());
+    }
+    const int F = ob.nfac, C = ob.ncoef, nreal = ob.n_lc - 1, N = ob.ndata;
+    shape_prologue<PS_FORM_FP64, 1>(ob, s, a);
+    const Chi2Plan cp = chi2_plan(L, s);
+    const int cap = cp.cap, lim = min(cap, kChi2Chunk);
+    const double omg = a[C + 2];
+    const double *bm = s.bmat;
+    const double cls = bm[30], cl = bm[31];
+    int *task = reinterpret_cast<int *>(s.misc + M_PIV);
+    // convexity residuals (conv.c:12-29)
+    if (warp < 3) {
+        const double *nc = (warp == 0) ? ob.nx : (warp == 1) ? ob.ny : ob.nz;
+        double res = 0;
+        for (int i = lane; i < F; i += 32) res = res + s.area[i] * nc[i];
+        res = warp_sum(res);
+        if (lane == 0) s.misc[M_CHK + warp] = res;
+    }
+    // chi^2 over the points [q0, q0 + n), their weighted squares in t, added in data order
+    double c2 = 0;   // the last warp's lane 0
+    auto chain = [&](const double *t, int q0, int n) {
+#pragma unroll 8
+        for (int i = 0; i < n; i++) c2 = c2 + t[i] * ob.weight[q0 + i];
+    };
+    int lc0 = 0, q0 = 0, buf = 0, prev_q = 0, prev_n = 0;
+    while (q0 < N) {
+        // the chunk [q0, q1): whole relative lightcurves, at most lim points
+        // (one longer relative lightcurve alone)
+        int lc1 = lc0, q1 = q0;
+        while (lc1 < nreal) {
+            const int end = ob.lc_start[lc1] + ob.lc_npts[lc1];
+            if (end - q0 <= lim) {
+                q1 = end;
+                lc1++;
+            } else {
+                if (!ob.lc_rel[lc1]) {
+                    q1 = q0 + lim;
+                } else if (q1 == q0) {
+                    q1 = end;
+                    lc1++;
+                }
+                break;
+            }
+        }
+        const int n = q1 - q0, npair = (n + 1) / 2;
+        double *ym = cp.ym + static_cast<size_t>(buf) * cap;
+        double *rec = cp.rec;
+        if (tid == 0) *task = 0;
+        // point set-up (bright.c:27-57): the directions and the phase
+        // function; of a cluster's points, the CTA's pairs
+        const int mine = ((npair - rank + cs - 1) / cs) * 2;
+        for (int k = tid; k < mine; k += NT) {
+            const int i = ((k >> 1) * cs + rank) * 2 + (k & 1);
+            if (i >= n) continue;
+            double e[6];
+            const double sc = setup_point_light(ob, cfg, q0 + i, omg, bm, e);
+#pragma unroll
+            for (int c = 0; c < 6; c++) rec[c * cap + i] = e[c];
+            rec[6 * cap + i] = sc;
+        }
+        __syncthreads();
+        if (warp == NW - 1 && lane == 0) chain(cp.ym + static_cast<size_t>(buf ^ 1) * cap, prev_q, prev_n);
+        // brightness, a warp per pair of points
+        for (;;) {
+            int k = 0;
+            if (lane == 0) k = atomicAdd(task, 1);
+            k = __shfl_sync(0xffffffffu, k, 0) * cs + rank;
+            if (k >= npair) break;
+            double br[2] = {0.0, 0.0};
+            int lit = 0;
+            uint16_t *idx = cp.idx + warp * L.wcols;
+#pragma unroll 1
+            for (int u = 0; u < 2; u++) {
+                const int i = 2 * k + u;
+                if (i >= n) break;
+                const double e1 = rec[i], e2 = rec[cap + i], e3 = rec[2 * cap + i];
+                const double f1 = rec[3 * cap + i], f2 = rec[4 * cap + i], f3 = rec[5 * cap + i];
+                const int nl = list_lit_fp64(ob, e1, e2, e3, f1, f2, f3, idx);
+                lit += nl;
+                double b = 0;
+#pragma unroll 2
+                for (int j = lane; j < nl; j += 32) {
+                    const int fi = idx[j];
+                    const double nx = ob.nx[fi], ny = ob.ny[fi], nz = ob.nz[fi];
+                    const double mu = e1 * nx + e2 * ny + e3 * nz;
+                    const double mu0 = f1 * nx + f2 * ny + f3 * nz;
+                    const LitTerms<double, PS_FORM_FP64> lt(mu, mu0, cl, cls);
+                    b = b + s.area[fi] * lt.sv;
+                }
+                if (u == 0) br[0] = b;
+                else br[1] = b;
+                __syncwarp();
+            }
+            // both sums by one butterfly: lanes 0..15 end with the first
+            int id;
+            double v = fold_pair(br[0], br[1], 0, 1, 16, lane, id);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) atomicAdd(lit_counter(s.misc), static_cast<unsigned long long>(lit));
+            const int i = 2 * k + id;
+            if ((lane & 15) == 0 && i < n) {
+                const double y = v * rec[6 * cap + i];
+                ym[i] = y;
+                if constexpr (SPLIT)
+                    for (int r = 0; r < cs; r++)
+                        if (r != rank) *cgr::this_cluster().map_shared_rank(ym + i, r) = y;
+            }
+        }
+        if constexpr (SPLIT) cgr::this_cluster().sync();
+        else __syncthreads();
+        // residuals (mrqcof.c:90-136): a warp per relative lightcurve, then
+        // the absolute lightcurves' points
+        for (int lc = lc0 + warp; lc < lc1; lc += NW) {
+            if (!ob.lc_rel[lc]) continue;
+            const int start = ob.lc_start[lc], npts = ob.lc_npts[lc];
+            double *y = ym + (start - q0);
+            double ave = 0;
+            if (lane == 0)
+                for (int p = 0; p < npts; p++) ave = ave + y[p];
+            ave = __shfl_sync(0xffffffffu, ave, 0);
+            for (int p = lane; p < npts; p += 32) {
+                const int q = start + p;
+                const double coef = ob.sig[q] * npts / ave;
+                const double yr = __dmul_rn(coef, y[p]);
+                const double dy = ob.bright[q] - yr;
+                y[p] = dy * dy * ob.sig2i[q];
+            }
+        }
+        for (int lc = lc0; lc < nreal && ob.lc_start[lc] < q1; lc++) {
+            if (ob.lc_rel[lc]) continue;
+            const int lo = max(ob.lc_start[lc], q0), hi = min(ob.lc_start[lc] + ob.lc_npts[lc], q1);
+            for (int q = lo + tid; q < hi; q += NT) {
+                const double dy = ob.bright[q] - ym[q - q0];
+                ym[q - q0] = dy * dy * ob.sig2i[q];
+            }
+        }
+        prev_q = q0;
+        prev_n = n;
+        q0 = q1;
+        lc0 = lc1;
+        buf ^= 1;
+        __syncthreads();
+    }
+    if (warp == NW - 1 && lane == 0) {
+        chain(cp.ym + static_cast<size_t>(buf ^ 1) * cap, prev_q, prev_n);
+        // the convexity rows
+        const double sig2i = 1 / (cfg.conv_sig * cfg.conv_sig);
+        for (int p = 0; p < 3; p++) {
+            const double dy = 0.0 - s.misc[M_CHK + p];
+            c2 = c2 + dy * dy * sig2i * ob.weight[N + p];
+        }
+        s.misc[M_CHISQ] = c2;
+    }
+    __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// chi^2 alone at parameters a[], tensor-core paths of the mixed form (the
+// counterpart of chi2_fp64: what decides whether a step is accepted).  No
+// contraction, no derivative sums, and so no operand tile and no per-tile
+// barriers: set-up with a thread per point, brightness with a warp per 8
+// points, residuals with a warp per 32-point tile, one thread's ordered sum.
+// Each value by evaluate's operations in their order (a point's brightness:
+// facet_stage_tc's four lanes and four facet quarters; chi^2: tile sums in
+// tile order), so chi^2 is evaluate's bit for bit.  The four quarters of a
+// point run side by side in a lane (four independent chains).
+// Buffers in the operand region (at least 1040 points: any relative
+// lightcurve fits).
+// Measured: 3010 fits of 980 points, 288 facets 290 -> 219 ms; 1010 fits with
+// 81 coefficients, 512 facets 247 -> 171 ms.
+// ---------------------------------------------------------------------------
+template <int KU>
+__device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<PS_FORM_MIXED> &s,
+                           const double *a)
+{
+    constexpr int NT = threads_of<PS_FORM_MIXED>(), NW = NT / 32, P = 32;
+    constexpr int kTiles = 16 * kRedStride;   // two tile sums each in s.red
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int F = ob.nfac, C = ob.ncoef, nreal = ob.n_lc - 1, N = ob.ndata;
+    shape_prologue<PS_FORM_MIXED, KU>(ob, s, a);
+    const int cap = static_cast<int>(2 * (L.blo - L.bhi) > 33280 ? 2 * (L.blo - L.bhi) : 33280) / 32 & ~31;
+    float *rec = reinterpret_cast<float *>(s.bhi);   // [7][cap] directions, phase function
+    float *ym = rec + 7 * cap;                       // [cap] model values
+    double *tsum = s.red, *c2sum = s.red + kTiles;
+    const double omg = a[C + 2];
+    const float cls = s.bmat[30], cl = s.bmat[31];
+    const int cq = tc_kpad(F) >> 5;   // 8-facet groups per facet quarter
+    int lc0 = 0, q0 = 0;
+    while (q0 < N) {
+        // the chunk [q0, q1): whole relative lightcurves, absolute ones cut
+        // at a tile, at most cap points and kTiles tiles
+        int lc1 = lc0, q1 = q0, tiles = 0;
+        while (lc1 < nreal) {
+            const int st = max(ob.lc_start[lc1], q0), end = ob.lc_start[lc1] + ob.lc_npts[lc1];
+            const int nt = (end - st + P - 1) / P;
+            if (end - q0 <= cap && tiles + nt <= kTiles) {
+                q1 = end;
+                tiles += nt;
+                lc1++;
+                continue;
+            }
+            if (!ob.lc_rel[lc1]) {
+                const int take = min((cap - (st - q0)) / P, kTiles - tiles);
+                q1 = st + take * P;
+                tiles += take;
+            }
+            break;
+        }
+        const int n = q1 - q0;
+        for (int i = tid; i < n; i += NT) {
+            float pt[32];
+            const float4 g0 = ob.geo_f[2 * (q0 + i)], g1 = ob.geo_f[2 * (q0 + i) + 1];
+            setup_mixed_phase(ob.tim[q0 + i], omg, cfg.phi0, pt);
+            setup_mixed_geo(g0, g1, s.bmat, pt, 0);
+            float e[6];
+            rotate_directions(pt, e);
+#pragma unroll
+            for (int c = 0; c < 6; c++) rec[c * cap + i] = e[c];
+            rec[6 * cap + i] = pt[24];
+        }
+        __syncthreads();
+        const float2 CL = make_float2(cl, cl), CLS = make_float2(cls, cls);
+        const int fl = lane & 3;
+        for (int g = warp; g * 8 < n; g += NW) {
+            const int i = g * 8 + (lane >> 2);
+            float e[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (i < n) {
+#pragma unroll
+                for (int c = 0; c < 6; c++) e[c] = rec[c * cap + i];
+            }
+            const float2 E1 = make_float2(e[0], e[0]), E2 = make_float2(e[1], e[1]), E3 = make_float2(e[2], e[2]);
+            const float2 F1 = make_float2(e[3], e[3]), F2 = make_float2(e[4], e[4]), F3 = make_float2(e[5], e[5]);
+            float2 br[4];
+#pragma unroll
+            for (int h = 0; h < 4; h++) br[h] = make_float2(0.f, 0.f);
+#pragma unroll 1
+            for (int kc = 0; kc < cq; kc++) {
+#pragma unroll
+                for (int h = 0; h < 4; h++) {
+                    const float4 *fp = s.fac + (h * cq + kc) * 8 + 2 * fl;
+                    const float4 fa = fp[0], fb = fp[1];
+                    const LitPair lp(fa, fb, E1, E2, E3, F1, F2, F3);
+                    // the product rounded by itself, as in facet_stage_tc
+                    // (which uses it twice): a paired product is fused into
+                    // the paired addition, scalar ones are not
+                    const float2 sv = lp.law(CL, CLS);
+                    br[h] = __fadd2_rn(br[h], make_float2(__fmul_rn(lp.ax.x, sv.x), __fmul_rn(lp.ax.y, sv.y)));
+                }
+            }
+            float t = 0.f;
+#pragma unroll
+            for (int h = 0; h < 4; h++) {
+                float v = br[h].x + br[h].y;
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                v += __shfl_xor_sync(0xffffffffu, v, 2);
+                t += v;
+            }
+            if (fl == 0 && i < n) ym[i] = t * rec[6 * cap + i];
+        }
+        __syncthreads();
+        // sums of the relative lightcurves' model values, a tile per warp
+        int k = 0;
+        for (int lc = lc0; lc < nreal && ob.lc_start[lc] < q1; lc++) {
+            const int lo = max(ob.lc_start[lc], q0), hi = min(ob.lc_start[lc] + ob.lc_npts[lc], q1);
+            for (int u = lo; u < hi; u += P, k++) {
+                if (k % NW != warp || !ob.lc_rel[lc]) continue;
+                const double y = warp_sum(u + lane < hi ? static_cast<double>(ym[u + lane - q0]) : 0.0);
+                if (lane == 0) tsum[k] = y;
+            }
+        }
+        __syncthreads();
+        // weighted squared residuals (mrqcof.c:90-136); the sums of a
+        // relative lightcurve's tiles are read before they are replaced
+        k = 0;
+        for (int lc = lc0; lc < nreal && ob.lc_start[lc] < q1; lc++) {
+            const int lo = max(ob.lc_start[lc], q0), hi = min(ob.lc_start[lc] + ob.lc_npts[lc], q1);
+            const bool rel = ob.lc_rel[lc] != 0;
+            const int npts = ob.lc_npts[lc], k0 = k;
+            for (int u = lo; u < hi; u += P, k++) {
+                if (k % NW != warp) continue;
+                double c2 = 0, inv_ave = 0;
+                if (rel) {
+                    double ave = 0;
+                    for (int w = 0; w * P < npts; w++) ave += tsum[k0 + w];
+                    inv_ave = 1.0 / ave;
+                }
+                if (u + lane < hi) {
+                    const int q = u + lane;
+                    const double yt = static_cast<double>(ym[q - q0]);
+                    const double sig2i = ob.sig2i[q], wg = ob.weight[q];
+                    double dy;
+                    if (rel) {
+                        const double coef = ob.sig[q] * npts * inv_ave;
+                        // (the wide path stores the renormalised value, the
+                        // other one contracts the product into the difference)
+                        dy = KU == 3 ? ob.bright[q] - __dmul_rn(coef, yt) : fma(-coef, yt, ob.bright[q]);
+                    } else {
+                        dy = ob.bright[q] - yt;
+                    }
+                    c2 = dy * dy * sig2i * wg;
+                }
+                c2 = warp_sum(c2);
+                if (lane == 0) c2sum[k] = c2;
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            double c = s.misc[M_CHISQ];
+#pragma unroll 4
+            for (int w = 0; w < tiles; w++) c += c2sum[w];
+            s.misc[M_CHISQ] = c;
+        }
+        q0 = q1;
+        lc0 = lc1;
+        // (the next chunk's set-up writes rec only; its first barrier comes
+        // before anything that replaces the sums)
+    }
+    // convexity rows (conv.c:12-29)
+    if (warp >= 1 && warp < 4) {
+        const double *nc = (warp == 1) ? ob.nx : (warp == 2) ? ob.ny : ob.nz;
+        double res = 0;
+        for (int i = lane; i < F; i += 32) res = res + s.area[i] * nc[i];
+        res = warp_sum(res);
+        if (lane == 0) s.misc[M_CHK + warp - 1] = res;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double c2 = 0;
+        if (lane < 3) {
+            const double sig2i = 1 / (cfg.conv_sig * cfg.conv_sig);
+            const double dy = 0.0 - s.misc[M_CHK + lane];
+            c2 = dy * dy * sig2i * ob.weight[N + lane];
+        }
+        c2 = warp_sum(c2);
+        if (lane == 0) s.misc[M_CHISQ] += c2;
     }
     __syncthreads();
 }
@@ -2668,15 +3119,29 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
 {
     constexpr bool kTensor = FORM == PS_FORM_MIXED && (KU == 0 || KU == 3);
     // one model evaluation; with split (FP64 form, cluster launch) spread
-    // over the cluster's CTAs (evaluate_split)
-    auto eval = [&](const double *a, double *M, double *bv) {
+    // over the cluster's CTAs (evaluate_split).  fresh = false: chi2 has just
+    // run at the same parameters.
+    auto eval = [&](const double *a, double *M, double *bv, bool fresh) {
         if constexpr (FORM == PS_FORM_FP64) {
             if (split) {
-                evaluate_split(ob, cfg, L, s, a, M, bv, scratch);
+                evaluate_split(ob, cfg, L, s, a, M, bv, scratch, fresh);
                 return;
             }
         }
-        evaluate<FORM, KU>(ob, cfg, L, s, a, M, bv, scratch, tcs);
+        evaluate<FORM, KU>(ob, cfg, L, s, a, M, bv, scratch, tcs, fresh);
+    };
+    // chi^2 alone where the form has it (about half of the steps are
+    // rejected, and need no more)
+    bool lazy = false;
+    if constexpr (FORM == PS_FORM_FP64) lazy = chi2_fits(ob, L, s);
+    else lazy = kTensor;
+    auto chi2 = [&](const double *a) {
+        if constexpr (FORM == PS_FORM_FP64) {
+            if (split) chi2_fp64<true>(ob, cfg, L, s, a);
+            else chi2_fp64<false>(ob, cfg, L, s, a);
+        } else if constexpr (kTensor) {
+            chi2_mixed<KU>(ob, cfg, L, s, a);
+        }
     };
     constexpr int NT = threads_of<FORM>();
     const int tid = threadIdx.x;
@@ -2711,6 +3176,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
     double chk_acc[3] = {0, 0, 0}, chk_first[3] = {0, 0, 0}, chk_trial[3] = {0, 0, 0};
     double area_first = 0, area_trial = 0, totarea = 0;
     int niter = 0, last_err = 0;
+    bool stale = false;   // alpha and beta are not yet those of the accepted step
     // learned early stop: accepted chi^2 and lambda of the first iterations
     double hist[5], lam_hist[4];
     double pred_dev = 0;
@@ -2731,7 +3197,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
         niter = static_cast<int>(st[ma + 11]);
         last_err = static_cast<int>(st[ma + 12]);
         pred_dev = st[ma + 13];
-        eval(s.cg, s.alpha, s.beta);
+        eval(s.cg, s.alpha, s.beta, true);
         if constexpr (kTensor) {
             if (*s.abort) last_err = kErrTcTimeout;
         }
@@ -2741,7 +3207,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
         bool accepted = false;
         if (alamda < 0) {
             alamda = cfg.alamda_start;
-            eval(s.cg, s.alpha, s.beta);
+            eval(s.cg, s.alpha, s.beta, true);
             if constexpr (kTensor) {
                 if (*s.abort) {
                     last_err = kErrTcTimeout;
@@ -2753,6 +3219,17 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
             area_first = s.misc[M_AREA];
             for (int c = 0; c < 3; c++) chk_first[c] = s.misc[M_CHK + c];
             totarea = area_first;
+        } else if (stale) {
+            // alpha and beta of the step accepted last, now that another
+            // step is taken from it
+            eval(s.cg, s.alpha, s.beta, false);
+            if constexpr (kTensor) {
+                if (*s.abort) {
+                    last_err = kErrTcTimeout;
+                    break;
+                }
+            }
+            stale = false;
         }
         for (int e = tid; e < mf * mf; e += NT) {
             const int j = e / mf, k = e - j * mf;
@@ -2785,7 +3262,8 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
                 s.atry[l] = s.cg[l] + s.da[j];
             }
             __syncthreads();
-            eval(s.atry, s.covar, s.da);
+            if (lazy) chi2(s.atry);
+            else eval(s.atry, s.covar, s.da, true);
             if constexpr (kTensor) {
                 if (*s.abort) {
                     last_err = kErrTcTimeout;
@@ -2798,8 +3276,11 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
             totarea = area_trial;
             if (chisq < ochisq) {
                 accepted = true;
-                for (int e = tid; e < mf * mf; e += NT) s.alpha[e] = s.covar[e];
-                for (int j = tid; j < mf; j += NT) s.beta[j] = s.da[j];
+                stale = lazy;
+                if (!lazy) {
+                    for (int e = tid; e < mf * mf; e += NT) s.alpha[e] = s.covar[e];
+                    for (int j = tid; j < mf; j += NT) s.beta[j] = s.da[j];
+                }
                 for (int l = tid; l < ma; l += NT) s.cg[l] = s.atry[l];
             } else {
                 chisq = ochisq;
