@@ -119,6 +119,7 @@ struct SlotLayout {
     size_t rels;            // relative-lightcurve rows in shared memory, or 0 (global scratch)
     size_t pref;            // tensor-core path: per-point data prefetched for the contraction window
     size_t flist;           // tensor-core path: the free parameters' columns
+    size_t phase, resid;    // FP64 form: first set-up part of the next tiles; residuals and point orders
     size_t lit;             // FP64 form: per point of a tile, its lit-facet count, then its lit facets
     size_t bytes;
 };
@@ -134,7 +135,7 @@ PSG_HD constexpr int threads_of()
     return FORM == PS_FORM_MIXED ? 512 : 384;
 }
 constexpr int kPointStride = 33;   // reals of per-point set-up (odd: a warp with one point per lane hits 32 banks)
-constexpr int kRedStride = 8;      // doubles of per-point facet sums
+constexpr int kRedStride = 9;      // doubles of per-point facet sums
 constexpr int kMisc = 40;
 // Prefetch area of the tensor-core path, for a 32-point tile: times (32
 // doubles), two copies of the FP32 geometry (32 x 2 float4 each) and sig^-2,
@@ -246,6 +247,9 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     L.bmat = take(32 * rs);
     L.rels = rel_rows > 0 ? take(static_cast<size_t>(rel_rows) * rel_row_stride(ma) * rs) : 0;
     // FP64 form: P counts (int) and P x wcols facet indices (uint16_t)
+    const int warps64 = threads_of<PS_FORM_FP64>() / 32;
+    L.phase = form == PS_FORM_FP64 ? take(static_cast<size_t>(4 * warps64) * P * d) : 0;
+    L.resid = form == PS_FORM_FP64 ? take(96 * d + static_cast<size_t>(32) * warps64) : 0;
     L.lit = form == PS_FORM_FP64 ? take(static_cast<size_t>(P) * (4 + 2 * L.wcols)) : 0;
     L.bytes = o;
     return L;

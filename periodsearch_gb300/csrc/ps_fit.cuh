@@ -99,6 +99,9 @@ struct Smem {
     // facets in increasing order ([P][wcols], the W row holds their values)
     int *nlit;
     uint16_t *lidx;
+    double *phase;          // FP64 form: [4][warps * P] first set-up part of the CTA's next tiles
+    double *resid;          // FP64 form: [3][32] a tile's residuals, their weighted squares, renormalisation factors
+    unsigned char *order;   // FP64 form: [warps][32] points of the tile by lit count
     uint32_t *tslot;
     int *abort;
 };
@@ -134,6 +137,9 @@ __device__ inline Smem<FORM> carve(char *base, const SlotLayout &L)
     s.nlit = L.form == PS_FORM_FP64 ? reinterpret_cast<int *>(base + L.lit) : nullptr;
     s.lidx = L.form == PS_FORM_FP64 ? reinterpret_cast<uint16_t *>(base + L.lit + 4 * static_cast<size_t>(L.P))
                                      : nullptr;
+    s.phase = L.form == PS_FORM_FP64 ? reinterpret_cast<double *>(base + L.phase) : nullptr;
+    s.resid = L.form == PS_FORM_FP64 ? reinterpret_cast<double *>(base + L.resid) : nullptr;
+    s.order = L.form == PS_FORM_FP64 ? reinterpret_cast<unsigned char *>(base + L.resid + 96 * sizeof(double)) : nullptr;
     s.dsph = L.dsph_smem == kBasisSmem ? reinterpret_cast<float *>(base + L.dsph) : nullptr;
     if (basis_on_tensor(L.dsph_smem)) {
         s.bhi = reinterpret_cast<unsigned char *>(base + L.bhi);
@@ -391,8 +397,8 @@ __device__ inline int list_lit_fp64(const DevObject &ob, double e1, double e2, d
 // lane busy (an FP64 instruction holds its sub-partition's FP64 unit for
 // the whole warp, however few lanes are active), lane l taking the list's
 // entries l, l + 32, ...  W is left in the W row at the list positions.
-// The facet sums go to s.red[p * kRedStride + 0..5]: brightness, the three
-// rotation derivatives, the Lambert and the scattering-weight derivatives.
+// The facet sums go to s.red[p * kRedStride + 0..8]: brightness, U, V, the
+// Lambert and the scattering-weight derivatives.
 // count: add the point's lit facets to the CTA's counter.
 __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> &s, int p, int wcols, double cl,
                                         double cls, bool count)
@@ -407,7 +413,7 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
     // (n_i . E_k)) (bright.c:87-104; D_k, E_k: the derivative directions of
     // the Earth and Sun vectors) are D_k . U + E_k . V with U = sum Area
     // dsmu n and V = sum Area dsmu0 n: the law accumulates U and V, the six
-    // dot products run once per point.
+    // dot products run once per point (tile_rows_fp64).
     double br = 0, ux = 0, uy = 0, uz = 0, vx = 0, vy = 0, vz = 0, dcl = 0, dcls = 0;
     double *Wp = s.W + static_cast<size_t>(p) * wcols;
     for (int j = lane; j < n; j += 32) {
@@ -429,23 +435,9 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
         dcl = dcl + mu * mu0 * ar;
         dcls = dcls + ar * lt.dcls_w;
     }
-    // the nine sums go through the point's J row (written by the
-    // contraction only after the stage's barrier)
-    double *sums = s.J + static_cast<size_t>(p) * ob.ma;
     const double v9[9] = {br, ux, uy, uz, vx, vy, vz, dcl, dcls};
-    warp_sum9(v9, sums, lane);
-    __syncwarp();
+    warp_sum9(v9, s.red + p * kRedStride, lane);
     if (lane == 0) {
-        // D_k = (de[k], de[3 + k], de[6 + k]), E_k likewise from de0
-        const double *de = pt + 6, *de0 = pt + 15;
-        double *rd = s.red + p * kRedStride;
-        rd[0] = sums[0];
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            rd[1 + k] = de[k] * sums[1] + de[3 + k] * sums[2] + de[6 + k] * sums[3] + de0[k] * sums[4] +
-                        de0[3 + k] * sums[5] + de0[6 + k] * sums[6];
-        rd[4] = sums[7];
-        rd[5] = sums[8];
         s.nlit[p] = n;
         if (count) atomicAdd(lit_counter(s.misc), static_cast<unsigned long long>(n));
     }
@@ -453,10 +445,9 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
 
 // Accumulates the rows J[0..np) (model values in ym) of one tile into the
 // normal matrix M (lower triangle), bv and chi^2 (mrqcof.c:106-136).  The
-// FP64 form sums every alpha element over points in data order in FP64; the
-// mixed form sums the tile in FP32 and adds the tile sum to the FP64 total.
-// Mixed form: every thread keeps its share of the alpha lower triangle
-// (elements tid + u*256) and of beta (element tid) as FP32 partial sums in
+// SIMT path of the mixed form sums the tile in FP32 and adds the tile sum to
+// the FP64 total: every thread keeps its share of the alpha lower triangle
+// (elements tid + u*512) and of beta (element tid) as FP32 partial sums in
 // registers and adds them to the FP64 totals every few tiles.
 constexpr int kAccPerThread = 8;    // with 512 threads: mfit <= 90
 constexpr int kTilesPerFlush = 8;
@@ -464,10 +455,9 @@ constexpr int kTilesPerFlush = 8;
 // of TF32 high/low parts) is added to the FP64 normal matrix every 16 tiles.
 constexpr int kTcTilesPerFlush = 16;
 
-template <int FORM>
 __device__ inline void flush_partials(double *M, double *bv, int mf, float (&accA)[kAccPerThread], float &accB)
 {
-    constexpr int NT = threads_of<FORM>();
+    constexpr int NT = threads_of<PS_FORM_MIXED>();
     const int tid = threadIdx.x;
     const int ntri = mf * (mf + 1) / 2;
 #pragma unroll
@@ -484,106 +474,54 @@ __device__ inline void flush_partials(double *M, double *bv, int mf, float (&acc
     accB = 0.f;
 }
 
-template <int FORM>
-__device__ void accumulate_tile(const DevObject &ob, Smem<FORM> &s, double *M, double *bv, int np, int q0pt,
-                                bool conv, double conv_sig, float (&accA)[kAccPerThread], float &accB,
-                                const double *Jrows = nullptr, const double *ymv = nullptr, int part = 0,
-                                int parts = 1)
+__device__ void accumulate_tile(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int np, int q0pt, bool conv,
+                                double conv_sig, float (&accA)[kAccPerThread], float &accB)
 {
-    using R = typename RealOf<FORM>::T;
-    constexpr int NT = threads_of<FORM>();
+    constexpr int NT = threads_of<PS_FORM_MIXED>();
     const int tid = threadIdx.x;
     const int ma = ob.ma, mf = ob.mfit;
-    R *wt = s.W;  // [np][mf], reuses the facet-weight tile
-    if constexpr (FORM == PS_FORM_FP64) {
-        // FP64 form: the tile's rows and model values (Jrows, ymv: another
-        // CTA's tile staged here, by default the CTA's own), and of the
-        // normal matrix only the elements e = part NT + tid (mod parts NT);
-        // chi^2 is summed whole
-        if (!Jrows) Jrows = s.J;
-        if (!ymv) ymv = s.ym;
-        for (int e = tid; e < np * mf; e += NT) {
-            const int p = e / mf, j = e - p * mf;
-            const int q = q0pt + p;
+    float *wt = s.W;  // [np][mf], reuses the facet-weight tile
+    // per point: FP32 weight sig2i*w and residual; chi^2 of the tile
+    // summed over one warp in FP64
+    float *dyv = s.accs;
+    float *wtp = dyv + 32;
+    if (tid < 32) {
+        double c2 = 0;
+        if (tid < np) {
+            const int q = q0pt + tid;
             const double sig2i = conv ? 1 / (conv_sig * conv_sig) : ob.sig2i[q];
             const double wg = ob.weight[q];
-            wt[p * mf + j] = Jrows[p * ma + ob.free_list[j]] * sig2i * wg;
+            const double dy = (conv ? 0.0 : ob.bright[q]) - s.ym[tid];
+            dyv[tid] = static_cast<float>(dy);
+            wtp[tid] = static_cast<float>(sig2i * wg);
+            c2 = dy * dy * sig2i * wg;
         }
-    } else {
-        // per point: FP32 weight sig2i*w and residual; chi^2 of the tile
-        // summed over one warp in FP64
-        float *dyv = s.accs;
-        float *wtp = dyv + 32;
-        if (tid < 32) {
-            double c2 = 0;
-            if (tid < np) {
-                const int q = q0pt + tid;
-                const double sig2i = conv ? 1 / (conv_sig * conv_sig) : ob.sig2i[q];
-                const double wg = ob.weight[q];
-                const double dy = (conv ? 0.0 : ob.bright[q]) - s.ym[tid];
-                dyv[tid] = static_cast<float>(dy);
-                wtp[tid] = static_cast<float>(sig2i * wg);
-                c2 = dy * dy * sig2i * wg;
-            }
-            c2 = warp_sum(c2);
-            if (tid == 0) s.misc[M_CHISQ] += c2;
-        }
-        __syncthreads();
-        for (int e = tid; e < np * mf; e += NT) {
-            const int p = e / mf, j = e - p * mf;
-            wt[p * mf + j] = s.J[p * ma + ob.free_list[j]] * wtp[p];
-        }
+        c2 = warp_sum(c2);
+        if (tid == 0) s.misc[M_CHISQ] += c2;
+    }
+    __syncthreads();
+    for (int e = tid; e < np * mf; e += NT) {
+        const int p = e / mf, j = e - p * mf;
+        wt[p * mf + j] = s.J[p * ma + ob.free_list[j]] * wtp[p];
     }
     __syncthreads();
     const int ntri = mf * (mf + 1) / 2;
-    if constexpr (FORM == PS_FORM_FP64) {
-        for (int e = part * NT + tid; e < ntri; e += parts * NT) {
+#pragma unroll
+    for (int u = 0; u < kAccPerThread; u++) {
+        const int e = tid + u * NT;
+        if (e < ntri) {
             const int j = tri_row(e);
             const int k = e - j * (j + 1) / 2;
             const int lk = ob.free_list[k];
-            double acc = M[j * mf + k];
-            for (int p = 0; p < np; p++) acc = acc + wt[p * mf + j] * Jrows[p * ma + lk];
-            M[j * mf + k] = acc;
-        }
-        for (int j = part * NT + tid; j < mf; j += parts * NT) {
-            double acc = bv[j];
-            for (int p = 0; p < np; p++) {
-                const double y = conv ? 0.0 : ob.bright[q0pt + p];
-                acc = acc + (y - ymv[p]) * wt[p * mf + j];
-            }
-            bv[j] = acc;
-        }
-    } else {
-        const float *dyv = s.accs;
-#pragma unroll
-        for (int u = 0; u < kAccPerThread; u++) {
-            const int e = tid + u * NT;
-            if (e < ntri) {
-                const int j = tri_row(e);
-                const int k = e - j * (j + 1) / 2;
-                const int lk = ob.free_list[k];
-                float acc = accA[u];
-                for (int p = 0; p < np; p++) acc = fmaf(wt[p * mf + j], s.J[p * ma + lk], acc);
-                accA[u] = acc;
-            }
-        }
-        if (tid < mf) {
-            float acc = accB;
-            for (int p = 0; p < np; p++) acc = fmaf(dyv[p], wt[p * mf + tid], acc);
-            accB = acc;
+            float acc = accA[u];
+            for (int p = 0; p < np; p++) acc = fmaf(wt[p * mf + j], s.J[p * ma + lk], acc);
+            accA[u] = acc;
         }
     }
-    if (FORM == PS_FORM_FP64 && tid == NT - 1) {
-        const double *yv = ymv ? ymv : s.ym;
-        double c2 = s.misc[M_CHISQ];
-        for (int p = 0; p < np; p++) {
-            const int q = q0pt + p;
-            const double sig2i = conv ? 1 / (conv_sig * conv_sig) : ob.sig2i[q];
-            const double y = conv ? 0.0 : ob.bright[q];
-            const double dy = y - yv[p];
-            c2 = c2 + dy * dy * sig2i * ob.weight[q];
-        }
-        s.misc[M_CHISQ] = c2;
+    if (tid < mf) {
+        float acc = accB;
+        for (int p = 0; p < np; p++) acc = fmaf(dyv[p], wt[p * mf + tid], acc);
+        accB = acc;
     }
     __syncthreads();
 }
@@ -766,104 +704,66 @@ __device__ inline double phase_scale_fp64(double a, double k, double ex, double 
 // Point set-up of observation q (bright.c:27-57, phasec.c, matrix.c): the
 // rotated Earth and Sun directions with their beta/lambda/omega derivatives,
 // the phase function and its derivatives, into pt[0..27].
-template <int FORM>
-__device__ inline void setup_point(const DevObject &ob, const FitConfig &cfg, int q, double omg,
-                                   const typename RealOf<FORM>::T *bm, typename RealOf<FORM>::T *pt)
+__device__ inline void setup_point(const DevObject &ob, const FitConfig &cfg, int q, double omg, const float *bm,
+                                   float *pt)
 {
-    if constexpr (FORM == PS_FORM_MIXED) {
-        setup_mixed_phase(ob.tim[q], omg, cfg.phi0, pt);
-        setup_mixed_geo(ob.geo_f[2 * q], ob.geo_f[2 * q + 1], bm, pt);
-        setup_mixed_rotate(pt);
-        return;
-    }
-    const typename RealOf<FORM>::T *B = bm, *DB0 = bm + 9, *DB1 = bm + 18;
-    const typename RealOf<FORM>::T php0 = bm[27], php1 = bm[28], php2 = bm[29];
-    using R = typename RealOf<FORM>::T;
-    constexpr bool kFP64 = FORM == PS_FORM_FP64;
-    R ee[3], e0v[3], alpha;
-    if constexpr (kFP64) {
-        ee[0] = ob.eex[q];
-        ee[1] = ob.eey[q];
-        ee[2] = ob.eez[q];
-        e0v[0] = ob.e0x[q];
-        e0v[1] = ob.e0y[q];
-        e0v[2] = ob.e0z[q];
-        alpha = ob.alpha_pt[q];
-    } else {
-        const float4 g0 = ob.geo_f[2 * q], g1 = ob.geo_f[2 * q + 1];
-        ee[0] = g0.x;
-        ee[1] = g0.y;
-        ee[2] = g0.z;
-        alpha = g0.w;
-        e0v[0] = g1.x;
-        e0v[1] = g1.y;
-        e0v[2] = g1.z;
-    }
-    const double td = ob.tim[q];
-    const R t = R(td);
-    R ex, scale;
-    R inv_w = 0;
-    if constexpr (kFP64) {
-        ex = exp(-alpha / php1);
-        scale = phase_scale_fp64(php0, php2, ex, alpha);
-    } else {
-        inv_w = 1.f / php1;
-        ex = expf(-alpha * inv_w);
-        scale = 1 + php0 * ex + php2 * alpha;
-    }
-    const double f = rotation_phase_fp64(omg, td, cfg.phi0);
-    const R cf = cos(f), sf = sin(f);
-    const R fm[9] = {cf, sf, R(0), -sf, cf, R(0), R(0), R(0), R(1)};
-    const R dfm[9] = {-t * sf, t * cf, R(0), -t * cf, -t * sf, R(0), R(0), R(0), R(0)};
-    R tm[9], d0[9], d1[9], d2[9];
+    setup_mixed_phase(ob.tim[q], omg, cfg.phi0, pt);
+    setup_mixed_geo(ob.geo_f[2 * q], ob.geo_f[2 * q + 1], bm, pt);
+    setup_mixed_rotate(pt);
+}
+
+// FP64 form: the point set-up in two parts.  The first is what every point
+// needs once, a point per lane: the cos and sin of the rotation phase, the
+// phase function's exponential and its derivative by d, into ph[0..3][stride].
+__device__ inline void setup_phase_fp64(const DevObject &ob, const FitConfig &cfg, int q, double omg,
+                                        const double *bm, double *ph, int stride)
+{
+    const double alpha = ob.alpha_pt[q], php0 = bm[27], php1 = bm[28];
+    const double ex = exp(-alpha / php1);
+    const double f = rotation_phase_fp64(omg, ob.tim[q], cfg.phi0);
+    ph[0] = cos(f);
+    ph[stride] = sin(f);
+    ph[2 * stride] = ex;
+    ph[3 * stride] = php0 * ex * alpha / (php1 * php1);
+}
+
+// The second, of the point's directions the row i of e = fm B ee (part 0) or
+// of its derivative by beta (1), lambda (2) or omega (3), and the same of the
+// Sun vector: twelve parts of at most 14 FP64 instructions, a warp each with
+// a point per lane.  The zeros and ones of the rotation fm are left out of
+// the reference's products (matrix.c), which changes no value.
+__device__ inline void setup_row_fp64(const DevObject &ob, int q, int part, int i, const double *bm,
+                                      const double *ph, int stride, double *pt)
+{
+    const double ee[3] = {ob.eex[q], ob.eey[q], ob.eez[q]}, es[3] = {ob.e0x[q], ob.e0y[q], ob.e0z[q]};
+    const double *B = bm + (part == 3 ? 0 : 9 * part);
+    double x = 0, y = 0;
+    if (i == 2) {
+        if (part < 3) {
 #pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            R x = 0, y0 = 0, y1 = 0, y2 = 0;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                x = x + fm[i * 3 + k] * B[k * 3 + j];
-                y0 = y0 + fm[i * 3 + k] * DB0[k * 3 + j];
-                y1 = y1 + fm[i * 3 + k] * DB1[k * 3 + j];
-                y2 = y2 + dfm[i * 3 + k] * B[k * 3 + j];
+            for (int j = 0; j < 3; j++) {
+                x = fma(B[6 + j], ee[j], x);
+                y = fma(B[6 + j], es[j], y);
             }
-            tm[i * 3 + j] = x;
-            d0[i * 3 + j] = y0;
-            d1[i * 3 + j] = y1;
-            d2[i * 3 + j] = y2;
         }
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        R x = 0, y = 0;
+    } else {
+        const double cf = ph[0], sf = ph[stride];
+        double f0 = i == 0 ? cf : -sf, f1 = i == 0 ? sf : cf;
+        if (part == 3) {
+            const double t = ob.tim[q];
+            f0 = __dmul_rn(-t, i == 0 ? sf : cf);
+            f1 = i == 0 ? __dmul_rn(t, cf) : __dmul_rn(-t, sf);
+        }
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            x = x + tm[i * 3 + j] * ee[j];
-            y = y + tm[i * 3 + j] * e0v[j];
+            const double m = fma(f1, B[3 + j], __dmul_rn(f0, B[j]));
+            x = fma(m, ee[j], x);
+            y = fma(m, es[j], y);
         }
-        pt[i] = x;
-        pt[3 + i] = y;
     }
-    // de[i][j] = sum_k dtm[j][i][k] ee[k]; stored de[i*3+j] (j = derivative)
-    const R *dd[3] = {d0, d1, d2};
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            R x = 0, y = 0;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                x = x + dd[j][i * 3 + k] * ee[k];
-                y = y + dd[j][i * 3 + k] * e0v[k];
-            }
-            pt[6 + i * 3 + j] = x;
-            pt[15 + i * 3 + j] = y;
-        }
-    pt[24] = scale;
-    pt[25] = ex;
-    if constexpr (kFP64) pt[26] = php0 * ex * alpha / (php1 * php1);
-    else pt[26] = php0 * ex * alpha * (inv_w * inv_w);
-    pt[27] = alpha;
+    // directions at pt[0..5], derivative column part - 1 at pt[6..14] and pt[15..23]
+    pt[part == 0 ? i : 6 + i * 3 + part - 1] = x;
+    pt[part == 0 ? 3 + i : 15 + i * 3 + part - 1] = y;
 }
 
 // The part of the FP64 form's set-up that the model value needs: the rotated
@@ -1619,48 +1519,33 @@ __device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double 
 }
 
 // ---------------------------------------------------------------------------
-// Model evaluation (mrqcof) at parameters a[] into matrix M (mfit x mfit,
+// Mixed form's model evaluation (mrqcof) at parameters a[] into M (mfit x mfit,
 // lower triangle accumulated then mirrored) and vector bv.  Leaves chi^2,
 // the facet-area sum and the convexity residuals in misc.  fresh = false:
 // shape_prologue has run at the same parameters already (the chi^2 of an
-// accepted step), and the FP64 form's lit facets have been counted.
+// accepted step).
 // ---------------------------------------------------------------------------
-template <int FORM, int KU>
-__device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<FORM> &s,
-                         const double *a, double *M, double *bv, typename RealOf<FORM>::T *scratch, TcState &tcs,
-                         bool fresh = true)
+template <int KU>
+__device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L,
+                               Smem<PS_FORM_MIXED> &s, const double *a, double *M, double *bv, float *scratch,
+                               TcState &tcs, bool fresh = true)
 {
-    using R = typename RealOf<FORM>::T;
-    constexpr bool kFP64 = FORM == PS_FORM_FP64;
+    using R = float;
     // tensor-core path: the point set-up of the next tile runs on warps 1..15
     // while thread 0 issues the current tile's MMAs
-    constexpr bool kPipe = !kFP64 && (KU == 0 || KU == 3);
+    constexpr bool kPipe = KU == 0 || KU == 3;
     // alpha/beta on the tensor cores (KU 0), or on the SIMT pipes behind the
     // wide tensor-core contraction (KU 3: 65..96 coefficients)
-    constexpr bool kTcAlpha = !kFP64 && KU == 0;
-    constexpr bool kWide = !kFP64 && KU == 3;
-    constexpr int NT = threads_of<FORM>();
+    constexpr bool kTcAlpha = KU == 0;
+    constexpr bool kWide = KU == 3;
+    constexpr int NT = threads_of<PS_FORM_MIXED>();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int F = ob.nfac, C = ob.ncoef, ma = ob.ma, mf = ob.mfit, P = L.P;
     const int wcols = L.wcols;
     const int RW = rel_row_stride(ma);   // parked row of a relative lightcurve
-    const R *nxR, *nyR, *nzR, *dareaR;
-    const R *dsphR;
-    if constexpr (kFP64) {
-        nxR = ob.nx;
-        nyR = ob.ny;
-        nzR = ob.nz;
-        dareaR = ob.darea;
-        dsphR = ob.dsph;
-    } else {
-        nxR = ob.nx_f;
-        nyR = ob.ny_f;
-        nzR = ob.nz_f;
-        dareaR = ob.darea_f;
-        dsphR = ob.dsph_f;
-    }
+    const R *nxR = ob.nx_f, *nyR = ob.ny_f, *nzR = ob.nz_f, *dareaR = ob.darea_f;
 
-    if (fresh) shape_prologue<FORM, KU>(ob, s, a);
+    if (fresh) shape_prologue<PS_FORM_MIXED, KU>(ob, s, a);
     else if (tid == 0) s.misc[M_CHISQ] = 0;
     for (int e = tid; e < mf * mf; e += NT) M[e] = 0;
     for (int j = tid; j < mf; j += NT) bv[j] = 0;
@@ -1678,14 +1563,11 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
 #pragma unroll
     for (int u = 0; u < kAccPerThread; u++) accA[u] = 0.f;
     int tiles_since_flush = 0;
-    const float *dsphF = nullptr;
-    if constexpr (!kFP64) dsphF = s.dsph ? s.dsph : ob.dsph_f;
+    const float *dsphF = s.dsph ? s.dsph : ob.dsph_f;
     // Point set-up threads.  An FP64 instruction holds its sub-partition's
     // FP64 unit for the whole warp however few lanes are active, so the
-    // set-up keeps its points on as few warps as possible: the mixed form
-    // (FP64 only for the rotation phase) on one warp, lane = point; the FP64
-    // form on warps 0..3, one per sub-partition.  On the tensor-core path
-    // warp 1 sets up the evaluation's first tile here; later tiles are set
+    // set-up keeps its points on one warp, lane = point (FP64 only for the
+    // rotation phase).  On the tensor-core path warp 1 sets up the evaluation's first tile here; later tiles are set
     // up in the contraction window of the tile before (warps 1..3).
     const int pipe_sp = warp == 1 ? lane : -1;
     if constexpr (kPipe) {
@@ -1714,11 +1596,8 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
                 // thread per point on as few warps as possible; with the
                 // tensor cores it was done during the previous tile's MMAs
                 if constexpr (!kPipe) {
-                    const int ppw = (P + 3) / 4;   // FP64 form: points per warp
-                    const int sp = kFP64 ? (lane < ppw && warp < 4 ? warp * ppw + lane : -1) : (warp == 0 ? lane : -1);
-                    if (sp >= 0 && sp < np)
-                        setup_point<FORM>(ob, cfg, start + t0 + sp, omg, s.bmat,
-                                          s.pt + sp * kPointStride);
+                    if (warp == 0 && lane < np)
+                        setup_point(ob, cfg, start + t0 + lane, omg, s.bmat, s.pt + lane * kPointStride);
                 }
                 // (with the tensor cores the set-up is a tile old: the
                 // barrier after the previous tile's contraction ordered it)
@@ -1754,9 +1633,6 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
                     }
                     facet_stage_tc<NT>(ob, s, np, cl, cls, wscale);
                 }
-                else if constexpr (kFP64) {
-                    for (int p = warp; p < np; p += NT / 32) facet_point_fp64(ob, s, p, wcols, cl, cls, fresh);
-                }
                 else
                 for (int p = warp; p < np; p += NT / 32) {
                     const R *pt = s.pt + p * kPointStride;
@@ -1777,7 +1653,7 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
                         R w = 0;
                         if (mu > R(kTinyMu) && mu0 > R(kTinyMu)) {
                             const R ar = s.areaR[i];
-                            const LitTerms<R, FORM> lt(mu, mu0, cl, cls);
+                            const LitTerms<R, PS_FORM_MIXED> lt(mu, mu0, cl, cls);
                             br = br + ar * lt.sv;
                             w = dareaR[i] * lt.sv * s.gvR[i];
                             const R s0 = nx * de[0] + ny * de[3] + nz * de[6];
@@ -1830,13 +1706,7 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
             // (the tensor-core issue below begins with a barrier of its own)
             if constexpr (!kPipe) __syncthreads();
             // 3. shape contraction and the remaining columns of J
-            if constexpr (kFP64) {
-                for (int o = tid; o < np * C; o += NT) {
-                    const int p = o / C, k = o - p * C;
-                    const double acc = contract_fp64(s, dsphR + k, p, C, F, wcols, conv);
-                    s.J[p * ma + k] = conv ? acc : s.pt[p * kPointStride + 24] * acc;
-                }
-            } else if constexpr (kPipe) {
+            if constexpr (kPipe) {
                 contract_tc_issue<NT, kWide>(s, F, tcs);   // the work below overlaps the MMAs
             } else {
                 if (s.dsph)
@@ -1958,24 +1828,11 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
                 if (!kPipe && tid < np) dst[static_cast<size_t>(tid) * RW + ma] = R(s.ym[tid]);
                 for (int l = kPipe ? tid - 64 : tid; l < ma; l += NT) {
                     if (l < 0) break;
-                    if constexpr (kFP64) {
-                        double d = s.dave[l];
-                        for (int p = 0; p < np; p++) d = d + s.J[p * ma + l];
-                        s.dave[l] = d;
-                    } else {
-                        float d = 0.f;
-                        for (int p = 0; p < np; p++) d += s.J[p * ma + l];
-                        s.dave[l] += static_cast<double>(d);
-                    }
+                    float d = 0.f;
+                    for (int p = 0; p < np; p++) d += s.J[p * ma + l];
+                    s.dave[l] += static_cast<double>(d);
                 }
-                if constexpr (kFP64) {
-                    // the reference's order
-                    if (tid == 0) {
-                        double av = s.misc[M_AVE];
-                        for (int p = 0; p < np; p++) av = av + s.ym[p];
-                        s.misc[M_AVE] = av;
-                    }
-                } else if (!kPipe && warp == 0) {
+                if (!kPipe && warp == 0) {
                     const double v = warp_sum(lane < np ? s.ym[lane] : 0.0);
                     if (lane == 0) s.misc[M_AVE] += v;
                 }
@@ -1990,28 +1847,23 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
                     tiles_since_flush = 0;
                 }
             } else {
-                accumulate_tile<FORM>(ob, s, M, bv, np, start + t0, conv, conv_sig, accA, accB);
-                if constexpr (!kFP64) {
-                    if (++tiles_since_flush == kTilesPerFlush) {
-                        flush_partials<FORM>(M, bv, mf, accA, accB);
-                        tiles_since_flush = 0;
-                    }
+                accumulate_tile(ob, s, np, start + t0, conv, conv_sig, accA, accB);
+                if (++tiles_since_flush == kTilesPerFlush) {
+                    flush_partials(M, bv, mf, accA, accB);
+                    tiles_since_flush = 0;
                 }
             }
         }
         if (!rel) continue;
         // ---- pass 2: renormalise and accumulate (mrqcof.c:90-136) ----
         const double ave = s.misc[M_AVE];
-        // the mixed form multiplies by one reciprocal of the lightcurve sum;
-        // the FP64 form divides as the reference does
-        // the mixed form's renormalisation runs in FP32 on FP32 copies, with
-        // one reciprocal of the lightcurve sum (computed once, not per warp)
-        if constexpr (!kFP64) {
-            for (int l = tid; l < ma; l += NT) s.davef[l] = static_cast<float>(s.dave[l]);
-            if (tid == 0) s.misc[M_INVAVE] = 1.0 / ave;
-            __syncthreads();
-        }
-        const double inv_ave = kFP64 ? 0.0 : s.misc[M_INVAVE];
+        // the renormalisation runs in FP32 on FP32 copies, with one
+        // reciprocal of the lightcurve sum (computed once, not per warp; the
+        // FP64 form divides as the reference does)
+        for (int l = tid; l < ma; l += NT) s.davef[l] = static_cast<float>(s.dave[l]);
+        if (tid == 0) s.misc[M_INVAVE] = 1.0 / ave;
+        __syncthreads();
+        const double inv_ave = s.misc[M_INVAVE];
         if constexpr (kTcAlpha) {
             // The per-point FP64 work of the whole lightcurve at once, one
             // tile per warp (the tiles' FP64 chains on different
@@ -2049,9 +1901,8 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
         for (int t0 = 0; t0 < npts; t0 += P) {
             const int np = min(P, npts - t0);
             const R *src = scratch + static_cast<size_t>(t0) * RW;
-            // model values of the tile in FP64 (the FP64 form keeps its own
-            // values; the mixed form parks them as FP32); on the tensor-core
-            // path they were prepared above, and the tile's residuals and
+            // model values of the tile in FP64 (parked as FP32); on the
+            // tensor-core path they were prepared above, and the tile's residuals and
             // weights go where the accumulation reads them
             if constexpr (kTcAlpha) {
                 // operands built from the parked rows (renormalised on the way)
@@ -2065,47 +1916,28 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
             if (tid < np) {
                 const int q = start + t0 + tid;
                 const double yt = static_cast<double>(src[static_cast<size_t>(tid) * RW + ma]);
-                double coef, ytr;
-                if constexpr (kFP64) {
-                    coef = ob.sig[q] * npts / ave;
-                    ytr = yt / ave;
-                } else {
-                    coef = ob.sig[q] * npts * inv_ave;
-                    ytr = yt * inv_ave;
-                }
+                const double coef = ob.sig[q] * npts * inv_ave, ytr = yt * inv_ave;
                 s.ym[tid] = coef * yt;
-                if constexpr (!kFP64) {
-                    s.accs[tid] = static_cast<float>(coef);        // consumed before the
-                    s.accs[32 + tid] = static_cast<float>(ytr);    // accumulation reuses it
-                }
+                s.accs[tid] = static_cast<float>(coef);        // consumed before the
+                s.accs[32 + tid] = static_cast<float>(ytr);    // accumulation reuses it
             }
             __syncthreads();
             for (int e = tid; e < np * ma; e += NT) {
                 const int p = e / ma, l = e - p * ma;
                 const R v = src[static_cast<size_t>(p) * RW + l];
-                R out;
-                if constexpr (kFP64) {
-                    const int q = start + t0 + p;
-                    const double coef = ob.sig[q] * npts / ave;
-                    const double yt = src[static_cast<size_t>(p) * RW + ma];
-                    out = coef * (v - yt * s.dave[l] / ave);
-                } else {
-                    out = s.accs[p] * (v - s.accs[32 + p] * s.davef[l]);
-                }
+                const R out = s.accs[p] * (v - s.accs[32 + p] * s.davef[l]);
                 s.J[e] = (l == 0) ? R(0) : out;
             }
             __syncthreads();
-            accumulate_tile<FORM>(ob, s, M, bv, np, start + t0, false, conv_sig, accA, accB);
-            if constexpr (!kFP64) {
-                if (++tiles_since_flush == kTilesPerFlush) {
-                    flush_partials<FORM>(M, bv, mf, accA, accB);
-                    tiles_since_flush = 0;
-                }
+            accumulate_tile(ob, s, np, start + t0, false, conv_sig, accA, accB);
+            if (++tiles_since_flush == kTilesPerFlush) {
+                flush_partials(M, bv, mf, accA, accB);
+                tiles_since_flush = 0;
             }
         }
     }
     if constexpr (kTcAlpha) tc_alpha_flush<NT>(ob, s, M, bv, tcs);
-    else if constexpr (!kFP64) flush_partials<FORM>(M, bv, mf, accA, accB);
+    else flush_partials(M, bv, mf, accA, accB);
     __syncthreads();
     // mirror the lower triangle (mrqcof.c:139-141)
     for (int e = tid; e < mf * mf; e += NT) {
@@ -2116,135 +1948,279 @@ __device__ void evaluate(const DevObject &ob, const FitConfig &cfg, const SlotLa
 }
 
 // ---------------------------------------------------------------------------
-// FP64 evaluation split over a thread-block cluster (kMaxSplit CTAs at most).
+// FP64 form's model evaluation (mrqcof), by one CTA or (SPLIT) by the CTAs of
+// a thread-block cluster.  Bound by the FP64 units: a warp's FP64 instruction
+// holds its sub-partition's unit for 64 cycles however few lanes are active,
+// so every stage keeps its lanes full and its warps spread evenly over the
+// four sub-partitions, and what is the same for a point is computed once.
 //
-// One fit's point tiles are dealt round-robin to the cluster's CTAs, which
-// compute their tiles' model rows (point set-up, facet stage, shape
-// contraction, the remaining columns) at the same time; after each round
-// every CTA takes the round's tiles in data order -- its own from its shared
-// memory, the others' through distributed shared memory -- and runs what
-// sums over points: the relative lightcurves' sums, parked rows and second
-// pass, and chi^2 in full, the normal matrix and beta for its share of the
-// elements only.  Every sum therefore runs in the same order as in the
-// single-CTA FP64 form, and the split fit is bit-identical to it.  Every
-// CTA computes the convexity rows; then each copies its share of the matrix
-// into the others, so that all of them take the same LM decisions and keep
-// the same control flow (and the same sequence of cluster barriers).
+// SPLIT: one fit's point tiles are dealt round-robin to the cluster's CTAs,
+// which compute their tiles' model rows (tile_rows_fp64) at the same time;
+// after each round every CTA takes the round's tiles in data order -- its own
+// from its shared memory, the others' through distributed shared memory --
+// and runs what sums over points: the relative lightcurves' sums, parked rows
+// and second pass, and chi^2 in full, the normal matrix and beta for its
+// share of the elements only.  Every sum therefore runs in the same order as
+// with one CTA, and the split fit is bit-identical to it.  Every CTA computes
+// the convexity rows; then each copies its share of the matrix into the
+// others, so that all of them take the same LM decisions and keep the same
+// control flow (and the same sequence of cluster barriers).
+//
+// Measured (980 points, 288 facets): one evaluation 4.97 -> 4.33 ms, 400 fits
+// 577 -> 548 ms with the set-up in twelve parts, the dot products, residuals
+// and renormalisation factors once per point, the contraction's points in
+// order of their lit counts and beta's elements among alpha's units.  Of an
+// evaluation's 8.8 Mcycles the FP64 instructions take 7.7 on full units
+// (contraction 3.3, facet law 3.0, alpha 0.8).
 // ---------------------------------------------------------------------------
 constexpr int kMaxSplit = 8;
+constexpr int kWarpsFp64 = threads_of<PS_FORM_FP64>() / 32;
 
-__device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<PS_FORM_FP64> &s,
-                               const double *a, double *M, double *bv, double *scratch, bool fresh)
+// First part of the set-up (setup_phase_fp64) of the CTA's next kWarpsFp64
+// tiles, warp w the w-th, a point per lane: with one tile at a time the
+// set-up ran on 8 lanes of 4 warps (28 of a tile's 320 kcycles; 7 now, with
+// the second part).  (lc, t0): the first of these tiles; step: tiles from one
+// of the CTA's tiles to its next.
+__device__ inline void setup_group_fp64(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L,
+                                        Smem<PS_FORM_FP64> &s, int lc, int t0, int step, double omg)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int skip = warp * step;
+    while (lc < ob.n_lc - 1) {
+        const int nt = (ob.lc_npts[lc] - t0 + L.P - 1) / L.P;
+        if (skip < nt) break;
+        skip -= nt;
+        lc++;
+        t0 = 0;
+    }
+    if (lc < ob.n_lc - 1) {
+        t0 += skip * L.P;
+        if (lane < min(L.P, ob.lc_npts[lc] - t0))
+            setup_phase_fp64(ob, cfg, ob.lc_start[lc] + t0 + lane, omg, s.bmat, s.phase + warp * L.P + lane,
+                             kWarpsFp64 * L.P);
+    }
+    __syncthreads();
+}
+
+// Model rows of one tile of np points from q0 on into s.J / s.ym
+// (bright.c:14-126), its first set-up part in slot `slot` of s.phase; conv:
+// the convexity rows (conv.c:12-29).  Leaves with a barrier.
+__device__ void tile_rows_fp64(const DevObject &ob, const SlotLayout &L, Smem<PS_FORM_FP64> &s, int q0, int np,
+                               bool conv, int slot, bool count)
+{
+    constexpr int NW = kWarpsFp64;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int F = ob.nfac, C = ob.ncoef, ma = ob.ma, wcols = L.wcols;
+    const double cls = s.bmat[30], cl = s.bmat[31];
+    if (!conv) {
+        // second part of the set-up: twelve parts, a warp each
+        static_assert(NW == 12, "twelve set-up parts");
+        const int part = warp & 3, i = warp >> 2;
+        if (lane < np) {
+            const double *ph = s.phase + slot * L.P + lane;
+            double *pt = s.pt + lane * kPointStride;
+            setup_row_fp64(ob, q0 + lane, part, i, s.bmat, ph, NW * L.P, pt);
+            if (part == 3 && i == 2) {
+                const double alpha = ob.alpha_pt[q0 + lane], ex = ph[2 * NW * L.P];
+                pt[24] = phase_scale_fp64(s.bmat[27], s.bmat[29], ex, alpha);
+                pt[25] = ex;
+                pt[26] = ph[3 * NW * L.P];
+                pt[27] = alpha;
+            }
+        }
+        __syncthreads();
+        for (int p = warp; p < np; p += NW) facet_point_fp64(ob, s, p, wcols, cl, cls, count);
+    } else {
+        for (int p = warp; p < np; p += NW) {
+            const double *nc = (p == 0) ? ob.nx : (p == 1) ? ob.ny : ob.nz;
+            double res = 0;
+            double *Wp = s.W + static_cast<size_t>(p) * wcols;
+            for (int i = lane; i < F; i += 32) {
+                res = res + s.area[i] * nc[i];
+                Wp[i] = ob.darea[i] * s.gv[i] * nc[i];
+            }
+            res = warp_sum(res);
+            if (lane == 0) s.red[p * kRedStride] = res;
+        }
+    }
+    __syncthreads();
+    // Contraction: outputs (point, coefficient) in units of 32 lanes.  A lane
+    // runs as long as its point's lit list, a unit as long as its longest, so
+    // the points are taken in order of their counts (each warp orders them
+    // itself): a unit's points then have nearly the same count.
+    unsigned char *ord = s.order + warp * 32;
+    {
+        const int n = lane < np ? (conv ? F : s.nlit[lane]) : -1;
+        int r = 0;
+#pragma unroll
+        for (int o = 0; o < 32; o++) {
+            const int m = __shfl_sync(0xffffffffu, n, o);
+            r += (m > n || (m == n && o < lane)) ? 1 : 0;
+        }
+        ord[r] = static_cast<unsigned char>(lane);
+        __syncwarp();
+    }
+    for (int o = tid; o < np * C; o += NW * 32) {
+        const int r = o / C, k = o - r * C, p = ord[r];
+        const double acc = contract_fp64(s, ob.dsph + k, p, C, F, wcols, conv);
+        s.J[p * ma + k] = conv ? acc : s.pt[p * kPointStride + 24] * acc;
+    }
+    // the remaining columns, a point per lane of the last warp (which has the
+    // fewest units): D_k . U + E_k . V with D_k = (de[k], de[3 + k], de[6 + k])
+    // and E_k likewise from de0
+    if (warp == NW - 1 && lane < np) {
+        const int p = lane;
+        double *Jp = s.J + p * ma;
+        const double *rd = s.red + p * kRedStride;
+        if (!conv) {
+            const double *pt = s.pt + p * kPointStride, *de = pt + 6, *de0 = pt + 15;
+            const double scale = pt[24];
+            const double br = rd[0];
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                double v = fma(de[k], rd[1], __dmul_rn(de[3 + k], rd[2]));
+                v = fma(de[6 + k], rd[3], v);
+                v = fma(de0[k], rd[4], v);
+                v = fma(de0[3 + k], rd[5], v);
+                v = fma(de0[6 + k], rd[6], v);
+                Jp[C + k] = scale * v;
+            }
+            Jp[C + 3] = br * pt[25];
+            Jp[C + 4] = br * pt[26];
+            Jp[C + 5] = br * pt[27];
+            Jp[C + 6] = scale * rd[7] * cl;
+            Jp[C + 7] = scale * rd[8];
+            s.ym[p] = br * scale;
+        } else {
+            for (int k = C; k < ma; k++) Jp[k] = 0;
+            s.ym[p] = rd[0];
+            s.misc[M_CHK + p] = rd[0];
+        }
+    }
+    __syncthreads();
+}
+
+// Elements of the normal matrix's lower triangle, then of beta, in units of
+// 32 lanes dealt to the cluster's CTAs and then to a CTA's warps: calls
+// fn(e) for the calling thread's elements e.
+template <class Fn>
+__device__ inline void for_share(int n, int rank, int cs, Fn fn)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int u = warp * cs + rank; u * 32 < n; u += kWarpsFp64 * cs) {
+        const int e = u * 32 + lane;
+        if (e < n) fn(e);
+    }
+}
+
+// Accumulates the rows Jrows[0..np) (model values ymv) of one tile into the
+// normal matrix M (lower triangle), bv and chi^2 (mrqcof.c:106-136), every
+// element over the points in data order; of M and bv the CTA's share, chi^2
+// whole.  Residuals once per point; beta's elements are units like alpha's.
+__device__ void accumulate_tile_fp64(const DevObject &ob, Smem<PS_FORM_FP64> &s, double *M, double *bv, int np,
+                                     int q0, bool conv, double conv_sig, const double *Jrows, const double *ymv,
+                                     int rank, int cs)
+{
+    constexpr int NT = threads_of<PS_FORM_FP64>();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ma = ob.ma, mf = ob.mfit;
+    double *wt = s.W;   // [np][mf], reuses the facet-weight tile
+    double *dyv = s.resid, *tv = dyv + 32;
+    const double conv_s2 = conv ? 1 / (conv_sig * conv_sig) : 0.0;
+    if (warp == kWarpsFp64 - 1 && lane < np) {
+        const double dy = (conv ? 0.0 : ob.bright[q0 + lane]) - ymv[lane];
+        dyv[lane] = dy;
+        tv[lane] = dy * dy * (conv ? conv_s2 : ob.sig2i[q0 + lane]);
+    }
+    for (int e = tid; e < np * mf; e += NT) {
+        const int p = e / mf, j = e - p * mf;
+        const double sig2i = conv ? conv_s2 : ob.sig2i[q0 + p];
+        wt[p * mf + j] = Jrows[p * ma + ob.free_list[j]] * sig2i * ob.weight[q0 + p];
+    }
+    __syncthreads();
+    if (tid == NT - 1) {
+        double c2 = s.misc[M_CHISQ];
+#pragma unroll 4
+        for (int p = 0; p < np; p++) c2 = fma(tv[p], ob.weight[q0 + p], c2);
+        s.misc[M_CHISQ] = c2;
+    }
+    const int ntri = mf * (mf + 1) / 2;
+    for_share(ntri + mf, rank, cs, [&](int e) {
+        const double *x, *y;
+        double *to;
+        int ys;
+        if (e < ntri) {
+            const int j = tri_row(e), k = e - j * (j + 1) / 2;
+            x = wt + j;
+            y = Jrows + ob.free_list[k];
+            ys = ma;
+            to = M + j * mf + k;
+        } else {
+            x = wt + (e - ntri);
+            y = dyv;
+            ys = 1;
+            to = bv + (e - ntri);
+        }
+        double acc = *to;
+#pragma unroll 4
+        for (int p = 0; p < np; p++) acc = fma(x[p * mf], y[p * ys], acc);
+        *to = acc;
+    });
+    __syncthreads();
+}
+
+template <bool SPLIT>
+__device__ void evaluate_fp64(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<PS_FORM_FP64> &s,
+                              const double *a, double *M, double *bv, double *scratch, bool fresh)
 {
     namespace cgr = cooperative_groups;
-    constexpr int NT = threads_of<PS_FORM_FP64>();
-    cgr::cluster_group cl = cgr::this_cluster();
-    const int rank = static_cast<int>(cl.block_rank()), cs = static_cast<int>(cl.num_blocks());
+    constexpr int NT = threads_of<PS_FORM_FP64>(), NW = NT / 32;
+    int rank = 0, cs = 1;
+    if constexpr (SPLIT) {
+        rank = static_cast<int>(cgr::this_cluster().block_rank());
+        cs = static_cast<int>(cgr::this_cluster().num_blocks());
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int F = ob.nfac, C = ob.ncoef, ma = ob.ma, mf = ob.mfit, P = L.P;
-    const int wcols = L.wcols;
+    const int C = ob.ncoef, ma = ob.ma, mf = ob.mfit, P = L.P;
     const int RW = rel_row_stride(ma);
+    const int ntri = mf * (mf + 1) / 2;
 
-    // curv.c:10-39 and blmatrix.c:9-46 on every CTA (as in evaluate)
     if (fresh) shape_prologue<PS_FORM_FP64, 1>(ob, s, a);
     else if (tid == 0) s.misc[M_CHISQ] = 0;
     for (int e = tid; e < mf * mf; e += NT) M[e] = 0;
     for (int j = tid; j < mf; j += NT) bv[j] = 0;
     const double omg = a[C + 2];
     __syncthreads();
-    const double cls = s.bmat[30], cl_w = s.bmat[31];
     const double conv_sig = cfg.conv_sig;
-    float accA[kAccPerThread];
-    float accB = 0.f;
 
-    // model rows of one tile into s.J / s.ym (bright.c:14-126, as in evaluate)
-    auto compute_tile = [&](int lc, int t0, int np, bool conv) {
-        const int start = ob.lc_start[lc];
-        if (!conv) {
-            const int ppw = (P + 3) / 4;
-            const int sp = (lane < ppw && warp < 4) ? warp * ppw + lane : -1;
-            if (sp >= 0 && sp < np)
-                setup_point<PS_FORM_FP64>(ob, cfg, start + t0 + sp, omg, s.bmat, s.pt + sp * kPointStride);
-            __syncthreads();
-            for (int p = warp; p < np; p += NT / 32) facet_point_fp64(ob, s, p, wcols, cl_w, cls, fresh);
-        } else {
-            for (int p = warp; p < np; p += NT / 32) {
-                const double *nc = (p == 0) ? ob.nx : (p == 1) ? ob.ny : ob.nz;
-                double res = 0;
-                double *Wp = s.W + static_cast<size_t>(p) * wcols;
-                for (int i = lane; i < F; i += 32) {
-                    res = res + s.area[i] * nc[i];
-                    Wp[i] = ob.darea[i] * s.gv[i] * nc[i];
-                }
-                res = warp_sum(res);
-                if (lane == 0) s.red[p * kRedStride] = res;
-            }
-        }
-        __syncthreads();
-        for (int o = tid; o < np * C; o += NT) {
-            const int p = o / C, k = o - p * C;
-            const double acc = contract_fp64(s, ob.dsph + k, p, C, F, wcols, conv);
-            s.J[p * ma + k] = conv ? acc : s.pt[p * kPointStride + 24] * acc;
-        }
-        if (tid < np) {
-            const int p = tid;
-            double *Jp = s.J + p * ma;
-            const double *rd = s.red + p * kRedStride;
-            if (!conv) {
-                const double *pt = s.pt + p * kPointStride;
-                const double scale = pt[24];
-                const double br = rd[0];
-                Jp[C] = scale * rd[1];
-                Jp[C + 1] = scale * rd[2];
-                Jp[C + 2] = scale * rd[3];
-                Jp[C + 3] = br * pt[25];
-                Jp[C + 4] = br * pt[26];
-                Jp[C + 5] = br * pt[27];
-                Jp[C + 6] = scale * rd[4] * cl_w;
-                Jp[C + 7] = scale * rd[5];
-                s.ym[p] = br * scale;
-            } else {
-                for (int k = C; k < ma; k++) Jp[k] = 0;
-                s.ym[p] = rd[0];
-                s.misc[M_CHK + p] = rd[0];
-            }
-        }
-        __syncthreads();
-    };
-
-    // A tile's sums (mrqcof.c:51-136), over points in data order, on every
-    // CTA: the relative lightcurves' sums and rows and chi^2 in full, of the
-    // normal matrix only the CTA's share of the elements (accumulate_tile's
-    // part).  Jt, yt: the tile's rows and model values (the CTA's own tile,
-    // or another CTA's staged in Jst/ymst); the second pass stages its
-    // renormalised rows there too, so that s.J, which the other CTAs read
-    // during the round, stays as computed.
+    // A tile's sums (mrqcof.c:51-136).  Jt, yt: the tile's rows and model
+    // values (the CTA's own tile, or another CTA's staged in Jst/ymst); the
+    // second pass stages its renormalised rows there too, so that s.J, which
+    // the other CTAs read during the round, stays as computed.
     double *Jst = s.W + static_cast<size_t>(P) * mf, *ymst = Jst + static_cast<size_t>(P) * ma;
+    double *coefv = s.resid + 64;
     auto consume_tile = [&](int lc, int t0, int np, const double *Jt, const double *yt) {
         const int start = ob.lc_start[lc], npts = ob.lc_npts[lc];
         if (!ob.lc_rel[lc]) {
-            accumulate_tile<PS_FORM_FP64>(ob, s, M, bv, np, start + t0, false, conv_sig, accA, accB, Jt, yt, rank,
-                                          cs);
+            accumulate_tile_fp64(ob, s, M, bv, np, start + t0, false, conv_sig, Jt, yt, rank, cs);
             return;
-        }
-        if (t0 == 0) {
-            for (int l = tid; l < ma; l += NT) s.dave[l] = 0;
-            if (tid == 0) s.misc[M_AVE] = 0;
-            __syncthreads();
         }
         double *dst = scratch + static_cast<size_t>(t0) * RW;
         for (int e = tid; e < np * ma; e += NT) {
-            int p = e / ma, l = e - p * ma;
+            const int p = e / ma, l = e - p * ma;
             dst[static_cast<size_t>(p) * RW + l] = Jt[e];
         }
         if (tid < np) dst[static_cast<size_t>(tid) * RW + ma] = yt[tid];
         for (int l = tid; l < ma; l += NT) {
-            double d = s.dave[l];
+            double d = t0 == 0 ? 0.0 : s.dave[l];
+#pragma unroll 8
             for (int p = 0; p < np; p++) d = d + Jt[p * ma + l];
             s.dave[l] = d;
         }
-        if (tid == 0) {
-            double av = s.misc[M_AVE];
+        // the reference's order (on a warp without column sums, C <= 121)
+        if (tid == NT - 1) {
+            double av = t0 == 0 ? 0.0 : s.misc[M_AVE];
+#pragma unroll 8
             for (int p = 0; p < np; p++) av = av + yt[p];
             s.misc[M_AVE] = av;
         }
@@ -2255,47 +2231,47 @@ __device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const 
         for (int u0 = 0; u0 < npts; u0 += P) {
             const int nq = min(P, npts - u0);
             const double *src = scratch + static_cast<size_t>(u0) * RW;
-            if (tid < nq) {
-                const int q = start + u0 + tid;
-                const double ytv = src[static_cast<size_t>(tid) * RW + ma];
-                const double coef = ob.sig[q] * npts / ave;
-                ymst[tid] = coef * ytv;
+            if (warp == NW - 1 && lane < nq) {
+                const double coef = ob.sig[start + u0 + lane] * npts / ave;
+                coefv[lane] = coef;
+                ymst[lane] = coef * src[static_cast<size_t>(lane) * RW + ma];
             }
+            // every element's quotient first, the point's factor after the barrier
             for (int e = tid; e < nq * ma; e += NT) {
                 const int p = e / ma, l = e - p * ma;
                 const double v = src[static_cast<size_t>(p) * RW + l];
-                const int q = start + u0 + p;
-                const double coef = ob.sig[q] * npts / ave;
                 const double ytv = src[static_cast<size_t>(p) * RW + ma];
-                const double out = coef * (v - ytv * s.dave[l] / ave);
-                Jst[e] = (l == 0) ? 0.0 : out;
+                Jst[e] = l == 0 ? 0.0 : v - ytv * s.dave[l] / ave;
             }
             __syncthreads();
-            accumulate_tile<PS_FORM_FP64>(ob, s, M, bv, nq, start + u0, false, conv_sig, accA, accB, Jst, ymst, rank,
-                                          cs);
+            for (int e = tid; e < nq * ma; e += NT) Jst[e] = coefv[e / ma] * Jst[e];
+            __syncthreads();
+            accumulate_tile_fp64(ob, s, M, bv, nq, start + u0, false, conv_sig, Jst, ymst, rank, cs);
         }
     };
 
     // rounds of cs tiles over the real lightcurves, in data order
-    int rlc[kMaxSplit], rt0[kMaxSplit], rnp[kMaxSplit];
-    int nround = 0;
+    int rlc[SPLIT ? kMaxSplit : 1], rt0[SPLIT ? kMaxSplit : 1], rnp[SPLIT ? kMaxSplit : 1];
+    int nround = 0, slot = NW;
     auto flush_round = [&]() {
-        cl.sync();   // every CTA's tile of the round is in its shared memory
+        if constexpr (SPLIT) cgr::this_cluster().sync();   // every CTA's tile of the round is in its shared memory
         for (int k = 0; k < nround; k++) {
             const double *Jt = s.J, *yt = s.ym;
-            if (k != rank) {
-                // rank k's tile, read through distributed shared memory
-                const double *rJ = cl.map_shared_rank(s.J, k);
-                const double *rY = cl.map_shared_rank(s.ym, k);
-                for (int e = tid; e < rnp[k] * ma; e += NT) Jst[e] = rJ[e];
-                if (tid < rnp[k]) ymst[tid] = rY[tid];
-                __syncthreads();
-                Jt = Jst;
-                yt = ymst;
+            if constexpr (SPLIT) {
+                if (k != rank) {
+                    // rank k's tile, read through distributed shared memory
+                    const double *rJ = cgr::this_cluster().map_shared_rank(s.J, k);
+                    const double *rY = cgr::this_cluster().map_shared_rank(s.ym, k);
+                    for (int e = tid; e < rnp[k] * ma; e += NT) Jst[e] = rJ[e];
+                    if (tid < rnp[k]) ymst[tid] = rY[tid];
+                    __syncthreads();
+                    Jt = Jst;
+                    yt = ymst;
+                }
             }
             consume_tile(rlc[k], rt0[k], rnp[k], Jt, yt);
         }
-        cl.sync();   // the round's tile buffers are free again
+        if constexpr (SPLIT) cgr::this_cluster().sync();   // the round's tile buffers are free again
         nround = 0;
     };
     const int nreal = ob.n_lc - 1;
@@ -2306,7 +2282,14 @@ __device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const 
             rlc[nround] = lc;
             rt0[nround] = t0;
             rnp[nround] = np;
-            if (nround == rank) compute_tile(lc, t0, np, false);
+            if (nround == rank) {
+                if (slot == NW) {
+                    setup_group_fp64(ob, cfg, L, s, lc, t0, cs, omg);
+                    slot = 0;
+                }
+                tile_rows_fp64(ob, L, s, ob.lc_start[lc] + t0, np, false, slot, fresh);
+                slot++;
+            }
             if (++nround == cs) flush_round();
         }
     }
@@ -2316,27 +2299,28 @@ __device__ void evaluate_split(const DevObject &ob, const FitConfig &cfg, const 
         const int lc = ob.n_lc - 1, start = ob.lc_start[lc], npts = ob.lc_npts[lc];
         for (int t0 = 0; t0 < npts; t0 += P) {
             const int np = min(P, npts - t0);
-            compute_tile(lc, t0, np, true);
-            accumulate_tile<PS_FORM_FP64>(ob, s, M, bv, np, start + t0, true, conv_sig, accA, accB, s.J, s.ym, rank,
-                                          cs);
+            tile_rows_fp64(ob, L, s, start + t0, np, true, 0, false);
+            accumulate_tile_fp64(ob, s, M, bv, np, start + t0, true, conv_sig, s.J, s.ym, rank, cs);
         }
     }
     // every CTA copies its share of the lower triangle and of bv into the
     // others, then mirrors (mrqcof.c:139-141): the same matrix, solve and
     // decisions everywhere
-    {
-        const int ntri = mf * (mf + 1) / 2;
+    if constexpr (SPLIT) {
         for (int r = 0; r < cs; r++) {
             if (r == rank) continue;
-            double *rM = cl.map_shared_rank(M, r), *rb = cl.map_shared_rank(bv, r);
-            for (int e = rank * NT + tid; e < ntri; e += cs * NT) {
-                const int j = tri_row(e), k = e - j * (j + 1) / 2;
-                rM[j * mf + k] = M[j * mf + k];
-            }
-            for (int j = rank * NT + tid; j < mf; j += cs * NT) rb[j] = bv[j];
+            double *rM = cgr::this_cluster().map_shared_rank(M, r), *rb = cgr::this_cluster().map_shared_rank(bv, r);
+            for_share(ntri + mf, rank, cs, [&](int e) {
+                if (e < ntri) {
+                    const int j = tri_row(e), k = e - j * (j + 1) / 2;
+                    rM[j * mf + k] = M[j * mf + k];
+                } else {
+                    rb[e - ntri] = bv[e - ntri];
+                }
+            });
         }
+        cgr::this_cluster().sync();
     }
-    cl.sync();
     for (int e = tid; e < mf * mf; e += NT) {
         const int j = e / mf, k = e - j * mf;
         if (k > j) M[e] = M[k * mf + j];
@@ -3119,16 +3103,15 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
 {
     constexpr bool kTensor = FORM == PS_FORM_MIXED && (KU == 0 || KU == 3);
     // one model evaluation; with split (FP64 form, cluster launch) spread
-    // over the cluster's CTAs (evaluate_split).  fresh = false: chi2 has just
+    // over the cluster's CTAs.  fresh = false: chi2 has just
     // run at the same parameters.
     auto eval = [&](const double *a, double *M, double *bv, bool fresh) {
         if constexpr (FORM == PS_FORM_FP64) {
-            if (split) {
-                evaluate_split(ob, cfg, L, s, a, M, bv, scratch, fresh);
-                return;
-            }
+            if (split) evaluate_fp64<true>(ob, cfg, L, s, a, M, bv, scratch, fresh);
+            else evaluate_fp64<false>(ob, cfg, L, s, a, M, bv, scratch, fresh);
+        } else {
+            evaluate_mixed<KU>(ob, cfg, L, s, a, M, bv, scratch, tcs, fresh);
         }
-        evaluate<FORM, KU>(ob, cfg, L, s, a, M, bv, scratch, tcs, fresh);
     };
     // chi^2 alone where the form has it (about half of the steps are
     // rejected, and need no more)
@@ -3444,7 +3427,7 @@ __global__ void __launch_bounds__(threads_of<FORM>(), 1)
     if (FORM == PS_FORM_FP64 && threadIdx.x == 0 && w.lit) atomicAdd(w.lit, *lit_counter(s.misc));
 }
 
-// FP64 fits, each spread over a thread-block cluster (evaluate_split): the
+// FP64 fits, each spread over a thread-block cluster (evaluate_fp64): the
 // cluster's leader takes fits from the work counter and hands every fit to
 // all of the cluster's CTAs, which run the same LM loop together; the
 // leader writes the result.  Bit-identical to fit_kernel<FP64>.
@@ -3506,7 +3489,8 @@ __global__ void __launch_bounds__(threads_of<FORM>(), 1) eval_kernel(DevObject o
     if (L.dsph_smem == kBasisTensorWide) s.alpha = alpha;
     __syncthreads();
     R *rows = L.rels ? reinterpret_cast<R *>(smem + L.rels) : reinterpret_cast<R *>(scratch);
-    evaluate<FORM, KU>(ob, cfg, L, s, s.cg, s.alpha, s.beta, rows, tcs);
+    if constexpr (FORM == PS_FORM_FP64) evaluate_fp64<false>(ob, cfg, L, s, s.cg, s.alpha, s.beta, rows, true);
+    else evaluate_mixed<KU>(ob, cfg, L, s, s.cg, s.alpha, s.beta, rows, tcs);
     if constexpr (kTensor) {
         const bool aborted = *s.abort != 0;
         tc_teardown(s, tcs, ob.nfac);
