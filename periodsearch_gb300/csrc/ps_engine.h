@@ -161,6 +161,12 @@ PSG_HD constexpr int rel_row_stride(int ma) { return ma + 3; }
 PSG_HD constexpr int tc_kpad(int nfac) { return (nfac + 31) & ~31; }
 
 
+// Workspace of the Gauss-Jordan solve of n equations: the scaled pivot row,
+// the pivot column and the right-hand side's entry; two column lists, the
+// pivoted flags and a candidate per warp.
+PSG_HD constexpr size_t gj_doubles(int n) { return 2 * static_cast<size_t>(n) + 1; }
+PSG_HD constexpr size_t gj_ints(int n) { return 3 * static_cast<size_t>(n) + 16; }
+
 // dsph_smem: the mixed form keeps the FP32 basis Dsph[F][C] in shared memory
 // for the whole launch (it is read once per point tile by every warp).
 // rel_rows > 0: the rows of relative lightcurves (up to rel_rows points)
@@ -205,9 +211,9 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     L.ym = take(P * d);
     L.red = take(static_cast<size_t>(P) * kRedStride * d);
     L.dave = take(ma * d);
-    L.col = take((mfit + 1) * d);
+    L.col = take(gj_doubles(mfit) * d);
     L.misc = take(kMisc * d);
-    L.ipiv = take(sizeof(int) * static_cast<size_t>(mfit + 2 + 16));
+    L.ipiv = take(sizeof(int) * gj_ints(mfit));
     L.dsph = dsph_smem == kBasisSmem ? take(static_cast<size_t>(nfac) * ncoef * sizeof(float)) : 0;
     if (basis_on_tensor(dsph_smem)) {
         const bool wide = dsph_smem == kBasisTensorWide;
