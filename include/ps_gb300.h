@@ -162,7 +162,7 @@ typedef struct ps_timing {
     int64_t fits;          /* fits computed */
     int64_t evals;         /* model evaluations (mrqcof calls) */
     int32_t launches;      /* kernel launches */
-    int32_t cluster_size;  /* CTAs per fit of the last launch: 1, or 2..4 when FP64 fits were each spread over a
+    int32_t cluster_size;  /* CTAs per fit of the last launch: 1, or 2..16 when FP64 fits were each spread over a
                               thread-block cluster (fewer fits than fit slots; bit-identical results) */
     int64_t lit_facets;    /* FP64 form: (point, facet) pairs on the lit side over all evaluations, the work of
                               the facet law and of the shape contraction (bright.c runs both on lit facets

@@ -30,6 +30,7 @@ struct FormPlan {
     int P = 16, dsph_smem = 0, slots = 0;
     int rel_rows = 0;   // relative-lightcurve rows parked in shared memory (0: global scratch)
     size_t smem = 0;
+    int clusters[psg::kMaxClusterCtas + 1] = {};   // FP64 form: clusters of k CTAs the device runs at once, 0: not asked yet
 };
 
 struct ps_ctx {
@@ -231,16 +232,44 @@ ps_status make_plan(ps_ctx *c, int form)
     return PS_ERR_LIMIT;
 }
 
+// Clusters of cs CTAs of the split FP64 kernel that the device runs at once
+// (0 where it runs none), asked of the runtime once per plan.
+int clusters_of(FormPlan &pl, int cs)
+{
+    int &n = pl.clusters[cs];
+    if (n == 0 && (psg::split_max_clusters(cs, pl.smem, &n) != 0 || n < 1)) n = -1;
+    return std::max(n, 0);
+}
+
+// Point tiles of the object's real lightcurves.
+int64_t tiles_of(const ps_ctx *c, int P)
+{
+    int64_t t = 0;
+    for (int i = 0; i < c->obj.n_lc; i++) t += (c->obj.lc_points[i] + P - 1) / P;
+    return t;
+}
+
 // CTAs per fit for a launch: FP64 fits without trajectories, saved states
 // or an iteration limit, fewer than the fit slots, are each spread over a
-// thread-block cluster of 2 or 4 CTAs (the most that the slots hold).
-int split_size(const ps_ctx *c, const psg::FitWork &w, int form)
+// thread-block cluster: of 2 or 4 CTAs where the slots hold them, and of as
+// many (up to 16, not more than the object has tiles) as still leave every
+// fit a cluster that is resident at once.  A cluster lies within one GPC, so
+// there are fewer than slots / cs of the larger ones (36 of 4, 13 of 10, 7 of
+// 16 CTAs on 152 SMs), and a second round of fits costs more than a larger
+// cluster gains.  Measured on 980 points, 288 facets (32 tiles), one launch in ms
+// by CTAs per fit: 175 (1), 105 (2), 76 (3), 62 (4), 54 (5), 49 (6), 39 (9 and
+// 10), 35 (12), 31 (16); 200 points (7 tiles): 40 (1), 27 (2), 20 (4), 17 (6),
+// 16 (7).
+int split_size(ps_ctx *c, const psg::FitWork &w, int form)
 {
     if (form != PS_FORM_FP64 || w.traj || w.state || w.iter_limit > 0 || w.nfits < 1) return 1;
-    const int64_t slots = c->plan[form].slots;
-    if (w.nfits * 4 <= slots) return 4;
-    if (w.nfits * 2 <= slots) return 2;
-    return 1;
+    FormPlan &pl = c->plan[form];
+    const int64_t slots = pl.slots;
+    int cs = w.nfits * 4 <= slots ? 4 : w.nfits * 2 <= slots ? 2 : 1;
+    const int most = static_cast<int>(std::min<int64_t>(psg::kMaxClusterCtas, tiles_of(c, pl.P)));
+    for (int k = most; k > cs && cs > 1; k--)
+        if (clusters_of(pl, k) >= w.nfits) cs = k;
+    return cs;
 }
 
 // Launches the fits described by w in the given form (queue and outputs
@@ -249,7 +278,7 @@ ps_status run_fits(ps_ctx *c, double conw_r, psg::FitWork w, int form)
 {
     ps_status st = make_plan(c, form);
     if (st != PS_OK) return st;
-    const FormPlan &pl = c->plan[form];
+    FormPlan &pl = c->plan[form];
     if (pl.slots > c->slots) {
         // a second form with more slots than the scratch was sized for
         cudaFree(c->d_scratch);
@@ -287,10 +316,7 @@ ps_status run_fits(ps_ctx *c, double conw_r, psg::FitWork w, int form)
     PSG_CUDA(c, cudaEventRecord(c->ev[0], c->stream));
     int e;
     if (cs > 1) {
-        int clusters = 0;
-        e = psg::split_max_clusters(cs, pl.smem, &clusters);
-        if (e != 0) return cuda_fail(c, static_cast<cudaError_t>(e), "cluster occupancy");
-        clusters = static_cast<int>(std::min<int64_t>(std::max(clusters, 1), w.nfits));
+        const int clusters = static_cast<int>(std::min<int64_t>(std::max(clusters_of(pl, cs), 1), w.nfits));
         e = psg::launch_fits_split(c->dob, cfg, w, clusters, cs, pl.P, pl.smem, c->stream);
     } else {
         e = psg::launch_fits(form, c->dob, cfg, w, grid, pl.P, pl.smem, pl.dsph_smem, c->stream);
@@ -888,8 +914,17 @@ ps_status ps_eval(ps_ctx *c, double conw_r, const double *cg, double *alpha, dou
            *d_ar = d_c2 + 1;
     PSG_CUDA(c, cudaMemcpyAsync(d_cg, cg, ma * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     psg::FitConfig cfg = make_config(c, conw_r);
-    int e = psg::launch_eval(c->opt.form, c->dob, cfg, d_cg, d_al, d_be, d_c2, d_ar, c->d_scratch, c->P, c->smem,
-                             c->dsph_smem, c->rel_rows, c->stream);
+    // an FP64 evaluation over the largest cluster that its tiles keep busy
+    int cs = 1;
+    if (c->opt.form == PS_FORM_FP64) {
+        FormPlan &pl = c->plan[PS_FORM_FP64];
+        cs = static_cast<int>(std::min<int64_t>(psg::kMaxClusterCtas, tiles_of(c, pl.P)));
+        while (cs > 1 && clusters_of(pl, cs) < 1) cs--;
+    }
+    int e = cs > 1 ? psg::launch_eval_split(c->dob, cfg, d_cg, d_al, d_be, d_c2, d_ar, c->d_scratch,
+                                            c->scratch_stride, cs, c->P, c->smem, c->rel_rows, c->stream)
+                   : psg::launch_eval(c->opt.form, c->dob, cfg, d_cg, d_al, d_be, d_c2, d_ar, c->d_scratch, c->P,
+                                      c->smem, c->dsph_smem, c->rel_rows, c->stream);
     if (e != 0) return cuda_fail(c, static_cast<cudaError_t>(e), "eval kernel launch");
     PSG_CUDA(c, cudaMemcpyAsync(alpha, d_al, static_cast<size_t>(mf) * mf * sizeof(double), cudaMemcpyDeviceToHost,
                                 c->stream));

@@ -179,6 +179,13 @@ int set_kernel_smem(int form, size_t smem, int ncoef, int dsph_smem)
             e = cudaFuncSetAttribute(eval_kernel<PS_FORM_FP64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(fit_kernel_split, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(eval_kernel_split, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        // clusters of more than 8 CTAs
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(fit_kernel_split, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(eval_kernel_split, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     } else if (form == PS_FORM_MIXED) {
         e = for_mixed(ncoef, dsph_smem, [&](auto ku) {
             constexpr int KU = decltype(ku)::value;
@@ -252,7 +259,10 @@ int split_max_clusters(int cs, size_t smem, int *clusters)
 {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t lc = split_config(1, cs, smem, nullptr, attr);
-    return static_cast<int>(cudaOccupancyMaxActiveClusters(clusters, fit_kernel_split, &lc));
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(clusters, fit_kernel_split, &lc);
+    if (e == cudaSuccess) return 0;
+    cudaGetLastError();
+    return static_cast<int>(e);
 }
 
 int launch_fits_split(const DevObject &ob, const FitConfig &cfg, const FitWork &w, int clusters, int cs, int P,
@@ -261,6 +271,16 @@ int launch_fits_split(const DevObject &ob, const FitConfig &cfg, const FitWork &
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t lc = split_config(clusters, cs, smem, static_cast<cudaStream_t>(stream), attr);
     return static_cast<int>(cudaLaunchKernelEx(&lc, fit_kernel_split, ob, cfg, w, P));
+}
+
+int launch_eval_split(const DevObject &ob, const FitConfig &cfg, const double *cg, double *alpha, double *beta,
+                      double *chisq, double *area, double *scratch, size_t scratch_stride, int cs, int P, size_t smem,
+                      int rel_rows, void *stream)
+{
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t lc = split_config(1, cs, smem, static_cast<cudaStream_t>(stream), attr);
+    return static_cast<int>(cudaLaunchKernelEx(&lc, eval_kernel_split, ob, cfg, cg, alpha, beta, chisq, area, scratch,
+                                               scratch_stride, P, rel_rows));
 }
 
 int launch_eval(int form, const DevObject &ob, const FitConfig &cfg, const double *cg, double *alpha, double *beta,

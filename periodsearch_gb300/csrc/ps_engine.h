@@ -255,7 +255,7 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     // FP64 form: P counts (int) and P x wcols facet indices (uint16_t)
     const int warps64 = threads_of<PS_FORM_FP64>() / 32;
     L.phase = form == PS_FORM_FP64 ? take(static_cast<size_t>(4 * warps64) * P * d) : 0;
-    L.resid = form == PS_FORM_FP64 ? take(96 * d + static_cast<size_t>(32) * warps64) : 0;
+    L.resid = form == PS_FORM_FP64 ? take(64 * d + static_cast<size_t>(32) * warps64) : 0;
     L.lit = form == PS_FORM_FP64 ? take(static_cast<size_t>(P) * (4 + 2 * L.wcols)) : 0;
     L.bytes = o;
     return L;
@@ -264,12 +264,18 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
 // Launchers (ps_engine.cu).  All enqueue on `stream`; return cudaError_t as int.
 int launch_fits(int form, const DevObject &ob, const FitConfig &cfg, const FitWork &w, int grid,
                 int P, size_t smem, int dsph_smem, void *stream);
-// FP64 fits each spread over a thread-block cluster of cs CTAs (2..8),
+// FP64 fits each spread over a thread-block cluster of cs CTAs (2..16),
 // bit-identical to launch_fits' FP64 kernel; w without trajectories, saved
 // states or an iteration limit.
 int launch_fits_split(const DevObject &ob, const FitConfig &cfg, const FitWork &w, int clusters, int cs, int P,
                       size_t smem, void *stream);
 int split_max_clusters(int cs, size_t smem, int *clusters);
+// One FP64 evaluation spread over a cluster of cs CTAs (scratch: a block of
+// scratch_stride doubles each).
+int launch_eval_split(const DevObject &ob, const FitConfig &cfg, const double *cg, double *alpha, double *beta,
+                      double *chisq, double *area, double *scratch, size_t scratch_stride, int cs, int P, size_t smem,
+                      int rel_rows, void *stream);
+constexpr int kMaxClusterCtas = 16;
 int launch_eval(int form, const DevObject &ob, const FitConfig &cfg, const double *cg, double *alpha,
                 double *beta, double *chisq, double *area, double *scratch, int P, size_t smem,
                 int dsph_smem, int rel_rows, void *stream);

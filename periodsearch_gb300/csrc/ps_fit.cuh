@@ -100,7 +100,7 @@ struct Smem {
     int *nlit;
     uint16_t *lidx;
     double *phase;          // FP64 form: [4][warps * P] first set-up part of the CTA's next tiles
-    double *resid;          // FP64 form: [3][32] a tile's residuals, their weighted squares, renormalisation factors
+    double *resid;          // FP64 form: [2][32] a tile's residuals and their weighted squares
     unsigned char *order;   // FP64 form: [warps][32] points of the tile by lit count
     uint32_t *tslot;
     int *abort;
@@ -139,7 +139,7 @@ __device__ inline Smem<FORM> carve(char *base, const SlotLayout &L)
                                      : nullptr;
     s.phase = L.form == PS_FORM_FP64 ? reinterpret_cast<double *>(base + L.phase) : nullptr;
     s.resid = L.form == PS_FORM_FP64 ? reinterpret_cast<double *>(base + L.resid) : nullptr;
-    s.order = L.form == PS_FORM_FP64 ? reinterpret_cast<unsigned char *>(base + L.resid + 96 * sizeof(double)) : nullptr;
+    s.order = L.form == PS_FORM_FP64 ? reinterpret_cast<unsigned char *>(base + L.resid + 64 * sizeof(double)) : nullptr;
     s.dsph = L.dsph_smem == kBasisSmem ? reinterpret_cast<float *>(base + L.dsph) : nullptr;
     if (basis_on_tensor(L.dsph_smem)) {
         s.bhi = reinterpret_cast<unsigned char *>(base + L.bhi);
@@ -1973,7 +1973,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
 // evaluation's 8.8 Mcycles the FP64 instructions take 7.7 on full units
 // (contraction 3.3, facet law 3.0, alpha 0.8).
 // ---------------------------------------------------------------------------
-constexpr int kMaxSplit = 8;
+constexpr int kMaxSplit = 16;
 constexpr int kWarpsFp64 = threads_of<PS_FORM_FP64>() / 32;
 
 // First part of the set-up (setup_phase_fp64) of the CTA's next kWarpsFp64
@@ -2197,8 +2197,10 @@ __device__ void evaluate_fp64(const DevObject &ob, const FitConfig &cfg, const S
     // values (the CTA's own tile, or another CTA's staged in Jst/ymst); the
     // second pass stages its renormalised rows there too, so that s.J, which
     // the other CTAs read during the round, stays as computed.
-    double *Jst = s.W + static_cast<size_t>(P) * mf, *ymst = Jst + static_cast<size_t>(P) * ma;
-    double *coefv = s.resid + 64;
+    // The staging area: stage_cap points' rows and model values.
+    const int stage_cap =
+        min((static_cast<int>((L.J - L.W) / sizeof(double)) - P * mf) / (ma + 1), P * kRedStride) / P * P;
+    double *Jst = s.W + static_cast<size_t>(P) * mf, *ymst = Jst + static_cast<size_t>(stage_cap) * ma;
     auto consume_tile = [&](int lc, int t0, int np, const double *Jt, const double *yt) {
         const int start = ob.lc_start[lc], npts = ob.lc_npts[lc];
         if (!ob.lc_rel[lc]) {
@@ -2226,27 +2228,45 @@ __device__ void evaluate_fp64(const DevObject &ob, const FitConfig &cfg, const S
         }
         __syncthreads();
         if (t0 + P < npts) return;
-        // second pass of the lightcurve (mrqcof.c:90-136)
+        // second pass of the lightcurve (mrqcof.c:90-136), as many tiles at a
+        // time as the staging area holds: of the renormalised rows every CTA
+        // computes its share of the points for all of the cluster (two
+        // divisions per point and one per element: 12 of a tile's 18 kcycles
+        // when each CTA computed them all)
         const double ave = s.misc[M_AVE];
-        for (int u0 = 0; u0 < npts; u0 += P) {
-            const int nq = min(P, npts - u0);
-            const double *src = scratch + static_cast<size_t>(u0) * RW;
-            if (warp == NW - 1 && lane < nq) {
-                const double coef = ob.sig[start + u0 + lane] * npts / ave;
-                coefv[lane] = coef;
-                ymst[lane] = coef * src[static_cast<size_t>(lane) * RW + ma];
-            }
-            // every element's quotient first, the point's factor after the barrier
-            for (int e = tid; e < nq * ma; e += NT) {
-                const int p = e / ma, l = e - p * ma;
-                const double v = src[static_cast<size_t>(p) * RW + l];
-                const double ytv = src[static_cast<size_t>(p) * RW + ma];
-                Jst[e] = l == 0 ? 0.0 : v - ytv * s.dave[l] / ave;
+        for (int b0 = 0; b0 < npts; b0 += stage_cap) {
+            const int nb = min(stage_cap, npts - b0), mine = (nb - rank + cs - 1) / cs;
+            const double *src = scratch + static_cast<size_t>(b0) * RW;
+            double *coef = s.red;
+            if constexpr (SPLIT) cgr::this_cluster().sync();   // every CTA's staging area is free
+            for (int i = tid; i < mine; i += NT) {
+                const int p = i * cs + rank;
+                const double c = ob.sig[start + b0 + p] * npts / ave;
+                coef[i] = c;
+                const double y = c * src[static_cast<size_t>(p) * RW + ma];
+                if constexpr (SPLIT) {
+                    for (int r = 0; r < cs; r++) *cgr::this_cluster().map_shared_rank(ymst + p, r) = y;
+                } else {
+                    ymst[p] = y;
+                }
             }
             __syncthreads();
-            for (int e = tid; e < nq * ma; e += NT) Jst[e] = coefv[e / ma] * Jst[e];
-            __syncthreads();
-            accumulate_tile_fp64(ob, s, M, bv, nq, start + u0, false, conv_sig, Jst, ymst, rank, cs);
+            for (int e = tid; e < mine * ma; e += NT) {
+                const int i = e / ma, l = e - i * ma, p = i * cs + rank;
+                const double *row = src + static_cast<size_t>(p) * RW;
+                const double out = l == 0 ? 0.0 : coef[i] * (row[l] - row[ma] * s.dave[l] / ave);
+                if constexpr (SPLIT) {
+                    for (int r = 0; r < cs; r++)
+                        *cgr::this_cluster().map_shared_rank(Jst + static_cast<size_t>(p) * ma + l, r) = out;
+                } else {
+                    Jst[static_cast<size_t>(p) * ma + l] = out;
+                }
+            }
+            if constexpr (SPLIT) cgr::this_cluster().sync();
+            else __syncthreads();
+            for (int u0 = 0; u0 < nb; u0 += P)
+                accumulate_tile_fp64(ob, s, M, bv, min(P, nb - u0), start + b0 + u0, false, conv_sig,
+                                     Jst + static_cast<size_t>(u0) * ma, ymst + u0, rank, cs);
         }
     };
 
@@ -2743,9 +2763,9 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
 // the last element in row-major order (the reference's >=).  The bits of |a|
 // order as its values do (NaN patterns, above +inf's, skipped as v >= 0 skips
 // them), so the search compares 64-bit integers, off the FP64 unit.
-// ws: 2 n + 1 doubles and 3 n + 32 ints of workspace (gj_doubles, gj_ints).
-// Measured (n = 55): ten fits of 980 points on 4-CTA clusters 68.8 -> 62.8 ms, 400 fits on one CTA each
-// 548 -> 523 ms.
+// wd, wi: gj_doubles(n) doubles and gj_ints(n) ints of workspace.
+// Measured (n = 55, 980 points): ten fits on 4-CTA clusters 68.8 -> 62.8 ms, 400
+// fits on one CTA each 548 -> 523 ms.
 template <int NT>
 __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
 {
@@ -3510,6 +3530,31 @@ __global__ void __launch_bounds__(threads_of<PS_FORM_FP64>(), 1)
         run_fit<PS_FORM_FP64, 1>(ob, cfg, L, s, scratch, n, pole, rank == 0 ? w.out + f : nullptr, w, f, tcs, true);
     }
     if (threadIdx.x == 0 && w.lit) atomicAdd(w.lit, *lit_counter(s.misc));
+}
+
+// One FP64 evaluation spread over one thread-block cluster, bit-identical to
+// eval_kernel<FP64>'s.
+__global__ void __launch_bounds__(threads_of<PS_FORM_FP64>(), 1)
+    eval_kernel_split(DevObject ob, FitConfig cfg, const double *cg, double *alpha, double *beta, double *chisq,
+                      double *area, double *scratch, size_t scratch_stride, int P, int rel_rows)
+{
+    constexpr int NT = threads_of<PS_FORM_FP64>();
+    extern __shared__ __align__(16) char smem[];
+    const SlotLayout L = make_layout(PS_FORM_FP64, ob.ma, ob.mfit, ob.nfac, ob.ncoef, P, 0, rel_rows);
+    Smem<PS_FORM_FP64> s = carve<PS_FORM_FP64>(smem, L);
+    for (int i = threadIdx.x; i < ob.ma; i += NT) s.cg[i] = cg[i];
+    if (threadIdx.x == 0) *lit_counter(s.misc) = 0;
+    __syncthreads();
+    double *rows = L.rels ? reinterpret_cast<double *>(smem + L.rels)
+                          : scratch + static_cast<size_t>(blockIdx.x) * scratch_stride;
+    evaluate_fp64<true>(ob, cfg, L, s, s.cg, s.alpha, s.beta, rows, true);
+    if (blockIdx.x != 0) return;   // the last remote accesses lie before evaluate_fp64's last cluster barrier
+    const int mf = ob.mfit;
+    for (int e = threadIdx.x; e < mf * mf; e += NT) alpha[e] = s.alpha[e];
+    for (int j = threadIdx.x; j < mf; j += NT) beta[j] = s.beta[j];
+    if (area)
+        for (int i = threadIdx.x; i < ob.nfac; i += NT) area[i] = s.area[i];
+    if (threadIdx.x == 0) *chisq = s.misc[M_CHISQ];
 }
 
 template <int FORM, int KU>
