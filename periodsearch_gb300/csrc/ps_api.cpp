@@ -30,6 +30,8 @@ struct FormPlan {
     int P = 16, dsph_smem = 0, slots = 0;
     int rel_rows = 0;   // relative-lightcurve rows parked in shared memory (0: global scratch)
     size_t smem = 0;
+    size_t pair_smem = 0;   // shared memory of the kernel with two fits per CTA, 0 where it does not apply
+    int pair_rel_rows = 0;
     int clusters[psg::kMaxClusterCtas + 1] = {};   // FP64 form: clusters of k CTAs the device runs at once, 0: not asked yet
 };
 
@@ -46,6 +48,7 @@ struct ps_ctx {
     size_t smem = 0;
     double *d_scratch = nullptr;
     size_t scratch_stride = 0;
+    int scratch_slots = 0;
     unsigned long long *d_queue = nullptr;
     ps_fit *d_out = nullptr;
     size_t out_cap = 0;
@@ -194,6 +197,22 @@ ps_status build_plan(ps_ctx *c, int form, int dsph_smem, int P, int per_sm_cap, 
     out->rel_rows = rel_rows;
     out->smem = bytes;
     out->slots = per_sm * c->sm_count;
+    // two fits per CTA where their slots fit the shared and the Tensor Memory
+    // (not when the caller asked for one slot per SM)
+    out->pair_smem = 0;
+    if (dsph_smem == psg::kBasisTensor && per_sm_cap != 1 && psg::tensor_pair_ok(F, o.mfit)) {
+        constexpr size_t kStatic = 64;   // the kernel's own static shared memory
+        for (int rows : {o.max_rel_points, 0}) {
+            const size_t need =
+                psg::kPairFits * psg::make_layout(form, o.ma, o.mfit, F, o.ncoef, P, dsph_smem, rows, true).bytes;
+            if (need + kStatic > smem_max) continue;
+            e = psg::set_pair_smem(std::max(need, floor_tc));
+            if (e != 0) return cuda_fail(c, static_cast<cudaError_t>(e), "cudaFuncSetAttribute");
+            out->pair_smem = std::max(need, floor_tc);
+            out->pair_rel_rows = rows;
+            break;
+        }
+    }
     out->ready = true;
     return PS_OK;
 }
@@ -279,12 +298,20 @@ ps_status run_fits(ps_ctx *c, double conw_r, psg::FitWork w, int form)
     ps_status st = make_plan(c, form);
     if (st != PS_OK) return st;
     FormPlan &pl = c->plan[form];
-    if (pl.slots > c->slots) {
-        // a second form with more slots than the scratch was sized for
+    // More mixed fits than slots: two fits side by side on each CTA.  A fit
+    // takes longer there (half the threads), two of them less than one after
+    // the other; with at most a fit per SM each keeps its SM.  Measured (980
+    // points, 288 facets), one against two per SM: 152 fits 11.2 ms, 304 fits
+    // 22.4 against 18.2 ms, 608 fits 45 against 36 ms.
+    const bool pair = form == PS_FORM_MIXED && pl.pair_smem > 0 && w.nfits > pl.slots;
+    const int fit_slots = pair ? psg::kPairFits * pl.slots : pl.slots;
+    if (pl.slots > c->slots) c->slots = pl.slots;   // a second form with more slots
+    if (fit_slots > c->scratch_slots) {
         cudaFree(c->d_scratch);
         c->d_scratch = nullptr;
-        PSG_CUDA(c, cudaMalloc(&c->d_scratch, c->scratch_stride * pl.slots * sizeof(double)));
-        c->slots = pl.slots;
+        c->scratch_slots = 0;
+        PSG_CUDA(c, cudaMalloc(&c->d_scratch, c->scratch_stride * fit_slots * sizeof(double)));
+        c->scratch_slots = fit_slots;
     }
     psg::FitConfig cfg = make_config(c, conw_r);
     st = ensure_out(c, static_cast<size_t>(w.nfits));
@@ -293,17 +320,17 @@ ps_status run_fits(ps_ctx *c, double conw_r, psg::FitWork w, int form)
     w.lit = c->d_queue + 1;   // the lit facet-point counter of the FP64 form
     w.scratch = c->d_scratch;
     w.scratch_stride = c->scratch_stride;
-    w.rel_rows = pl.rel_rows;
+    w.rel_rows = pair ? pl.pair_rel_rows : pl.rel_rows;
     w.out = c->d_out;
-    if (pl.dsph_smem == psg::kBasisTensorWide) {
-        // the wide tensor-core path keeps each slot's normal matrix in global memory
+    if (pl.dsph_smem == psg::kBasisTensorWide || pair) {
+        // each slot's normal matrix in global memory
         const size_t stride = static_cast<size_t>(c->obj.mfit) * c->obj.mfit;
-        if (c->alpha_g_slots < static_cast<size_t>(pl.slots)) {
+        if (c->alpha_g_slots < static_cast<size_t>(fit_slots)) {
             cudaFree(c->d_alpha_g);
             c->d_alpha_g = nullptr;
             c->alpha_g_slots = 0;
-            PSG_CUDA(c, cudaMalloc(&c->d_alpha_g, stride * pl.slots * sizeof(double)));
-            c->alpha_g_slots = static_cast<size_t>(pl.slots);
+            PSG_CUDA(c, cudaMalloc(&c->d_alpha_g, stride * fit_slots * sizeof(double)));
+            c->alpha_g_slots = static_cast<size_t>(fit_slots);
         }
         w.alpha_g = c->d_alpha_g;
         w.alpha_stride = stride;
@@ -318,6 +345,8 @@ ps_status run_fits(ps_ctx *c, double conw_r, psg::FitWork w, int form)
     if (cs > 1) {
         const int clusters = static_cast<int>(std::min<int64_t>(std::max(clusters_of(pl, cs), 1), w.nfits));
         e = psg::launch_fits_split(c->dob, cfg, w, clusters, cs, pl.P, pl.smem, c->stream);
+    } else if (pair) {
+        e = psg::launch_fits_pair(c->dob, cfg, w, grid, pl.pair_smem, c->stream);
     } else {
         e = psg::launch_fits(form, c->dob, cfg, w, grid, pl.P, pl.smem, pl.dsph_smem, c->stream);
     }
@@ -757,7 +786,8 @@ ps_status upload_object(std::unique_ptr<ps_ctx> &c, ps_ctx **out)
     c->slots = c->plan[c->opt.form].slots;
     c->scratch_stride = static_cast<size_t>(std::max(o.max_rel_points, 1)) * psg::rel_row_stride(o.ma);
     c->scratch_stride = (c->scratch_stride + 31) & ~size_t(31);
-    PSG_CUDA(cp, cudaMalloc(&c->d_scratch, c->scratch_stride * c->slots * sizeof(double)));
+    c->scratch_slots = c->slots * (c->plan[c->opt.form].pair_smem > 0 ? psg::kPairFits : 1);
+    PSG_CUDA(cp, cudaMalloc(&c->d_scratch, c->scratch_stride * c->scratch_slots * sizeof(double)));
     PSG_CUDA(cp, cudaMalloc(&c->d_queue, 256));
     size_t ev_doubles = static_cast<size_t>(o.ma) + static_cast<size_t>(o.mfit) * o.mfit + o.mfit + 1 + F;
     PSG_CUDA(cp, cudaMalloc(&c->d_eval, ev_doubles * sizeof(double)));
@@ -1335,7 +1365,7 @@ struct ps_pack {
     size_t scratch_stride = 0;
     double *d_alpha_g = nullptr;       // per-slot normal matrices of the wide tensor-core path
     int slots = 0, P = 0, dsph_smem = 0;
-    size_t smem = 0;
+    size_t smem = 0, pair_smem = 0;    // pair_smem: of the kernel with two fits per CTA, 0 where it does not apply
     unsigned long long *d_queue = nullptr;
     int *d_obj = nullptr, *d_pole = nullptr;
     int64_t *d_pidx = nullptr;
@@ -1402,11 +1432,23 @@ ps_status ps_pack_create(ps_ctx *const *ctxs, int32_t n, int32_t form, ps_pack *
     PSG_PACK_CUDA(k.get(), cudaEventCreate(&k->ev[1]));
     PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_objs, sizeof(psg::DevObject) * n));
     PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_cfgs, sizeof(psg::FitConfig) * n));
-    PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_scratch, k->scratch_stride * k->slots * sizeof(double)));
+    if (pl.pair_smem > 0) {
+        const psg::HostObject &o = c0->obj;
+        k->pair_smem = std::max(psg::kPairFits * psg::make_layout(form, o.ma, o.mfit, o.shape.nfac, o.ncoef, k->P,
+                                                                  k->dsph_smem, 0, true).bytes,
+                                k->smem);
+        // (the packed kernel's static shared memory may leave no room)
+        if (psg::set_pack_pair_smem(k->pair_smem) != 0) {
+            cudaGetLastError();
+            k->pair_smem = 0;
+        }
+    }
+    const int fit_slots = k->slots * (k->pair_smem > 0 ? psg::kPairFits : 1);
+    PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_scratch, k->scratch_stride * fit_slots * sizeof(double)));
     PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_queue, 2 * sizeof(unsigned long long)));
-    if (k->dsph_smem == psg::kBasisTensorWide)
+    if (k->dsph_smem == psg::kBasisTensorWide || k->pair_smem > 0)
         PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_alpha_g, static_cast<size_t>(c0->obj.mfit) * c0->obj.mfit *
-                                                            k->slots * sizeof(double)));
+                                                            fit_slots * sizeof(double)));
     std::vector<psg::DevObject> objs(static_cast<size_t>(n));
     for (int32_t i = 0; i < n; i++) objs[static_cast<size_t>(i)] = ctxs[i]->dob;
     PSG_PACK_CUDA(k.get(), cudaMemcpy(k->d_objs, objs.data(), sizeof(psg::DevObject) * n, cudaMemcpyHostToDevice));
@@ -1507,7 +1549,10 @@ ps_status pack_run(ps_pack *k, const double *conw_r, int64_t n_fits, const int32
     }
     const int grid = static_cast<int>(std::min<int64_t>(k->slots, n_fits));
     PSG_PACK_CUDA(k, cudaEventRecord(k->ev[0], k->stream));
-    int e = psg::launch_pack(k->form, w, k->ctx[0]->obj.ncoef, grid, k->P, k->smem, k->dsph_smem, k->stream);
+    // more fits than slots: two side by side on each CTA (see run_fits)
+    int e = k->pair_smem > 0 && n_fits > k->slots
+                ? psg::launch_pack_pair(w, grid, k->pair_smem, k->stream)
+                : psg::launch_pack(k->form, w, k->ctx[0]->obj.ncoef, grid, k->P, k->smem, k->dsph_smem, k->stream);
     if (e != 0) return pack_fail(k, static_cast<cudaError_t>(e), "packed fit kernel launch");
     PSG_PACK_CUDA(k, cudaEventRecord(k->ev[1], k->stream));
     std::vector<ps_fit> sorted(static_cast<size_t>(n_fits));

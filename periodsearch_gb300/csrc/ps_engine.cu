@@ -235,6 +235,28 @@ int launch_fits(int form, const DevObject &ob, const FitConfig &cfg, const FitWo
     return static_cast<int>(cudaGetLastError());
 }
 
+// As set_kernel_smem, for the kernel with two fits per CTA.
+int set_pair_smem(size_t smem)
+{
+    static std::mutex mu;
+    static int raised[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    std::lock_guard<std::mutex> lock(mu);
+    int *cur = dev >= 0 && dev < 64 ? &raised[dev] : nullptr;
+    if (cur && *cur >= static_cast<int>(smem)) return 0;
+    e = cudaFuncSetAttribute(fit_kernel_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e == cudaSuccess && cur) *cur = static_cast<int>(smem);
+    return static_cast<int>(e);
+}
+
+int launch_fits_pair(const DevObject &ob, const FitConfig &cfg, const FitWork &w, int grid, size_t smem, void *stream)
+{
+    fit_kernel_pair<<<grid, threads_of<PS_FORM_MIXED>(), smem, static_cast<cudaStream_t>(stream)>>>(ob, cfg, w);
+    return static_cast<int>(cudaGetLastError());
+}
+
 namespace {
 cudaLaunchConfig_t split_config(int clusters, int cs, size_t smem, cudaStream_t st, cudaLaunchAttribute *attr)
 {

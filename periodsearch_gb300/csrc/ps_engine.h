@@ -134,6 +134,8 @@ PSG_HD constexpr int threads_of()
 {
     return FORM == PS_FORM_MIXED ? 512 : 384;
 }
+// Threads of a team of the kernel that runs two mixed fits per CTA.
+constexpr int kTeamThreads = 256, kPairFits = 2;
 constexpr int kPointStride = 33;   // reals of per-point set-up (odd: a warp with one point per lane hits 32 banks)
 constexpr int kRedStride = 9;      // doubles of per-point facet sums
 constexpr int kMisc = 40;
@@ -162,17 +164,20 @@ PSG_HD constexpr int tc_kpad(int nfac) { return (nfac + 31) & ~31; }
 
 
 // Workspace of the Gauss-Jordan solve of n equations: the scaled pivot row,
-// the pivot column and the right-hand side's entry; two column lists, the
-// pivoted flags and a candidate per warp.
-PSG_HD constexpr size_t gj_doubles(int n) { return 2 * static_cast<size_t>(n) + 1; }
+// the pivot column, the right-hand side's entry and a candidate's bits per
+// warp; two column lists, the pivoted flags and a candidate per warp.
+PSG_HD constexpr size_t gj_doubles(int n) { return 2 * static_cast<size_t>(n) + 1 + 16; }
 PSG_HD constexpr size_t gj_ints(int n) { return 3 * static_cast<size_t>(n) + 16; }
 
 // dsph_smem: the mixed form keeps the FP32 basis Dsph[F][C] in shared memory
 // for the whole launch (it is read once per point tile by every warp).
 // rel_rows > 0: the rows of relative lightcurves (up to rel_rows points)
 // are parked in shared memory instead of the per-slot global scratch.
+// pair: a slot of the kernel with two fits per CTA (tensor-core path): the
+// kept normal matrix in global memory, alpha's operands over the
+// contraction's, one after the other.
 PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int ncoef, int P, int dsph_smem,
-                                     int rel_rows = 0)
+                                     int rel_rows = 0, bool pair = false)
 {
     SlotLayout L{};
     L.form = form;
@@ -195,12 +200,13 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     L.atry = take(ma * d);
     L.beta = take(mfit * d);
     L.da = take(mfit * d);
-    L.alpha = take(dsph_smem == kBasisTensorWide ? 0 : static_cast<size_t>(mfit) * mfit * d);
+    L.alpha = take(dsph_smem == kBasisTensorWide || pair ? 0 : static_cast<size_t>(mfit) * mfit * d);
     L.covar = take(static_cast<size_t>(mfit) * mfit * d);
     L.area = take(nfac * d);
     L.gv = take(nfac * d);
-    L.areaR = form == PS_FORM_MIXED ? take(nfac * rs) : L.area;
-    L.gvR = form == PS_FORM_MIXED ? take(nfac * rs) : L.gv;
+    // (FP32 copies of the SIMT paths; the tensor-core paths have fac)
+    L.areaR = form == PS_FORM_MIXED && !basis_on_tensor(dsph_smem) ? take(nfac * rs) : L.area;
+    L.gvR = form == PS_FORM_MIXED && !basis_on_tensor(dsph_smem) ? take(nfac * rs) : L.gv;
     // the tensor-core path writes W straight into the MMA operand
     // (FP64 form: room for the accumulation weights of a tile, [P][mfit],
     // and a staged tile of rows and model values, [P][ma] + [P], behind them)
@@ -233,9 +239,12 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
             readback = 2 * 128 * 33 * sizeof(float);
             if (wt > readback) readback = wt;
         }
+        // (whole 128-byte lines: a core matrix is one line)
+        o = (o + 127) & ~size_t(127);
         L.bhi = take(2 * tile > readback ? 2 * tile : readback);
         L.blo = L.bhi + tile;
-        L.aop = take(wide ? 0 : kTcAlphaOperands);
+        o = (o + 127) & ~size_t(127);
+        L.aop = pair ? L.bhi : take(wide ? 0 : kTcAlphaOperands);
         L.tcm = take(32);
         L.pt2 = take(static_cast<size_t>(P) * kPointStride * rs);
         L.fac = take(static_cast<size_t>(tc_kpad(nfac)) * 4 * sizeof(float));
@@ -257,13 +266,26 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     L.phase = form == PS_FORM_FP64 ? take(static_cast<size_t>(4 * warps64) * P * d) : 0;
     L.resid = form == PS_FORM_FP64 ? take(64 * d + static_cast<size_t>(32) * warps64) : 0;
     L.lit = form == PS_FORM_FP64 ? take(static_cast<size_t>(P) * (4 + 2 * L.wcols)) : 0;
-    L.bytes = o;
+    L.bytes = (o + 127) & ~size_t(127);
     return L;
 }
+
+// Tensor Memory of the tensor-core path (ps_fit.cuh): the column of the first
+// contraction accumulator, and the rows of alpha's operands (the free
+// parameters and the residual row, in groups of 8).
+PSG_HD inline uint32_t tc_dcol(int F, bool wide = false)
+{
+    return static_cast<uint32_t>(((wide ? 3 * (tc_kpad(F) >> 2) : (tc_kpad(F) >> 1)) + 31) & ~31);
+}
+PSG_HD inline int tc_arows(int mfit) { return (mfit + 1 + 7) & ~7; }
 
 // Launchers (ps_engine.cu).  All enqueue on `stream`; return cudaError_t as int.
 int launch_fits(int form, const DevObject &ob, const FitConfig &cfg, const FitWork &w, int grid,
                 int P, size_t smem, int dsph_smem, void *stream);
+// Mixed fits (tensor-core path), two side by side on each CTA: w.rel_rows,
+// w.scratch and w.alpha_g are those of kPairFits slots per CTA.
+int launch_fits_pair(const DevObject &ob, const FitConfig &cfg, const FitWork &w, int grid, size_t smem, void *stream);
+int set_pair_smem(size_t smem);
 // FP64 fits each spread over a thread-block cluster of cs CTAs (2..16),
 // bit-identical to launch_fits' FP64 kernel; w without trajectories, saved
 // states or an iteration limit.
@@ -286,7 +308,16 @@ int set_kernel_smem(int form, size_t smem, int ncoef, int dsph_smem);
 // fits.  The basis and facet constants are taken from w.objs[0].
 int launch_pack(int form, const FitWork &w, int ncoef, int grid, int P, size_t smem, int dsph_smem, void *stream);
 int set_pack_smem(int form, size_t smem, int ncoef, int dsph_smem);
+int launch_pack_pair(const FitWork &w, int grid, size_t smem, void *stream);
+int set_pack_pair_smem(size_t smem);
 int occupancy_slots(int form, size_t smem, int ncoef, int dsph_smem, int *per_sm);
+// Whether two fits share a CTA's Tensor Memory on the tensor-core path: the
+// basis, two contraction and two alpha accumulators within 512 columns (55
+// free parameters: up to 288 facets).
+PSG_HD inline bool tensor_pair_ok(int nfac, int mfit)
+{
+    return static_cast<int>(tc_dcol(nfac)) + 2 * (64 + 2 * tc_arows(mfit)) <= 512;
+}
 // Whether the tensor-core path supports an object: at most 64 coefficients
 // (the high and low FP16 parts of the basis fill 128 Tensor Memory lanes),
 // at most 63 free parameters (alpha and the beta column in 64 rows), a

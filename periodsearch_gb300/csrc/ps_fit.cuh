@@ -213,6 +213,24 @@ __device__ inline int tri_row(int e)
     return j;
 }
 
+constexpr int kSlotThreads = threads_of<PS_FORM_MIXED>();   // of a whole CTA of the mixed form
+
+// The threads of one fit.  A fit slot is a CTA, or (NT = kTeamThreads) one of
+// the two teams of a CTA that runs two fits side by side (fit_kernel_pair):
+// the thread's number in its team, and the team's barrier (named barriers 2
+// and 3; 1, 4 and 5 serve the Cholesky solve's helper warp).
+template <int NT>
+__device__ inline int team_thread()
+{
+    return NT == kTeamThreads ? static_cast<int>(threadIdx.x) % kTeamThreads : static_cast<int>(threadIdx.x);
+}
+template <int NT>
+__device__ inline void team_sync()
+{
+    if constexpr (NT == kTeamThreads) __barrier_sync_count(2 + threadIdx.x / kTeamThreads, NT);
+    else __syncthreads();
+}
+
 template <class T>
 __device__ inline T warp_sum(T v)
 {
@@ -801,24 +819,20 @@ constexpr uint32_t kTcWaitTries = 1u << 22;   // mbarrier polls before a wait gi
 constexpr int kErrTcTimeout = 16;             // ps_fit.err_code of a fit cut short by a failed wait
 
 // Tensor Memory columns: the basis [0, Fp/2) (FP16 pairs of facets, Fp =
-// tc_kpad(F)), the contraction accumulator [tc_dcol, tc_dcol + 64) (column
-// p: A W_hi^T for point p, 32 + p: A W_lo^T) and the alpha accumulator
-// [tc_acol, tc_acol + 128).  The wide path (kBasisTensorWide) has the
-// second basis region R2 at [Fp/2, 3 Fp/4), the accumulator at tc_dcol and
-// R2's accumulator at tc_dcol + 64 (columns 0..31: products with the first
-// half of the facets, 32..63: with the second half), and no alpha
-// accumulator.
+// tc_kpad(F)), from tc_dcol on a contraction accumulator of 64 columns for
+// each team (column p: A W_hi^T for point p, 32 + p: A W_lo^T), then an alpha
+// accumulator of 2 tc_arows(mfit) columns for each team.  The wide path
+// (kBasisTensorWide) has the second basis region R2 at [Fp/2, 3 Fp/4), the
+// accumulator at tc_dcol and R2's accumulator at tc_dcol + 64 (columns
+// 0..31: products with the first half of the facets, 32..63: with the second
+// half), and no alpha accumulator.
 __device__ inline uint32_t tc_r2col(int F) { return static_cast<uint32_t>(tc_kpad(F) >> 1); }
-__device__ inline uint32_t tc_dcol(int F, bool wide = false)
-{
-    return static_cast<uint32_t>(((wide ? 3 * (tc_kpad(F) >> 2) : (tc_kpad(F) >> 1)) + 31) & ~31);
-}
-__device__ inline uint32_t tc_acol(int F) { return tc_dcol(F) + 64; }
 
-__device__ inline uint32_t tc_cols(int F, bool wide = false)
+__device__ inline uint32_t tc_cols(int F, int mf, bool wide, int teams)
 {
     uint32_t n = 32;
-    while (n < (wide ? tc_dcol(F, true) + 128 : tc_acol(F) + 128)) n <<= 1;
+    while (n < (wide ? tc_dcol(F, true) + 128u : tc_dcol(F) + static_cast<uint32_t>(teams * (64 + 2 * tc_arows(mf)))))
+        n <<= 1;
     return n;
 }
 
@@ -832,65 +846,82 @@ struct TcState {
     bool apending = false;  // alpha MMAs committed and not waited for
     bool afresh = true;     // the alpha accumulator holds nothing since the last flush
     bool wide = false;      // kBasisTensorWide layout
+    uint32_t dcol = 0, acol = 0;   // Tensor Memory columns of the contraction and the alpha accumulator
 };
+
+// Every thread of the team waits for the barrier's phase; true when all saw
+// it, else the abort flag is set.
+template <int NT>
+__device__ inline bool team_wait(Smem<PS_FORM_MIXED> &s, uint64_t *mbar, uint32_t phase)
+{
+    const bool ok = tc::mbar_wait(mbar, phase, kTcWaitTries);
+    if constexpr (NT == kTeamThreads) {
+        if (!ok) *s.abort = 1;
+        team_sync<NT>();
+        return !*s.abort;
+    } else {
+        if (__syncthreads_and(ok)) return true;
+        if (threadIdx.x == 0) *s.abort = 1;
+        __syncthreads();
+        return false;
+    }
+}
 
 // Waits for the committed alpha MMAs (their operands' shared memory is then
 // free); a wait that gives up sets the abort flag.
+template <int NT>
 __device__ inline void tc_alpha_wait(Smem<PS_FORM_MIXED> &s, TcState &t)
 {
     if (!t.apending || *s.abort) return;
-    const bool ok = __syncthreads_and(tc::mbar_wait(s.mbar2, t.aphase, kTcWaitTries));
     t.apending = false;
-    if (!ok) {
-        if (threadIdx.x == 0) *s.abort = 1;
-        __syncthreads();
+    if (!team_wait<NT>(s, s.mbar2, t.aphase)) {
+        t.apending = true;   // tc_teardown waits once more
         return;
     }
     t.aphase ^= 1u;
     tc::fence_after_sync();
 }
 
-// Allocates the CTA's Tensor Memory, initialises the barriers, stages the
-// facet constants (zero for the padding facets) and loads the basis into
+// Allocates the CTA's Tensor Memory (s0: the shared memory of its first
+// team), initialises the team's barriers, stages the team's facet constants (zero for the padding facets) and loads the basis into
 // Tensor Memory as A = [Dsph_hi^T; Dsph_lo^T]: lane m < 64 holds coefficient
 // m, lane 64 + m what remains of it, both FP16 and scaled by 2^basis_exp
 // (the largest magnitude just below 2^14, so that the low parts stay normal
 // FP16 numbers for elements down to 2^-3 of it); column j holds facets 2j
 // and 2j + 1.
 template <int NT, bool WIDE = false>
-__device__ void tc_setup(const DevObject &ob, Smem<PS_FORM_MIXED> &s, TcState &t)
+__device__ void tc_setup(const DevObject &ob, Smem<PS_FORM_MIXED> &s0, Smem<PS_FORM_MIXED> &s, TcState &t)
 {
+    constexpr int NC = threads_of<PS_FORM_MIXED>(), kTeams = NC / NT;   // the CTA's threads and teams
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ttid = team_thread<NT>(), team = tid / NT;
     const int F = ob.nfac, C = ob.ncoef, Fp = tc_kpad(F);
-    if (warp == 0) tc::tmem_alloc(s.tslot, tc_cols(F, WIDE));
-    if (tid == 0) {
+    if (warp == 0) tc::tmem_alloc(s0.tslot, tc_cols(F, ob.mfit, WIDE, kTeams));
+    if (ttid == 0) {
         tc::mbar_init(s.mbar, 1);
         tc::mbar_init(s.mbar2, 1);
         *s.abort = 0;
     }
     double mx = 0.0;
-    for (int e = tid; e < F * C; e += NT) mx = fmax(mx, fabs(ob.dsph[e]));
+    for (int e = tid; e < F * C; e += NC) mx = fmax(mx, fabs(ob.dsph[e]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s.red[warp] = mx;
+    if (lane == 0) s0.red[warp] = mx;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     mx = 0.0;
-    for (int w = 0; w < NT / 32; w++) mx = fmax(mx, s.red[w]);
+    for (int w = 0; w < NC / 32; w++) mx = fmax(mx, s0.red[w]);
     const int bexp = (mx > 0.0 && mx < 1e300) ? 13 - ilogb(mx) : 0;
     const double bscale = ldexp(1.0, bexp);
-    const uint32_t tbase = *s.tslot;
-    for (int i = tid; i < Fp; i += NT) {
+    const uint32_t tbase = *s0.tslot;
+    for (int i = ttid; i < Fp; i += NT) {
         fac_at(s.fac, i, 0) = i < F ? ob.nx_f[i] : 0.f;
         fac_at(s.fac, i, 1) = i < F ? ob.ny_f[i] : 0.f;
         fac_at(s.fac, i, 2) = i < F ? ob.nz_f[i] : 0.f;
         fac_at(s.fac, i, 3) = 0.f;
     }
-    if constexpr (!WIDE)
-        for (int i = tid; i < static_cast<int>(kTcAlphaOperands / 4); i += NT)
-            reinterpret_cast<uint32_t *>(s.aop)[i] = 0;
-    for (int j = tid; j < ob.mfit; j += NT) s.flist[j] = ob.free_list[j];
+    for (int j = ttid; j < ob.mfit; j += NT) s.flist[j] = ob.free_list[j];
     if (warp < 4) {
         // lane m of R1: coefficient c, high part (low = false) or low part;
         // lane m of R2 (wide path): low part of coefficient c2 for the
@@ -942,19 +973,23 @@ __device__ void tc_setup(const DevObject &ob, Smem<PS_FORM_MIXED> &s, TcState &t
     t.tbase = tbase;
     t.basis_exp = bexp;
     t.wide = WIDE;
+    t.dcol = tc_dcol(F, WIDE) + 64u * team;
+    t.acol = tc_dcol(F) + 64u * kTeams + static_cast<uint32_t>(2 * tc_arows(ob.mfit) * team);
 }
 
 // Releases the Tensor Memory.  After an abandoned wait the MMAs in flight
 // get one more bounded wait first.
-__device__ void tc_teardown(Smem<PS_FORM_MIXED> &s, const TcState &t, int F)
+template <int NT>
+__device__ void tc_teardown(Smem<PS_FORM_MIXED> &s, const TcState &t, int F, int mf)
 {
-    if (*s.abort && threadIdx.x == 0) {
+    if (*s.abort && team_thread<NT>() == 0) {
         tc::mbar_wait(s.mbar, t.phase, kTcWaitTries);
         if (t.apending) tc::mbar_wait(s.mbar2, t.aphase, kTcWaitTries);
     }
     tc::fence_before_sync();
-    __syncthreads();
-    if ((threadIdx.x >> 5) == 0) tc::tmem_dealloc(t.tbase, tc_cols(F, t.wide));
+    __syncthreads();   // both teams
+    if ((threadIdx.x >> 5) == 0)
+        tc::tmem_dealloc(t.tbase, tc_cols(F, mf, t.wide, threads_of<PS_FORM_MIXED>() / NT));
 }
 
 // Issues the alpha/beta MMAs of the operands in s.aop (built and fenced,
@@ -962,12 +997,13 @@ __device__ void tc_teardown(Smem<PS_FORM_MIXED> &s, const TcState &t, int F)
 // every thread; thread 0 issues.  (Issuing them from an idle warp during
 // the next contraction window measured no faster: the MMA issue slots of an
 // SM are shared by its threads.)
-__device__ inline void tc_alpha_issue(Smem<PS_FORM_MIXED> &s, TcState &t, int F)
+template <int NT>
+__device__ inline void tc_alpha_issue(Smem<PS_FORM_MIXED> &s, TcState &t, int mf)
 {
-    if (threadIdx.x == 0 && !*s.abort) {
+    if (team_thread<NT>() == 0 && !*s.abort) {
         tc::fence_after_sync();
-        const uint32_t idesc = tc::idesc_tf32(128, 128);
-        const uint32_t a0 = tc::smem_u32(s.aop), b0 = tc::smem_u32(s.aop + 16384), d = t.tbase + tc_acol(F);
+        const uint32_t idesc = tc::idesc_tf32(128, 2 * tc_arows(mf));
+        const uint32_t a0 = tc::smem_u32(s.aop), b0 = tc::smem_u32(s.aop + 16384), d = t.tbase + t.acol;
         for (int kk = 0; kk < 4; kk++) {
             const uint32_t off = static_cast<uint32_t>(kk) * 256;
             tc::mma_tf32_ss(d, tc::smem_desc(a0 + off, 128, 1024), tc::smem_desc(b0 + off, 128, 1024), idesc,
@@ -988,17 +1024,17 @@ __device__ inline void tc_alpha_issue(Smem<PS_FORM_MIXED> &s, TcState &t, int F)
 template <int NT, bool WIDE = false>
 __device__ void contract_tc_issue(Smem<PS_FORM_MIXED> &s, int F, TcState &t)
 {
-    const int tid = threadIdx.x;
+    const int tid = team_thread<NT>();
     const int Fp = tc_kpad(F), kcs = Fp >> 3;
     const uint32_t tbase = t.tbase;
     tc::fence_proxy_async();
     tc::fence_before_sync();
-    __syncthreads();
+    team_sync<NT>();
     if (tid == 0 && !*s.abort) {
         tc::fence_after_sync();
         const uint32_t idesc = tc::idesc_f16(128, 64);
         const uint32_t sbo = static_cast<uint32_t>(kcs) * 128;
-        const uint32_t bh = tc::smem_u32(s.bhi), d = tbase + tc_dcol(F, WIDE);
+        const uint32_t bh = tc::smem_u32(s.bhi), d = tbase + t.dcol;
         for (int ks = 0; ks < Fp / 16; ks++) {
             const uint32_t a = tbase + static_cast<uint32_t>(ks) * 8, off = static_cast<uint32_t>(ks) * 256;
             tc::mma_f16_ts(d, a, tc::smem_desc(bh + off, 128, sbo), idesc, ks > 0);
@@ -1082,11 +1118,11 @@ template <int NT>
 __device__ void facet_stage_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int np, float cl, float cls,
                                float wscale)
 {
-    static_assert(NT == 512, "16 warps: 4 point groups x 4 facet quarters");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    static_assert(NT % 128 == 0, "warps: 4 point groups x facet quarters");
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int kcs = tc_kpad(ob.nfac) >> 3;   // 8-facet core matrices per row group
     const int cq = kcs >> 2;                 // per facet quarter
-    const int quarter = warp >> 2, g = warp & 3, p = g * 8 + (lane >> 2), fl = lane & 3;
+    const int g = warp & 3, p = g * 8 + (lane >> 2), fl = lane & 3;
     // The point records of this path hold the pole products before the
     // rotation about the spin axis (setup_mixed_geo) and its cos/sin
     // (setup_mixed_phase): Earth and Sun directions rotated here.
@@ -1112,49 +1148,54 @@ __device__ void facet_stage_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int 
     const float2 F1 = make_float2(f1, f1), F2 = make_float2(f2, f2), F3 = make_float2(f3, f3);
     const float2 CL = make_float2(cl, cl), CLS = make_float2(cls, cls), WS = make_float2(wscale, wscale);
     const float2 z2 = make_float2(0.f, 0.f);
-    float2 br = z2, dcl = z2, dcls = z2, ux = z2, uy = z2, uz = z2, vx = z2, vy = z2, vz = z2;
     uint32_t *bh = reinterpret_cast<uint32_t *>(s.bhi), *bl = reinterpret_cast<uint32_t *>(s.blo);
-    for (int kc = quarter * cq; kc < (quarter + 1) * cq; kc++) {
-        const int i = kc * 8 + 2 * fl;
-        const int cm = g * kcs + kc;    // core matrix (8-point group, 8-facet group)
-        const float4 fa = s.fac[i], fb = s.fac[i + 1];
-        const float2 nx = make_float2(fa.x, fa.y), ny = make_float2(fa.z, fa.w), nz = make_float2(fb.x, fb.y);
-        // (unlit facets carry zero area: no branch, see LitPair)
-        const LitPair lp(fa, fb, E1, E2, E3, F1, F2, F3);
-        const float2 ax = lp.ax, m = lp.m, m0 = lp.m0, r = lp.r, mm = lp.mm;
-        const float2 sv = lp.law(CL, CLS);
-        const float2 q0 = __fmul2_rn(m0, r), q1 = __fmul2_rn(m, r);
-        const float2 dsmu = __ffma2_rn(CLS, __fmul2_rn(q0, q0), __fmul2_rn(CL, m0));
-        const float2 dsmu0 = __ffma2_rn(CLS, __fmul2_rn(q1, q1), __fmul2_rn(CL, m));
-        const float2 axs = __fmul2_rn(ax, sv);
-        br = __fadd2_rn(br, axs);
-        const float2 wv = __fmul2_rn(axs, WS);
-        const float2 cu = __fmul2_rn(ax, dsmu), cv = __fmul2_rn(ax, dsmu0);
-        ux = __ffma2_rn(cu, nx, ux);
-        uy = __ffma2_rn(cu, ny, uy);
-        uz = __ffma2_rn(cu, nz, uz);
-        vx = __ffma2_rn(cv, nx, vx);
-        vy = __ffma2_rn(cv, ny, vy);
-        vz = __ffma2_rn(cv, nz, vz);
-        dcl = __ffma2_rn(mm, ax, dcl);
-        dcls = __ffma2_rn(ax, __fmul2_rn(mm, r), dcls);
-        const uint32_t hp = tc::pack_f16x2(wv.x, wv.y);
-        bh[cm * 32 + lane] = hp;
-        bl[cm * 32 + lane] = tc::pack_f16x2(wv.x - tc::f16_lo(hp), wv.y - tc::f16_hi(hp));
-    }
-    float v[9] = {br.x + br.y, dcl.x + dcl.y, dcls.x + dcls.y, ux.x + ux.y, uy.x + uy.y,
-                  uz.x + uz.y, vx.x + vx.y, vy.x + vy.y, vz.x + vz.y};
+    // (a team of 8 warps takes two quarters per warp, one after the other)
+#pragma unroll 1
+    for (int part = 0; part < kSlotThreads / NT; part++) {
+        const int quarter = (warp >> 2) + part * (NT / 128);
+        float2 br = z2, dcl = z2, dcls = z2, ux = z2, uy = z2, uz = z2, vx = z2, vy = z2, vz = z2;
+        for (int kc = quarter * cq; kc < (quarter + 1) * cq; kc++) {
+            const int i = kc * 8 + 2 * fl;
+            const int cm = g * kcs + kc;    // core matrix (8-point group, 8-facet group)
+            const float4 fa = s.fac[i], fb = s.fac[i + 1];
+            const float2 nx = make_float2(fa.x, fa.y), ny = make_float2(fa.z, fa.w), nz = make_float2(fb.x, fb.y);
+            // (unlit facets carry zero area: no branch, see LitPair)
+            const LitPair lp(fa, fb, E1, E2, E3, F1, F2, F3);
+            const float2 ax = lp.ax, m = lp.m, m0 = lp.m0, r = lp.r, mm = lp.mm;
+            const float2 sv = lp.law(CL, CLS);
+            const float2 q0 = __fmul2_rn(m0, r), q1 = __fmul2_rn(m, r);
+            const float2 dsmu = __ffma2_rn(CLS, __fmul2_rn(q0, q0), __fmul2_rn(CL, m0));
+            const float2 dsmu0 = __ffma2_rn(CLS, __fmul2_rn(q1, q1), __fmul2_rn(CL, m));
+            const float2 axs = __fmul2_rn(ax, sv);
+            br = __fadd2_rn(br, axs);
+            const float2 wv = __fmul2_rn(axs, WS);
+            const float2 cu = __fmul2_rn(ax, dsmu), cv = __fmul2_rn(ax, dsmu0);
+            ux = __ffma2_rn(cu, nx, ux);
+            uy = __ffma2_rn(cu, ny, uy);
+            uz = __ffma2_rn(cu, nz, uz);
+            vx = __ffma2_rn(cv, nx, vx);
+            vy = __ffma2_rn(cv, ny, vy);
+            vz = __ffma2_rn(cv, nz, vz);
+            dcl = __ffma2_rn(mm, ax, dcl);
+            dcls = __ffma2_rn(ax, __fmul2_rn(mm, r), dcls);
+            const uint32_t hp = tc::pack_f16x2(wv.x, wv.y);
+            bh[cm * 32 + lane] = hp;
+            bl[cm * 32 + lane] = tc::pack_f16x2(wv.x - tc::f16_lo(hp), wv.y - tc::f16_hi(hp));
+        }
+        float v[9] = {br.x + br.y, dcl.x + dcl.y, dcls.x + dcls.y, ux.x + ux.y, uy.x + uy.y,
+                      uz.x + uz.y, vx.x + vx.y, vy.x + vy.y, vz.x + vz.y};
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-        v[k] += __shfl_xor_sync(0xffffffffu, v[k], 1);
-        v[k] += __shfl_xor_sync(0xffffffffu, v[k], 2);
-    }
-    if (fl == 0) {
-        float *fp = s.fpart + (quarter * 32 + p) * 9;
+        for (int k = 0; k < 9; k++) {
+            v[k] += __shfl_xor_sync(0xffffffffu, v[k], 1);
+            v[k] += __shfl_xor_sync(0xffffffffu, v[k], 2);
+        }
+        if (fl == 0) {
+            float *fp = s.fpart + (quarter * 32 + p) * 9;
 #pragma unroll
-        for (int k = 0; k < 9; k++) fp[k] = v[k];
+            for (int k = 0; k < 9; k++) fp[k] = v[k];
+        }
     }
-    __syncthreads();
+    team_sync<NT>();
     if (tid < np) {
         float t[9];
 #pragma unroll
@@ -1192,7 +1233,7 @@ __device__ void facet_stage_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int 
 template <int NT>
 __device__ void conv_rows_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, float wscale)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int F = ob.nfac, half = tc_kpad(F) >> 1;
     uint32_t *bh = reinterpret_cast<uint32_t *>(s.bhi), *bl = reinterpret_cast<uint32_t *>(s.blo);
     for (int e = tid; e < 3 * half; e += NT) {
@@ -1227,15 +1268,10 @@ template <int NT, bool WIDE = false>
 __device__ void contract_tc_finish(Smem<PS_FORM_MIXED> &s, int np, int F, int C, int ma, bool conv, TcState &t,
                                    float jscale)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const uint32_t tbase = t.tbase;
     if (*s.abort) return;
-    const bool ok = __syncthreads_and(tc::mbar_wait(s.mbar, t.phase, kTcWaitTries));
-    if (!ok) {
-        if (tid == 0) *s.abort = 1;
-        __syncthreads();
-        return;
-    }
+    if (!team_wait<NT>(s, s.mbar, t.phase)) return;
     t.phase ^= 1u;
     tc::fence_after_sync();
     // every warp reads, for 8 points of its lane quadrant's rows (warp w may
@@ -1243,9 +1279,10 @@ __device__ void contract_tc_finish(Smem<PS_FORM_MIXED> &s, int np, int F, int C,
     // (column p) and W_lo (column 32 + p) and stages their sum Y[m][p]
     float *Y = reinterpret_cast<float *>(s.bhi);   // [128][33]
     float *Y2 = Y + 128 * 33;                      // wide path: [128][33] from R2's accumulator
-    {
-        const int quad = warp & 3, pg = warp >> 2;
-        const uint32_t taddr = tbase + (static_cast<uint32_t>(quad * 32) << 16) + tc_dcol(F, WIDE) + 8 * pg;
+#pragma unroll
+    for (int part = 0; part < kSlotThreads / NT; part++) {
+        const int quad = warp & 3, pg = (warp >> 2) + part * (NT / 128);
+        const uint32_t taddr = tbase + (static_cast<uint32_t>(quad * 32) << 16) + t.dcol + 8 * pg;
         float *yr = Y + (quad * 32 + lane) * 33 + 8 * pg;
         uint32_t vh[8], vl[8];
         tc::tmem_ld8(taddr, vh);
@@ -1264,7 +1301,7 @@ __device__ void contract_tc_finish(Smem<PS_FORM_MIXED> &s, int np, int F, int C,
             for (int j = 0; j < 8; j++) y2[j] = __uint_as_float(v2[j]);
         }
     }
-    __syncthreads();
+    team_sync<NT>();
     if constexpr (WIDE) {
         // J[p][k] = Scale_p jscale (high part of k times W_hi and W_lo + low
         // part of k times W: from R1's lanes C + k for k < 128 - C, else
@@ -1298,8 +1335,9 @@ __device__ void contract_tc_finish(Smem<PS_FORM_MIXED> &s, int np, int F, int C,
 // D += A B^T over the tile's points with A = [Wt_hi; Wt_lo] (row j: the
 // weighted column J[.][l_j] sig^-2 w of free parameter j, 128 x 32) and B =
 // [Jt_hi; Jt_lo] (row k < mfit: column J[.][l_k]; row mfit: the residuals
-// dy), both split into TF32 high and low parts, so that the four quadrants
-// of the 128 x 128 FP32 accumulator sum to alpha (and beta in column mfit)
+// dy; the low parts from row tc_arows(mfit) on), both split into TF32 high
+// and low parts, so that the four quadrants of the FP32 accumulator (128
+// lanes x 2 tc_arows(mfit) columns) sum to alpha (and beta in column mfit)
 // at FP32 accuracy.  The accumulator stays in Tensor Memory across tiles
 // until tc_alpha_flush.  chi^2 is summed in FP64 by warp 0, unless the
 // caller has prepared the weights, residuals and chi^2 (prepared).  With
@@ -1312,7 +1350,7 @@ __device__ void accumulate_tile_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, 
                                    double conv_sig, TcState &t, bool prepared, const float *rows = nullptr,
                                    int rw = 0)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int ma = ob.ma, mf = ob.mfit;
     float *dyv = s.accs;
     float *wtp = dyv + 32;
@@ -1330,20 +1368,22 @@ __device__ void accumulate_tile_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, 
         c2 = warp_sum(c2);
         if (tid == 0) s.misc[M_CHISQ] += c2;
     }
-    tc_alpha_wait(s, t);
-    __syncthreads();
+    tc_alpha_wait<NT>(s, t);
+    team_sync<NT>();
     // operands in the canonical K-major layout, K = the tile's 32 points
     // (zero beyond np): 8-row x 4-point core matrices, K-adjacent ones 128
     // bytes apart, 8-row groups 1024 bytes apart; high parts in rows 0..63,
     // low parts in rows 64..127
     unsigned char *Ab = s.aop, *Bb = s.aop + 16384;
-    const int rg_end = (mf + 1 + 7) >> 3;   // row groups past it stay zero (cleared at set-up)
-    static_assert(NT == 512, "16 warps x 4 core matrices of each operand");
-    // warp w: core matrices c = w + 16 i of both operands (row group c / 8,
+    // (row groups of A past rg_end hold what was there: their lanes of the
+    // accumulator are not read; B has none)
+    const int rg_end = tc_arows(mf) >> 3;
+    // warp w: core matrices c = w + (warps) i of both operands (row group c / 8,
     // points 4 (c % 8) .. + 3), the same J element feeding A and B
+    constexpr int NW = NT / 32;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int c = warp + 16 * i, rg = c >> 3, kc = c & 7;
+    for (int i = 0; i < 64 / NW; i++) {
+        const int c = warp + NW * i, rg = c >> 3, kc = c & 7;
         if (rg < rg_end) {
             const int row = rg * 8 + (lane >> 2), p = kc * 4 + (lane & 3);
             float va = 0.f, vb = 0.f;
@@ -1369,13 +1409,13 @@ __device__ void accumulate_tile_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, 
             reinterpret_cast<uint32_t *>(Ab + (rg * 8 + kc) * 128)[lane] = ah;
             reinterpret_cast<uint32_t *>(Ab + ((rg + 8) * 8 + kc) * 128)[lane] = al;
             reinterpret_cast<uint32_t *>(Bb + (rg * 8 + kc) * 128)[lane] = bh;
-            reinterpret_cast<uint32_t *>(Bb + ((rg + 8) * 8 + kc) * 128)[lane] = bl;
+            reinterpret_cast<uint32_t *>(Bb + ((rg + rg_end) * 8 + kc) * 128)[lane] = bl;
         }
     }
     tc::fence_proxy_async();
     tc::fence_before_sync();
-    __syncthreads();
-    tc_alpha_issue(s, t, ob.nfac);
+    team_sync<NT>();
+    tc_alpha_issue<NT>(s, t, mf);
 }
 
 // Adds the alpha accumulator to the FP64 normal matrix M (lower triangle)
@@ -1384,29 +1424,25 @@ __device__ void accumulate_tile_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, 
 template <int NT>
 __device__ void tc_alpha_flush(const DevObject &ob, Smem<PS_FORM_MIXED> &s, double *M, double *bv, TcState &t)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int mf = ob.mfit;
     if (t.afresh) return;
-    tc_alpha_wait(s, t);
+    tc_alpha_wait<NT>(s, t);
     if (*s.abort) return;
     float *S = reinterpret_cast<float *>(s.bhi);   // [128][65], after the tile's contraction
-    {
-        // every warp: 16 of the 64 column pairs of its lane quadrant
-        const int quad = warp & 3, cgrp = warp >> 2;
-        const uint32_t taddr =
-            t.tbase + (static_cast<uint32_t>(quad * 32) << 16) + tc_acol(ob.nfac) + 16 * cgrp;
-        float *sr = S + (quad * 32 + lane) * 65 + 16 * cgrp;
+    // 8 of the column pairs (k, nb + k) of the warp's lane quadrant at a time
+    const int quad = warp & 3, nb = tc_arows(mf);
+    for (int c0 = 8 * (warp >> 2); c0 < nb; c0 += NT / 16) {
+        const uint32_t taddr = t.tbase + (static_cast<uint32_t>(quad * 32) << 16) + t.acol + c0;
+        float *sr = S + (quad * 32 + lane) * 65 + c0;
+        uint32_t vh[8], vl[8];
+        tc::tmem_ld8(taddr, vh);
+        tc::tmem_ld8(taddr + nb, vl);
+        tc::tmem_wait_ld();
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            uint32_t vh[8], vl[8];
-            tc::tmem_ld8(taddr + 8 * q, vh);
-            tc::tmem_ld8(taddr + 64 + 8 * q, vl);
-            tc::tmem_wait_ld();
-#pragma unroll
-            for (int j = 0; j < 8; j++) sr[8 * q + j] = __uint_as_float(vh[j]) + __uint_as_float(vl[j]);
-        }
+        for (int j = 0; j < 8; j++) sr[j] = __uint_as_float(vh[j]) + __uint_as_float(vl[j]);
     }
-    __syncthreads();
+    team_sync<NT>();
     const int ntri = mf * (mf + 1) / 2;
     for (int e = tid; e < ntri; e += NT) {
         const int j = tri_row(e);
@@ -1416,21 +1452,20 @@ __device__ void tc_alpha_flush(const DevObject &ob, Smem<PS_FORM_MIXED> &s, doub
     for (int j = tid; j < mf; j += NT) bv[j] += static_cast<double>(S[j * 65 + mf] + S[(64 + j) * 65 + mf]);
     t.afresh = true;
     tc::fence_before_sync();
-    __syncthreads();
+    team_sync<NT>();
 }
 
 // The parts of an evaluation at parameters a[] that do not depend on the
 // points: facet areas (s.area, s.gv), their sum, the rotation matrices and
 // the phase and scattering parameters (s.bmat), the scale of the tensor-core
 // operand; clears chi^2.  Ends with a barrier.
-template <int FORM, int KU>
+template <int FORM, int KU, int NT>
 __device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double *a)
 {
     using R = typename RealOf<FORM>::T;
     constexpr bool kFP64 = FORM == PS_FORM_FP64;
     constexpr bool kPipe = !kFP64 && (KU == 0 || KU == 3);
-    constexpr int NT = threads_of<FORM>();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int F = ob.nfac, C = ob.ncoef, ma = ob.ma;
     // The scalars' exp, cos and sin on the last warp (the pole angles on two
     // lanes at once), which has no facets on the usual grids, while the
@@ -1446,40 +1481,50 @@ __device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double 
         }
     }
     // curv.c:10-39 -- g_i = exp(sum over (m,l) of P_l^m (c cos + c' sin)), FP64.
-    double asum = 0;
-    for (int i = tid; i < F; i += NT) {
-        double g = 0;
-        if constexpr (kFP64) {
-            for (int q = 0; q < ob.npairs; q++) {
-                int m = ob.pair_m[q], n = ob.pair_n[q];
-                double fsum = a[n] * ob.fc[m * F + i];
-                if (m != 0) fsum = fsum + a[n + 1] * ob.fs[m * F + i];
-                g = g + ob.pleg[q * F + i] * fsum;
-            }
-        } else {
-            // the same sum as the dot product of the facet's FP64 basis row
-            // (Dsph[i][n] = P_l^m cos(m phi_i), Dsph[i][n + 1] = P_l^m
-            // sin(m phi_i)) with the shape coefficients: independent loads
-            // instead of a pair-index chain per term; it rounds differently
-            // from curv.c's order by about 1e-16
-            const double *drow = ob.dsph + static_cast<size_t>(i) * ob.ncoef;
+    // (a team of fewer threads takes the places of several: the area sum's
+    // order is that of the form's full slot)
+    constexpr int NV = threads_of<FORM>();
+#pragma unroll
+    for (int part = 0; part < NV / NT; part++) {
+        const int vt = tid + part * NT;
+        double asum = 0;
+        for (int i = vt; i < F; i += NV) {
+            double g = 0;
+            if constexpr (kFP64) {
+                for (int q = 0; q < ob.npairs; q++) {
+                    int m = ob.pair_m[q], n = ob.pair_n[q];
+                    double fsum = a[n] * ob.fc[m * F + i];
+                    if (m != 0) fsum = fsum + a[n + 1] * ob.fs[m * F + i];
+                    g = g + ob.pleg[q * F + i] * fsum;
+                }
+            } else {
+                // the same sum as the dot product of the facet's FP64 basis row
+                // (Dsph[i][n] = P_l^m cos(m phi_i), Dsph[i][n + 1] = P_l^m
+                // sin(m phi_i)) with the shape coefficients: independent loads
+                // instead of a pair-index chain per term; it rounds differently
+                // from curv.c's order by about 1e-16
+                const double *drow = ob.dsph + static_cast<size_t>(i) * ob.ncoef;
 #pragma unroll 7
-            for (int k = 0; k < ob.ncoef; k++) g = fma(drow[k], a[k], g);
+                for (int k = 0; k < ob.ncoef; k++) g = fma(drow[k], a[k], g);
+            }
+            g = exp(g);
+            double ar = ob.darea[i] * g;
+            s.area[i] = ar;
+            s.gv[i] = g;
+            if constexpr (!kFP64) {
+                if constexpr (kPipe) {
+                    fac_at(s.fac, i, 3) = static_cast<float>(ar);
+                } else {
+                    s.areaR[i] = static_cast<R>(ar);
+                    s.gvR[i] = static_cast<R>(g);
+                }
+            }
+            asum += ar;
         }
-        g = exp(g);
-        double ar = ob.darea[i] * g;
-        s.area[i] = ar;
-        s.gv[i] = g;
-        if constexpr (!kFP64) {
-            s.areaR[i] = static_cast<R>(ar);
-            s.gvR[i] = static_cast<R>(g);
-            if constexpr (kPipe) fac_at(s.fac, i, 3) = static_cast<float>(ar);
-        }
-        asum += ar;
+        asum = warp_sum(asum);
+        if (lane == 0) s.misc[M_RED + (vt >> 5)] = asum;
     }
-    asum = warp_sum(asum);
-    if (lane == 0) s.misc[M_RED + warp] = asum;
-    __syncthreads();
+    team_sync<NT>();
     // Every scalar once, on a warp of its own (an FP64 instruction holds the
     // FP64 unit for the whole warp): the area sum, blmatrix.c:9-46 in FP64
     // from the angles' cos/sin, one entry per lane, stored in the
@@ -1487,7 +1532,7 @@ __device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double 
     if (tid == 0) {
         double t = 0;
 #pragma unroll
-        for (int i = 0; i < NT / 32; i++) t += s.misc[M_RED + i];
+        for (int i = 0; i < NV / 32; i++) t += s.misc[M_RED + i];
         s.misc[M_AREA] = t;
     } else if (warp == 2) {
         R v;
@@ -1515,7 +1560,7 @@ __device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double 
             mx * fmaxf(1.f, fabsf(static_cast<float>(s.misc[M_CL])) + 0.5f * fabsf(static_cast<float>(a[C + 7])));
         if (lane == 0) s.misc[M_WEXP] = (wmax > 0.f && wmax < 1e30f) ? static_cast<double>(13 - ilogbf(wmax)) : 0.0;
     }
-    __syncthreads();
+    team_sync<NT>();
 }
 
 // ---------------------------------------------------------------------------
@@ -1525,7 +1570,7 @@ __device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double 
 // shape_prologue has run at the same parameters already (the chi^2 of an
 // accepted step).
 // ---------------------------------------------------------------------------
-template <int KU>
+template <int KU, int NT>
 __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L,
                                Smem<PS_FORM_MIXED> &s, const double *a, double *M, double *bv, float *scratch,
                                TcState &tcs, bool fresh = true)
@@ -1538,19 +1583,20 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
     // wide tensor-core contraction (KU 3: 65..96 coefficients)
     constexpr bool kTcAlpha = KU == 0;
     constexpr bool kWide = KU == 3;
-    constexpr int NT = threads_of<PS_FORM_MIXED>();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr bool kAlias = NT == kTeamThreads;   // alpha's operands lie over the contraction's (make_layout)
+    static_assert(NT == threads_of<PS_FORM_MIXED>() || KU == 0, "teams: the tensor-core path only");
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int F = ob.nfac, C = ob.ncoef, ma = ob.ma, mf = ob.mfit, P = L.P;
     const int wcols = L.wcols;
     const int RW = rel_row_stride(ma);   // parked row of a relative lightcurve
     const R *nxR = ob.nx_f, *nyR = ob.ny_f, *nzR = ob.nz_f, *dareaR = ob.darea_f;
 
-    if (fresh) shape_prologue<PS_FORM_MIXED, KU>(ob, s, a);
+    if (fresh) shape_prologue<PS_FORM_MIXED, KU, NT>(ob, s, a);
     else if (tid == 0) s.misc[M_CHISQ] = 0;
     for (int e = tid; e < mf * mf; e += NT) M[e] = 0;
     for (int j = tid; j < mf; j += NT) bv[j] = 0;
     const double omg = a[C + 2];
-    __syncthreads();
+    team_sync<NT>();
     const R cls = s.bmat[30], cl = s.bmat[31];
     // power-of-two scales of the tensor-core contraction's operands
     const int wexp = kPipe ? static_cast<int>(s.misc[M_WEXP]) : 0;
@@ -1577,7 +1623,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
             setup_mixed_phase(ob.tim[q], omg, cfg.phi0, pt0);
             setup_mixed_geo(ob.geo_f[2 * q], ob.geo_f[2 * q + 1], s.bmat, pt0);
         }
-        __syncthreads();   // the first tile's facet stage reads it
+        team_sync<NT>();   // the first tile's facet stage reads it
     }
 
     for (int lc = 0; lc < ob.n_lc; lc++) {
@@ -1601,13 +1647,13 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 }
                 // (with the tensor cores the set-up is a tile old: the
                 // barrier after the previous tile's contraction ordered it)
-                if constexpr (!kPipe) __syncthreads();
+                if constexpr (!kPipe) team_sync<NT>();
                 // 2. facet stage (bright.c:59-120), one warp per point
                 if constexpr (kPipe) {
                     // prefetch for the contraction window: the next tile's
                     // times (warp 1) and geometry (warps 2 and 3, a copy
                     // each), this tile's accumulation data (warp 14)
-                    if (kTcAlpha && warp == 14) {
+                    if (kTcAlpha && warp == NT / 32 - 2) {
                         if (!rel && lane < np) {
                             const int q = start + t0 + lane;
                             double *d = reinterpret_cast<double *>(s.pref + kPrefAcc) + 3 * lane;
@@ -1631,6 +1677,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                         }
                         cp_async_commit();
                     }
+                    if constexpr (kAlias) tc_alpha_wait<NT>(s, tcs);   // the operands share their memory
                     facet_stage_tc<NT>(ob, s, np, cl, cls, wscale);
                 }
                 else
@@ -1687,6 +1734,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                     }
                 }
             } else if constexpr (kPipe) {
+                if constexpr (kAlias) tc_alpha_wait<NT>(s, tcs);
                 conv_rows_tc<NT>(ob, s, wscale);
             } else {
                 // convexity rows (conv.c:12-29): W = Darea g n_c, residual =
@@ -1704,7 +1752,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 }
             }
             // (the tensor-core issue below begins with a barrier of its own)
-            if constexpr (!kPipe) __syncthreads();
+            if constexpr (!kPipe) team_sync<NT>();
             // 3. shape contraction and the remaining columns of J
             if constexpr (kPipe) {
                 contract_tc_issue<NT, kWide>(s, F, tcs);   // the work below overlaps the MMAs
@@ -1751,8 +1799,8 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
             if constexpr (kPipe) {
                 // the accumulation's per-point FP64 work (weights, residuals,
                 // chi^2) of an absolute lightcurve or of the convexity rows,
-                // here on warp 14 (its own copy of the model value) while
-                // thread 0 issues the contraction and warp 15 writes the J
+                // here on the last warp but one (its own copy of the model value) while
+                // thread 0 issues the contraction and the last writes the J
                 // columns (same per-point values and reduction as in the
                 // accumulation itself)
                 if (rel && warp == NT / 32 - 1) {
@@ -1809,7 +1857,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 }
                 contract_tc_finish<NT, kWide>(s, np, F, C, ma, conv, tcs, jscale);
             }
-            __syncthreads();
+            team_sync<NT>();
             if (next_setup) {
                 R *t = s.pt;
                 s.pt = s.pt2;
@@ -1817,7 +1865,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
             }
             if (rel) {
                 // 4a. lightcurve sums and a copy of the rows (mrqcof.c:51-88)
-                // (on the tensor-core path warp 15 has parked the model
+                // (on the tensor-core path the last warp has parked the model
                 // values and summed them during the contraction; the FP64
                 // column sums run on sub-partitions 2 and 3)
                 R *dst = scratch + static_cast<size_t>(t0) * RW;
@@ -1836,7 +1884,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                     const double v = warp_sum(lane < np ? s.ym[lane] : 0.0);
                     if (lane == 0) s.misc[M_AVE] += v;
                 }
-                __syncthreads();
+                team_sync<NT>();
                 continue;
             }
             // 5. accumulate (mrqcof.c:106-136)
@@ -1862,7 +1910,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
         // FP64 form divides as the reference does)
         for (int l = tid; l < ma; l += NT) s.davef[l] = static_cast<float>(s.dave[l]);
         if (tid == 0) s.misc[M_INVAVE] = 1.0 / ave;
-        __syncthreads();
+        team_sync<NT>();
         const double inv_ave = s.misc[M_INVAVE];
         if constexpr (kTcAlpha) {
             // The per-point FP64 work of the whole lightcurve at once, one
@@ -1892,10 +1940,10 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 }
                 c2 = warp_sum(c2);
                 if (lane == 0) s.red[warp] = c2;
-                __syncthreads();
+                team_sync<NT>();
                 if (tid == 0)
                     for (int w = 0; w < NT / 32 && (r0 + w) * P < npts; w++) s.misc[M_CHISQ] += s.red[w];
-                if ((r0 + NT / 32) * P < npts) __syncthreads();
+                if ((r0 + NT / 32) * P < npts) team_sync<NT>();
             }
         }
         for (int t0 = 0; t0 < npts; t0 += P) {
@@ -1921,14 +1969,14 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 s.accs[tid] = static_cast<float>(coef);        // consumed before the
                 s.accs[32 + tid] = static_cast<float>(ytr);    // accumulation reuses it
             }
-            __syncthreads();
+            team_sync<NT>();
             for (int e = tid; e < np * ma; e += NT) {
                 const int p = e / ma, l = e - p * ma;
                 const R v = src[static_cast<size_t>(p) * RW + l];
                 const R out = s.accs[p] * (v - s.accs[32 + p] * s.davef[l]);
                 s.J[e] = (l == 0) ? R(0) : out;
             }
-            __syncthreads();
+            team_sync<NT>();
             accumulate_tile(ob, s, np, start + t0, false, conv_sig, accA, accB);
             if (++tiles_since_flush == kTilesPerFlush) {
                 flush_partials(M, bv, mf, accA, accB);
@@ -1938,13 +1986,13 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
     }
     if constexpr (kTcAlpha) tc_alpha_flush<NT>(ob, s, M, bv, tcs);
     else flush_partials(M, bv, mf, accA, accB);
-    __syncthreads();
+    team_sync<NT>();
     // mirror the lower triangle (mrqcof.c:139-141)
     for (int e = tid; e < mf * mf; e += NT) {
         const int j = e / mf, k = e - j * mf;
         if (k > j) M[e] = M[k * mf + j];
     }
-    __syncthreads();
+    team_sync<NT>();
 }
 
 // ---------------------------------------------------------------------------
@@ -2185,7 +2233,7 @@ __device__ void evaluate_fp64(const DevObject &ob, const FitConfig &cfg, const S
     const int RW = rel_row_stride(ma);
     const int ntri = mf * (mf + 1) / 2;
 
-    if (fresh) shape_prologue<PS_FORM_FP64, 1>(ob, s, a);
+    if (fresh) shape_prologue<PS_FORM_FP64, 1, threads_of<PS_FORM_FP64>()>(ob, s, a);
     else if (tid == 0) s.misc[M_CHISQ] = 0;
     for (int e = tid; e < mf * mf; e += NT) M[e] = 0;
     for (int j = tid; j < mf; j += NT) bv[j] = 0;
@@ -2411,7 +2459,7 @@ __device__ void chi2_fp64(const DevObject &ob, const FitConfig &cfg, const SlotL
         cs = static_cast<int>(cgr::this_cluster().num_blocks());
     }
     const int F = ob.nfac, C = ob.ncoef, nreal = ob.n_lc - 1, N = ob.ndata;
-    shape_prologue<PS_FORM_FP64, 1>(ob, s, a);
+    shape_prologue<PS_FORM_FP64, 1, threads_of<PS_FORM_FP64>()>(ob, s, a);
     const Chi2Plan cp = chi2_plan(L, s);
     const int cap = cp.cap, lim = min(cap, kChi2Chunk);
     const double omg = a[C + 2];
@@ -2579,15 +2627,15 @@ __device__ void chi2_fp64(const DevObject &ob, const FitConfig &cfg, const SlotL
 // Measured: 3010 fits of 980 points, 288 facets 290 -> 219 ms; 1010 fits with
 // 81 coefficients, 512 facets 247 -> 171 ms.
 // ---------------------------------------------------------------------------
-template <int KU>
+template <int KU, int NT>
 __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<PS_FORM_MIXED> &s,
                            const double *a)
 {
-    constexpr int NT = threads_of<PS_FORM_MIXED>(), NW = NT / 32, P = 32;
+    constexpr int NW = NT / 32, P = 32;
     constexpr int kTiles = 16 * kRedStride;   // two tile sums each in s.red
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int F = ob.nfac, C = ob.ncoef, nreal = ob.n_lc - 1, N = ob.ndata;
-    shape_prologue<PS_FORM_MIXED, KU>(ob, s, a);
+    shape_prologue<PS_FORM_MIXED, KU, NT>(ob, s, a);
     const int cap = static_cast<int>(2 * (L.blo - L.bhi) > 33280 ? 2 * (L.blo - L.bhi) : 33280) / 32 & ~31;
     float *rec = reinterpret_cast<float *>(s.bhi);   // [7][cap] directions, phase function
     float *ym = rec + 7 * cap;                       // [cap] model values
@@ -2628,7 +2676,7 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
             for (int c = 0; c < 6; c++) rec[c * cap + i] = e[c];
             rec[6 * cap + i] = pt[24];
         }
-        __syncthreads();
+        team_sync<NT>();
         const float2 CL = make_float2(cl, cl), CLS = make_float2(cls, cls);
         const int fl = lane & 3;
         for (int g = warp; g * 8 < n; g += NW) {
@@ -2667,7 +2715,7 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
             }
             if (fl == 0 && i < n) ym[i] = t * rec[6 * cap + i];
         }
-        __syncthreads();
+        team_sync<NT>();
         // sums of the relative lightcurves' model values, a tile per warp
         int k = 0;
         for (int lc = lc0; lc < nreal && ob.lc_start[lc] < q1; lc++) {
@@ -2678,7 +2726,7 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
                 if (lane == 0) tsum[k] = y;
             }
         }
-        __syncthreads();
+        team_sync<NT>();
         // weighted squared residuals (mrqcof.c:90-136); the sums of a
         // relative lightcurve's tiles are read before they are replaced
         k = 0;
@@ -2713,7 +2761,7 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
                 if (lane == 0) c2sum[k] = c2;
             }
         }
-        __syncthreads();
+        team_sync<NT>();
         if (tid == 0) {
             double c = s.misc[M_CHISQ];
 #pragma unroll 4
@@ -2733,7 +2781,7 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
         res = warp_sum(res);
         if (lane == 0) s.misc[M_CHK + warp - 1] = res;
     }
-    __syncthreads();
+    team_sync<NT>();
     if (warp == 0) {
         double c2 = 0;
         if (lane < 3) {
@@ -2744,7 +2792,7 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
         c2 = warp_sum(c2);
         if (lane == 0) s.misc[M_CHISQ] += c2;
     }
-    __syncthreads();
+    team_sync<NT>();
 }
 
 // Gauss-Jordan elimination with full pivoting on A (n x n, row-major in
@@ -2771,12 +2819,12 @@ __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
 {
     constexpr int NW = NT / 32;
     constexpr long long kInfBits = 0x7ff0000000000000LL;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     double *prow = wd, *pcol = wd + n;   // scaled pivot row, pivot column; pcol[n]: the scaled pivot row of b
     int *col[2] = {wi, wi + n};          // columns not yet pivoted, in increasing order
     int *flag = wi + 2 * n;              // 1: row and column not yet pivoted
     int *candi = wi + 3 * n;             // candidates of the warps
-    __shared__ long long candv[NW];
+    long long *candv = reinterpret_cast<long long *>(wd + 2 * n + 1);
     for (int k = tid; k < n; k += NT) {
         col[0][k] = k;
         flag[k] = 1;
@@ -2807,7 +2855,7 @@ __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
             candv[warp] = bv;
             candi[warp] = bi;
         }
-        __syncthreads();
+        team_sync<NT>();
         // every warp takes the best candidate by itself
         bv = lane < NW ? candv[lane] : -1;
         bi = lane < NW ? candi[lane] : -1;
@@ -2845,7 +2893,7 @@ __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
             for (int r = tid - 64; r < n; r += NT - 64) pcol[r] = A[(r == irow ? icol : r) * n + icol];
             if (tid == 64) flag[icol] = 0;
         }
-        __syncthreads();
+        team_sync<NT>();
         bv = -1;
         bi = -1;
         const int m1 = m - 1;
@@ -2886,7 +2934,7 @@ __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
             b[r] = v - pb * pcol[r];
         }
     }
-    __syncthreads();
+    team_sync<NT>();
     return 0;
 }
 
@@ -2949,10 +2997,18 @@ __device__ inline void chol_pivot_pair(double *A, double *b, int n, int j, doubl
     }
 }
 
+// Named barrier of warps 0 and 1 of a team in the Cholesky solve.
+template <int NT>
+__device__ inline int helper_barrier()
+{
+    return NT == kTeamThreads ? 4 + static_cast<int>(threadIdx.x) / kTeamThreads : 1;
+}
+
 // The 2 x 2 block [a bq; bq c] of pair (j, j + 1) and its rows bj, bj1 of
 // b, already updated, in registers of every lane of warp 0: stores 1/L_jj,
 // 1/L_j+1,j+1 (col) and L_j+1,j, arrives on the helper warp's named barrier
 // (the helper scales the columns below), then stores y (b).
+template <int NT>
 __device__ inline void chol_pivot_block(double a, double bq, double c, double bj, double bj1, double *A, double *b,
                                         int n, int j, bool two, double *col, double *flag, int lane)
 {
@@ -2979,7 +3035,7 @@ __device__ inline void chol_pivot_block(double a, double bq, double c, double bj
         }
     }
     // the helper warp may scale the columns now
-    asm volatile("bar.arrive 1, 64;" ::: "memory");
+    asm volatile("bar.arrive %0, 64;" ::"r"(helper_barrier<NT>()) : "memory");
     if (lane == 0 && two) b[j + 1] = (bj1 - l10 * y0) * i1;
 }
 
@@ -2987,14 +3043,14 @@ template <int NT>
 __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *flag)
 {
     static_assert(NT % 128 == 0 && NT >= 256, "whole warps on every sub-partition");
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     // trailing-update workers: the warps of sub-partitions 1..3 but warp 1
     constexpr int kWorkers = (NT / 128 * 3 - 1) * 32;
     const bool worker = (warp & 3) != 0 && warp != 1;
     const int wtid = ((warp >> 2) * 3 + (warp & 3) - 2) * 32 + lane;
-    __syncthreads();
+    team_sync<NT>();
     if (warp == 0) chol_pivot_pair(A, b, n, 0, col, flag, lane);
-    __syncthreads();
+    team_sync<NT>();
     if (*flag == 0.0) return 2;
     for (int j = 0; j + 2 < n; j += 2) {
         // pair (j, j + 1) is factored; b[j], b[j + 1] hold its y
@@ -3020,7 +3076,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
             const double cc = __shfl_sync(0xffffffffu, xu, 2);
             const double bj = __shfl_sync(0xffffffffu, xu, 3);
             const double bj1 = __shfl_sync(0xffffffffu, xu, 4);
-            chol_pivot_block(a, bq, cc, bj, bj1, A, b, n, jn, twon, col, flag, lane);
+            chol_pivot_block<NT>(a, bq, cc, bj, bj1, A, b, n, jn, twon, col, flag, lane);
         } else if (warp == 1) {
             // the rest of the next pair's columns: update now, scale once
             // warp 0 has published the pivot
@@ -3036,7 +3092,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
                 d0 = A[i2 * n + jn] - li0 * p0 - li1 * p1;
                 if (twon) d1 = A[i2 * n + jn + 1] - li0 * q0 - li1 * q1;
             }
-            asm volatile("bar.sync 1, 64;" ::: "memory");
+            asm volatile("bar.sync %0, 64;" ::"r"(helper_barrier<NT>()) : "memory");
             const double i0 = col[jn];
             const double i1 = twon ? col[jn + 1] : 0.0, l10 = twon ? A[(jn + 1) * n + jn] : 0.0;
             if (i < n) {
@@ -3080,7 +3136,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
                 }
             }
         }
-        __syncthreads();
+        team_sync<NT>();
         if (*flag == 0.0) return 2;
     }
     // L^T x = y: with the rows of L scaled, L'_jk = L_jk / L_jj (k < j),
@@ -3091,7 +3147,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
         const int cc = e - r * (r - 1) / 2;
         A[r * n + cc] *= col[r];
     }
-    __syncthreads();
+    team_sync<NT>();
     if (warp == 0) {
         if (n <= 96) {
             double z0 = lane < n ? b[lane] : 0.0, z1 = lane + 32 < n ? b[lane + 32] : 0.0,
@@ -3117,7 +3173,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
             for (int i = lane; i < n; i += 32) b[i] *= col[i];
         }
     }
-    __syncthreads();
+    team_sync<NT>();
     return 0;
 }
 
@@ -3160,7 +3216,7 @@ __device__ float mlp_predict_warp(const float *W, const float *f, float *sh)
 // ---------------------------------------------------------------------------
 // One fit (period_search_BOINC.cpp:817-921 with mrqmin.c:11-110).
 // ---------------------------------------------------------------------------
-template <int FORM, int KU>
+template <int FORM, int KU, int NT = threads_of<FORM>()>
 __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<FORM> &s,
                         typename RealOf<FORM>::T *scratch, int64_t n, int pole, ps_fit *out, const FitWork &w,
                         long long fidx, TcState &tcs, bool split = false)
@@ -3174,7 +3230,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
             if (split) evaluate_fp64<true>(ob, cfg, L, s, a, M, bv, scratch, fresh);
             else evaluate_fp64<false>(ob, cfg, L, s, a, M, bv, scratch, fresh);
         } else {
-            evaluate_mixed<KU>(ob, cfg, L, s, a, M, bv, scratch, tcs, fresh);
+            evaluate_mixed<KU, NT>(ob, cfg, L, s, a, M, bv, scratch, tcs, fresh);
         }
     };
     // chi^2 alone where the form has it (about half of the steps are
@@ -3187,11 +3243,10 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
             if (split) chi2_fp64<true>(ob, cfg, L, s, a);
             else chi2_fp64<false>(ob, cfg, L, s, a);
         } else if constexpr (kTensor) {
-            chi2_mixed<KU>(ob, cfg, L, s, a);
+            chi2_mixed<KU, NT>(ob, cfg, L, s, a);
         }
     };
-    constexpr int NT = threads_of<FORM>();
-    const int tid = threadIdx.x;
+    const int tid = team_thread<NT>();
     const int C = ob.ncoef, ma = ob.ma, mf = ob.mfit;
     const double freq = cfg.freq_start - (n - 1) * cfg.freq_step;
     const double prd = 1 / freq;
@@ -3216,7 +3271,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
         s.cg[i] = v;
         s.atry[i] = v;
     }
-    __syncthreads();
+    team_sync<NT>();
 
     double alamda = -1, ochisq = 0, chisq = 0, rchisq = -1;
     double iter_diff = 1e40, dev_old = 1e30, dev_new = 0;
@@ -3283,7 +3338,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
             s.covar[e] = (j == k) ? s.alpha[e] * (1 + alamda) : s.alpha[e];
         }
         for (int j = tid; j < mf; j += NT) s.da[j] = s.beta[j];
-        __syncthreads();
+        team_sync<NT>();
         int err;
         if constexpr (FORM == PS_FORM_FP64) {
             err = gauss_jordan<NT>(s.covar, s.da, mf, s.col, s.ipiv);
@@ -3298,17 +3353,17 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
                     s.covar[e] = (j == k) ? s.alpha[e] * (1 + alamda) : s.alpha[e];
                 }
                 for (int j = tid; j < mf; j += NT) s.da[j] = s.beta[j];
-                __syncthreads();
+                team_sync<NT>();
                 err = gauss_jordan<NT>(s.covar, s.da, mf, s.col, s.ipiv);
             }
         }
-        __syncthreads();
+        team_sync<NT>();
         if (err == 0) {
             for (int j = tid; j < mf; j += NT) {
                 const int l = ob.free_list[j];
                 s.atry[l] = s.cg[l] + s.da[j];
             }
-            __syncthreads();
+            team_sync<NT>();
             if (lazy) chi2(s.atry);
             else eval(s.atry, s.covar, s.da, true);
             if constexpr (kTensor) {
@@ -3363,7 +3418,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
             s.misc[M_LM + 2] = dev_new;
             s.misc[M_LM + 3] = iter_diff;
         }
-        __syncthreads();
+        team_sync<NT>();
         alamda = s.misc[M_LM];
         ochisq = s.misc[M_LM + 1];
         dev_new = s.misc[M_LM + 2];
@@ -3397,7 +3452,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
                     if (tid == 0) pred_dev = dev_new * exp(static_cast<double>(y));
                 }
             }
-            __syncthreads();
+            team_sync<NT>();
         }
         if (w.iter_limit > 0 && niter >= w.iter_limit) {
             screened = true;
@@ -3444,7 +3499,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
         r.reserved = 0;
         if (out) *out = r;
     }
-    __syncthreads();
+    team_sync<NT>();
 }
 
 template <int FORM, int KU>
@@ -3460,7 +3515,7 @@ __global__ void __launch_bounds__(threads_of<FORM>(), 1)
     if (s.dsph)
         for (int e = threadIdx.x; e < ob.nfac * ob.ncoef; e += NT) s.dsph[e] = ob.dsph_f[e];
     TcState tcs;
-    if constexpr (kTensor) tc_setup<NT, KU == 3>(ob, s, tcs);
+    if constexpr (kTensor) tc_setup<NT, KU == 3>(ob, s, s, tcs);
     // the wide tensor-core path keeps the slot's normal matrix in global memory
     if (L.dsph_smem == kBasisTensorWide) s.alpha = w.alpha_g + static_cast<size_t>(blockIdx.x) * w.alpha_stride;
     R *scratch = L.rels ? reinterpret_cast<R *>(smem + L.rels)
@@ -3487,8 +3542,49 @@ __global__ void __launch_bounds__(threads_of<FORM>(), 1)
         }
         run_fit<FORM, KU>(ob, cfg, L, s, scratch, n, pole, w.out + f, w, f, tcs);
     }
-    if constexpr (kTensor) tc_teardown(s, tcs, ob.nfac);
+    if constexpr (kTensor) tc_teardown<NT>(s, tcs, ob.nfac, ob.mfit);
     if (FORM == PS_FORM_FP64 && threadIdx.x == 0 && w.lit) atomicAdd(w.lit, *lit_counter(s.misc));
+}
+
+// Two fits of the mixed form's tensor-core path side by side on one SM: the
+// CTA's two teams of kTeamThreads threads each run fits from the queue, with
+// their own slot of shared memory, barriers and accumulators; the basis in
+// Tensor Memory is common.  One fit alone leaves the SM idle two cycles of
+// three (barriers, FP64 and MMA latency); two teams fill each other's gaps.
+// A team's kept normal matrix lies in global memory and alpha's operands over
+// the contraction's, so that two slots fit the shared memory.  A fit's
+// results do not depend on which kernel runs it.
+// Measured (980 points, 288 facets): 304 fits 22.8 ms as two launches of one per
+// SM, 18.2 ms here; 3010 fits 217 -> 171 ms; 1510 fits of 817 relative points
+// 126 -> 94 ms.  Issue slots 33 -> 45 % busy; what is left is FP64 and
+// shared-memory latency and the barriers (stalls per issue: wait 2.3, barrier
+// 1.6, short scoreboard 1.5).
+__global__ void __launch_bounds__(threads_of<PS_FORM_MIXED>(), 1)
+    fit_kernel_pair(DevObject ob, FitConfig cfg, FitWork w)
+{
+    constexpr int NT = kTeamThreads, kTeams = kPairFits;
+    extern __shared__ __align__(16) char smem[];
+    const SlotLayout L =
+        make_layout(PS_FORM_MIXED, ob.ma, ob.mfit, ob.nfac, ob.ncoef, 32, kBasisTensor, w.rel_rows, true);
+    const int team = threadIdx.x / NT, slot = blockIdx.x * kTeams + team;
+    Smem<PS_FORM_MIXED> s0 = carve<PS_FORM_MIXED>(smem, L), s = carve<PS_FORM_MIXED>(smem + team * L.bytes, L);
+    TcState tcs;
+    tc_setup<NT>(ob, s0, s, tcs);
+    s.alpha = w.alpha_g + static_cast<size_t>(slot) * w.alpha_stride;
+    float *scratch = L.rels ? reinterpret_cast<float *>(smem + team * L.bytes + L.rels)
+                            : reinterpret_cast<float *>(w.scratch + static_cast<size_t>(slot) * w.scratch_stride);
+    __shared__ long long next[kTeams];
+    for (;;) {
+        if (team_thread<NT>() == 0) next[team] = static_cast<long long>(atomicAdd(w.queue, 1ULL));
+        team_sync<NT>();
+        const long long f = next[team];
+        team_sync<NT>();
+        if (f >= w.nfits || *s.abort) break;
+        const int64_t n = w.period_index ? w.period_index[f] : w.n_lo + f / PS_N_POLES;
+        const int pole = w.period_index ? w.pole[f] : static_cast<int>(f % PS_N_POLES) + 1;
+        run_fit<PS_FORM_MIXED, 0, NT>(ob, cfg, L, s, scratch, n, pole, w.out + f, w, f, tcs);
+    }
+    tc_teardown<NT>(s, tcs, ob.nfac, ob.mfit);
 }
 
 // FP64 fits, each spread over a thread-block cluster (evaluate_fp64): the
@@ -3571,7 +3667,7 @@ __global__ void __launch_bounds__(threads_of<FORM>(), 1) eval_kernel(DevObject o
     if (s.dsph)
         for (int e = threadIdx.x; e < ob.nfac * ob.ncoef; e += NT) s.dsph[e] = ob.dsph_f[e];
     TcState tcs;
-    if constexpr (kTensor) tc_setup<NT, KU == 3>(ob, s, tcs);
+    if constexpr (kTensor) tc_setup<NT, KU == 3>(ob, s, s, tcs);
     for (int i = threadIdx.x; i < ob.ma; i += NT) s.cg[i] = cg[i];
     if (FORM == PS_FORM_FP64 && threadIdx.x == 0) *lit_counter(s.misc) = 0;
     // the wide tensor-core path accumulates straight into the output matrix
@@ -3579,10 +3675,10 @@ __global__ void __launch_bounds__(threads_of<FORM>(), 1) eval_kernel(DevObject o
     __syncthreads();
     R *rows = L.rels ? reinterpret_cast<R *>(smem + L.rels) : reinterpret_cast<R *>(scratch);
     if constexpr (FORM == PS_FORM_FP64) evaluate_fp64<false>(ob, cfg, L, s, s.cg, s.alpha, s.beta, rows, true);
-    else evaluate_mixed<KU>(ob, cfg, L, s, s.cg, s.alpha, s.beta, rows, tcs);
+    else evaluate_mixed<KU, NT>(ob, cfg, L, s, s.cg, s.alpha, s.beta, rows, tcs);
     if constexpr (kTensor) {
         const bool aborted = *s.abort != 0;
-        tc_teardown(s, tcs, ob.nfac);
+        tc_teardown<NT>(s, tcs, ob.nfac, ob.mfit);
         if (aborted) {
             if (threadIdx.x == 0) *chisq = NAN;
             return;
