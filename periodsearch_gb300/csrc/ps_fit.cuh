@@ -994,13 +994,11 @@ __device__ void tc_teardown(Smem<PS_FORM_MIXED> &s, const TcState &t, int F, int
 
 // Issues the alpha/beta MMAs of the operands in s.aop (built and fenced,
 // behind a CTA barrier) and commits them to the alpha barrier.  Called by
-// every thread; thread 0 issues.  (Issuing them from an idle warp during
-// the next contraction window measured no faster: the MMA issue slots of an
-// SM are shared by its threads.)
+// every thread; the elected thread of warp 0 issues.
 template <int NT>
 __device__ inline void tc_alpha_issue(Smem<PS_FORM_MIXED> &s, TcState &t, int mf)
 {
-    if (team_thread<NT>() == 0 && !*s.abort) {
+    if (__shfl_sync(0xffffffffu, team_thread<NT>() >> 5, 0) == 0 && !*s.abort && tc::elect_one()) {
         tc::fence_after_sync();
         const uint32_t idesc = tc::idesc_tf32(128, 2 * tc_arows(mf));
         const uint32_t a0 = tc::smem_u32(s.aop), b0 = tc::smem_u32(s.aop + 16384), d = t.tbase + t.acol;
@@ -1016,41 +1014,46 @@ __device__ inline void tc_alpha_issue(Smem<PS_FORM_MIXED> &s, TcState &t, int mf
 }
 
 // Issues D = A [W_hi; W_lo]^T for the tile as Fp/16 FP16 MMAs of 128 x 64 x
-// 16 (one MMA costs the issuing thread about the same for N = 32 and N = 64,
-// and the same for K = 8 TF32 and K = 16 FP16 elements) and a commit to the
-// barrier.  The facet stage has written the operand: FP16 high parts of W
+// 16 and a commit to the barrier.  The issuing thread is elected
+// (elect.sync in a warp-uniform branch): picked by its number, it took about
+// 70 cycles per MMA whatever the shape, more than the MMAs themselves (18 MMAs
+// of 288 facets: issue 1.8 -> 1.1 kcycles a tile; the wide path's 64: 4.9 ->
+// 2.4; 1010 wide fits 174 -> 165 ms).  The facet stage has written the operand: FP16 high parts of W
 // in rows 0..31, low parts in rows 32..63, canonical K-major layout (8-row x
 // 8-facet core matrices, K-adjacent ones 128 bytes apart).
 template <int NT, bool WIDE = false>
 __device__ void contract_tc_issue(Smem<PS_FORM_MIXED> &s, int F, TcState &t)
 {
-    const int tid = team_thread<NT>();
+    const int tid = team_thread<NT>(), warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int Fp = tc_kpad(F), kcs = Fp >> 3;
     const uint32_t tbase = t.tbase;
     tc::fence_proxy_async();
     tc::fence_before_sync();
     team_sync<NT>();
-    if (tid == 0 && !*s.abort) {
+    if (warp == 0 && !*s.abort && tc::elect_one()) {
         tc::fence_after_sync();
         const uint32_t idesc = tc::idesc_f16(128, 64);
         const uint32_t sbo = static_cast<uint32_t>(kcs) * 128;
-        const uint32_t bh = tc::smem_u32(s.bhi), d = tbase + t.dcol;
-        for (int ks = 0; ks < Fp / 16; ks++) {
-            const uint32_t a = tbase + static_cast<uint32_t>(ks) * 8, off = static_cast<uint32_t>(ks) * 256;
-            tc::mma_f16_ts(d, a, tc::smem_desc(bh + off, 128, sbo), idesc, ks > 0);
-        }
+        const uint32_t d = tbase + t.dcol;
+        const uint64_t b0 = tc::smem_desc(tc::smem_u32(s.bhi), 128, sbo);
+        // one K step: 8 columns of A, 256 bytes (16 in the descriptor) of B
+        const int steps = Fp / 16;
+        tc::mma_f16_ts(d, tbase, b0, idesc, 0);
+#pragma unroll 4
+        for (int ks = 1; ks < steps; ks++) tc::mma_f16_ts(d, tbase + 8u * ks, b0 + 16u * ks, idesc, 1);
         if constexpr (WIDE) {
             // R2 against the W_hi rows (N = 32) of each facet half: the
             // products of lanes 0.. with the first half land in columns
             // 0..31, those of lanes 64.. with the second half in 32..63
             const uint32_t idesc32 = tc::idesc_f16(128, 32), d2 = d + 64, a2 = tbase + tc_r2col(F);
             const int half_steps = Fp / 32;
-            for (int h = 0; h < 2; h++)
-                for (int ks = 0; ks < half_steps; ks++) {
-                    const uint32_t off = static_cast<uint32_t>(h * half_steps + ks) * 256;
-                    tc::mma_f16_ts(d2 + 32u * h, a2 + static_cast<uint32_t>(ks) * 8, tc::smem_desc(bh + off, 128, sbo),
-                                   idesc32, ks > 0);
-                }
+            for (int h = 0; h < 2; h++) {
+                const uint64_t bh = b0 + static_cast<uint64_t>(16 * h * half_steps);
+                tc::mma_f16_ts(d2 + 32u * h, a2, bh, idesc32, 0);
+#pragma unroll 4
+                for (int ks = 1; ks < half_steps; ks++)
+                    tc::mma_f16_ts(d2 + 32u * h, a2 + 8u * ks, bh + 16u * ks, idesc32, 1);
+            }
         }
         tc::mma_commit(s.mbar);
     }

@@ -105,6 +105,19 @@ __device__ inline void tmem_ld8(uint32_t taddr, uint32_t (&v)[8])
 
 __device__ inline void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// True in one thread of the (converged) warp, the same every time: the
+// thread that issues the MMAs.
+__device__ inline bool elect_one()
+{
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
+
 // ---- MMA: D[tmem] (+)= A[tmem] * B[smem]^T, issued by one thread ----
 __device__ inline void mma_tf32_ts(uint32_t d_taddr, uint32_t a_taddr, uint64_t b_desc, uint32_t idesc,
                                    uint32_t accumulate)
