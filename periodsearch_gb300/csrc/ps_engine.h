@@ -187,7 +187,7 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     L.ncoef = ncoef;
     L.P = P;
     L.dsph_smem = dsph_smem;
-    L.wcols = ((nfac > mfit ? nfac : mfit) + 3) & ~3;
+    L.wcols = ((nfac > mfit ? nfac : mfit) + 3) & ~3;   // (mixed form: also the weighted rows' pitch)
     const size_t rs = form == PS_FORM_MIXED ? sizeof(float) : sizeof(double);
     size_t o = 0;
     auto take = [&o](size_t bytes) {
@@ -235,7 +235,7 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
         const size_t tile = static_cast<size_t>(P) * tc_kpad(nfac) * 2;
         size_t readback = 128 * 65 * sizeof(float);
         if (wide) {
-            const size_t wt = static_cast<size_t>(P) * mfit * sizeof(float);
+            const size_t wt = static_cast<size_t>(P) * ((mfit + 3) & ~3) * sizeof(float);
             readback = 2 * 128 * 33 * sizeof(float);
             if (wt > readback) readback = wt;
         }

@@ -462,43 +462,71 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
 }
 
 // Accumulates the rows J[0..np) (model values in ym) of one tile into the
-// normal matrix M (lower triangle), bv and chi^2 (mrqcof.c:106-136).  The
-// SIMT path of the mixed form sums the tile in FP32 and adds the tile sum to
-// the FP64 total: every thread keeps its share of the alpha lower triangle
-// (elements tid + u*512) and of beta (element tid) as FP32 partial sums in
-// registers and adds them to the FP64 totals every few tiles.
-constexpr int kAccPerThread = 8;    // with 512 threads: mfit <= 90
-constexpr int kTilesPerFlush = 8;
+// normal matrix M (lower triangle), bv and chi^2 (mrqcof.c:106-136) on the
+// SIMT pipes of the mixed form: FP32 partial sums, every element over the
+// points in data order, kept in registers and added to the FP64 totals every
+// few tiles.  A warp takes units of 4 rows by 32 columns of the matrix (a
+// lane one column, four rows from one 16-byte broadcast of the weighted
+// rows): two loads for four products, where an element per thread takes two
+// each and waits for shared memory.  Unit u is unit u of the list of row
+// groups' column panels (alpha_unit); warp w takes w, w + 16, ...
+// Measured (87 free parameters): an evaluation's accumulation of 33 tiles 566 -> 280
+// kcycles, 1010 fits 165 -> 148 ms.
 // The tensor-core path's FP32 alpha accumulator in Tensor Memory (products
 // of TF32 high/low parts) is added to the FP64 normal matrix every 16 tiles.
 constexpr int kTcTilesPerFlush = 16;
 
-__device__ inline void flush_partials(double *M, double *bv, int mf, float (&accA)[kAccPerThread], float &accB)
+constexpr int kTilesPerFlush = 8;
+// Units of a warp by kernel variant: at most 45 units (90 free parameters), or
+// 80 with up to 128 coefficients (KU 2).
+template <int KU>
+constexpr int kAlphaUnits = KU == 2 ? 5 : 3;
+
+// Unit u: its first row (a group of four rows has the panels of 32 columns
+// that reach its last row's diagonal) and, in the upper half, its first
+// column; -1 past the end.
+__device__ inline int alpha_unit(int u, int mf)
 {
-    constexpr int NT = threads_of<PS_FORM_MIXED>();
-    const int tid = threadIdx.x;
-    const int ntri = mf * (mf + 1) / 2;
+    for (int r = 0; r < mf; r += 4) {
+        const int panels = (min(r + 4, mf) + 31) / 32;
+        if (u < panels) return r | (32 * u) << 16;
+        u -= panels;
+    }
+    return -1;
+}
+
+// Pitch of the weighted rows (16-byte groups of four).
+PSG_HD inline int alpha_pitch(int mf) { return (mf + 3) & ~3; }
+
+template <int KU>
+__device__ inline void flush_partials(double *M, double *bv, int mf, const int (&unit)[kAlphaUnits<KU>],
+                                      float4 (&accA)[kAlphaUnits<KU>], float &accB)
+{
+    const int tid = threadIdx.x, lane = tid & 31;
 #pragma unroll
-    for (int u = 0; u < kAccPerThread; u++) {
-        const int e = tid + u * NT;
-        if (e < ntri) {
-            const int j = tri_row(e);
-            const int k = e - j * (j + 1) / 2;
-            M[j * mf + k] += static_cast<double>(accA[u]);
+    for (int q = 0; q < kAlphaUnits<KU>; q++) {
+        if (unit[q] >= 0) {
+            const int r0 = unit[q] & 0xffff, k = (unit[q] >> 16) + lane;
+            const float v[4] = {accA[q].x, accA[q].y, accA[q].z, accA[q].w};
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+                if (r0 + r < mf && k <= r0 + r) M[(r0 + r) * mf + k] += static_cast<double>(v[r]);
         }
-        accA[u] = 0.f;
+        accA[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (tid < mf) bv[tid] += static_cast<double>(accB);
     accB = 0.f;
 }
 
+template <int KU>
 __device__ void accumulate_tile(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int np, int q0pt, bool conv,
-                                double conv_sig, float (&accA)[kAccPerThread], float &accB)
+                                double conv_sig, const int (&unit)[kAlphaUnits<KU>],
+                                float4 (&accA)[kAlphaUnits<KU>], float &accB)
 {
     constexpr int NT = threads_of<PS_FORM_MIXED>();
-    const int tid = threadIdx.x;
-    const int ma = ob.ma, mf = ob.mfit;
-    float *wt = s.W;  // [np][mf], reuses the facet-weight tile
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int ma = ob.ma, mf = ob.mfit, mp = alpha_pitch(mf);
+    float *wt = s.W;  // [np][mp], reuses the facet-weight tile
     // per point: FP32 weight sig2i*w and residual; chi^2 of the tile
     // summed over one warp in FP64
     float *dyv = s.accs;
@@ -518,27 +546,31 @@ __device__ void accumulate_tile(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int
         if (tid == 0) s.misc[M_CHISQ] += c2;
     }
     __syncthreads();
-    for (int e = tid; e < np * mf; e += NT) {
-        const int p = e / mf, j = e - p * mf;
-        wt[p * mf + j] = s.J[p * ma + ob.free_list[j]] * wtp[p];
+    for (int e = tid; e < np * mp; e += NT) {
+        const int p = e / mp, j = e - p * mp;
+        wt[e] = j < mf ? s.J[p * ma + ob.free_list[j]] * wtp[p] : 0.f;
     }
     __syncthreads();
-    const int ntri = mf * (mf + 1) / 2;
 #pragma unroll
-    for (int u = 0; u < kAccPerThread; u++) {
-        const int e = tid + u * NT;
-        if (e < ntri) {
-            const int j = tri_row(e);
-            const int k = e - j * (j + 1) / 2;
-            const int lk = ob.free_list[k];
-            float acc = accA[u];
-            for (int p = 0; p < np; p++) acc = fmaf(wt[p * mf + j], s.J[p * ma + lk], acc);
-            accA[u] = acc;
+    for (int q = 0; q < kAlphaUnits<KU>; q++) {
+        if (unit[q] < 0) continue;
+        const float *jc = s.J + ob.free_list[min((unit[q] >> 16) + lane, mf - 1)];
+        const float4 *wr = reinterpret_cast<const float4 *>(wt + (unit[q] & 0xffff));
+        float4 acc = accA[q];
+#pragma unroll 8
+        for (int p = 0; p < np; p++) {
+            const float x = jc[p * ma];
+            const float4 w = wr[p * (mp / 4)];
+            acc.x = fmaf(w.x, x, acc.x);
+            acc.y = fmaf(w.y, x, acc.y);
+            acc.z = fmaf(w.z, x, acc.z);
+            acc.w = fmaf(w.w, x, acc.w);
         }
+        accA[q] = acc;
     }
     if (tid < mf) {
         float acc = accB;
-        for (int p = 0; p < np; p++) acc = fmaf(dyv[p], wt[p * mf + tid], acc);
+        for (int p = 0; p < np; p++) acc = fmaf(dyv[p], wt[p * mp + tid], acc);
         accB = acc;
     }
     __syncthreads();
@@ -1607,10 +1639,15 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
     const float jscale = ldexpf(1.f, -(wexp + tcs.basis_exp));
 
     const double conv_sig = cfg.conv_sig;
-    float accA[kAccPerThread];
+    float4 accA[kAlphaUnits<KU>];
     float accB = 0.f;
 #pragma unroll
-    for (int u = 0; u < kAccPerThread; u++) accA[u] = 0.f;
+    for (int u = 0; u < kAlphaUnits<KU>; u++) accA[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    int unit[kAlphaUnits<KU>];
+    if constexpr (!kTcAlpha) {
+#pragma unroll
+        for (int u = 0; u < kAlphaUnits<KU>; u++) unit[u] = alpha_unit(warp + u * (NT / 32), mf);
+    }
     int tiles_since_flush = 0;
     const float *dsphF = s.dsph ? s.dsph : ob.dsph_f;
     // Point set-up threads.  An FP64 instruction holds its sub-partition's
@@ -1898,9 +1935,9 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                     tiles_since_flush = 0;
                 }
             } else {
-                accumulate_tile(ob, s, np, start + t0, conv, conv_sig, accA, accB);
+                accumulate_tile<KU>(ob, s, np, start + t0, conv, conv_sig, unit, accA, accB);
                 if (++tiles_since_flush == kTilesPerFlush) {
-                    flush_partials(M, bv, mf, accA, accB);
+                    flush_partials<KU>(M, bv, mf, unit, accA, accB);
                     tiles_since_flush = 0;
                 }
             }
@@ -1980,15 +2017,15 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 s.J[e] = (l == 0) ? R(0) : out;
             }
             team_sync<NT>();
-            accumulate_tile(ob, s, np, start + t0, false, conv_sig, accA, accB);
+            accumulate_tile<KU>(ob, s, np, start + t0, false, conv_sig, unit, accA, accB);
             if (++tiles_since_flush == kTilesPerFlush) {
-                flush_partials(M, bv, mf, accA, accB);
+                flush_partials<KU>(M, bv, mf, unit, accA, accB);
                 tiles_since_flush = 0;
             }
         }
     }
     if constexpr (kTcAlpha) tc_alpha_flush<NT>(ob, s, M, bv, tcs);
-    else flush_partials(M, bv, mf, accA, accB);
+    else flush_partials<KU>(M, bv, mf, unit, accA, accB);
     team_sync<NT>();
     // mirror the lower triangle (mrqcof.c:139-141)
     for (int e = tid; e < mf * mf; e += NT) {
