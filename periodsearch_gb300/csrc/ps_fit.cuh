@@ -520,7 +520,7 @@ __device__ inline void flush_partials(double *M, double *bv, int mf, const int (
 
 template <int KU>
 __device__ void accumulate_tile(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int np, int q0pt, bool conv,
-                                double conv_sig, const int (&unit)[kAlphaUnits<KU>],
+                                double conv_sig, bool chi2, const int (&unit)[kAlphaUnits<KU>],
                                 float4 (&accA)[kAlphaUnits<KU>], float &accB)
 {
     constexpr int NT = threads_of<PS_FORM_MIXED>();
@@ -540,10 +540,12 @@ __device__ void accumulate_tile(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int
             const double dy = (conv ? 0.0 : ob.bright[q]) - s.ym[tid];
             dyv[tid] = static_cast<float>(dy);
             wtp[tid] = static_cast<float>(sig2i * wg);
-            c2 = dy * dy * sig2i * wg;
+            if (chi2) c2 = dy * dy * sig2i * wg;
         }
-        c2 = warp_sum(c2);
-        if (tid == 0) s.misc[M_CHISQ] += c2;
+        if (chi2) {
+            c2 = warp_sum(c2);
+            if (tid == 0) s.misc[M_CHISQ] += c2;
+        }
     }
     __syncthreads();
     for (int e = tid; e < np * mp; e += NT) {
@@ -1602,8 +1604,8 @@ __device__ void shape_prologue(const DevObject &ob, Smem<FORM> &s, const double 
 // Mixed form's model evaluation (mrqcof) at parameters a[] into M (mfit x mfit,
 // lower triangle accumulated then mirrored) and vector bv.  Leaves chi^2,
 // the facet-area sum and the convexity residuals in misc.  fresh = false:
-// shape_prologue has run at the same parameters already (the chi^2 of an
-// accepted step).
+// chi2_mixed has just run at the same parameters (an accepted step): neither
+// the shape's terms nor chi^2 are formed again.
 // ---------------------------------------------------------------------------
 template <int KU, int NT>
 __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L,
@@ -1868,10 +1870,12 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                         const double dy = (conv ? 0.0 : pa[2]) - ymv;
                         s.accs[lane] = static_cast<float>(dy);
                         s.accs[32 + lane] = static_cast<float>(sig2i * wg);
-                        c2 = dy * dy * sig2i * wg;
+                        if (fresh) c2 = dy * dy * sig2i * wg;
                     }
-                    c2 = warp_sum(c2);
-                    if (lane == 0) s.misc[M_CHISQ] += c2;
+                    if (fresh) {
+                        c2 = warp_sum(c2);
+                        if (lane == 0) s.misc[M_CHISQ] += c2;
+                    }
                 }
             }
             bool next_setup = false;
@@ -1935,7 +1939,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                     tiles_since_flush = 0;
                 }
             } else {
-                accumulate_tile<KU>(ob, s, np, start + t0, conv, conv_sig, unit, accA, accB);
+                accumulate_tile<KU>(ob, s, np, start + t0, conv, conv_sig, fresh, unit, accA, accB);
                 if (++tiles_since_flush == kTilesPerFlush) {
                     flush_partials<KU>(M, bv, mf, unit, accA, accB);
                     tiles_since_flush = 0;
@@ -1976,8 +1980,9 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                     row[ma] = static_cast<float>(yt * inv_ave);
                     row[ma + 1] = static_cast<float>(dy);
                     row[ma + 2] = static_cast<float>(sig2i * wg);
-                    c2 = dy * dy * sig2i * wg;
+                    if (fresh) c2 = dy * dy * sig2i * wg;
                 }
+                if (!fresh) continue;   // chi^2 is known
                 c2 = warp_sum(c2);
                 if (lane == 0) s.red[warp] = c2;
                 team_sync<NT>();
@@ -2017,7 +2022,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 s.J[e] = (l == 0) ? R(0) : out;
             }
             team_sync<NT>();
-            accumulate_tile<KU>(ob, s, np, start + t0, false, conv_sig, unit, accA, accB);
+            accumulate_tile<KU>(ob, s, np, start + t0, false, conv_sig, fresh, unit, accA, accB);
             if (++tiles_since_flush == kTilesPerFlush) {
                 flush_partials<KU>(M, bv, mf, unit, accA, accB);
                 tiles_since_flush = 0;
