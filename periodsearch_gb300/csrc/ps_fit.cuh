@@ -2661,12 +2661,11 @@ __device__ void chi2_fp64(const DevObject &ob, const FitConfig &cfg, const SlotL
 // chi^2 alone at parameters a[], tensor-core paths of the mixed form (the
 // counterpart of chi2_fp64: what decides whether a step is accepted).  No
 // contraction, no derivative sums, and so no operand tile and no per-tile
-// barriers: set-up with a thread per point, brightness with a warp per 8
+// barriers: set-up with a thread per point, brightness with a warp per 16
 // points, residuals with a warp per 32-point tile, one thread's ordered sum.
 // Each value by evaluate's operations in their order (a point's brightness:
 // facet_stage_tc's four lanes and four facet quarters; chi^2: tile sums in
-// tile order), so chi^2 is evaluate's bit for bit.  The four quarters of a
-// point run side by side in a lane (four independent chains).
+// tile order), so chi^2 is evaluate's bit for bit.
 // Buffers in the operand region (at least 1040 points: any relative
 // lightcurve fits).
 // Measured: 3010 fits of 980 points, 288 facets 290 -> 219 ms; 1010 fits with
@@ -2724,41 +2723,68 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
         team_sync<NT>();
         const float2 CL = make_float2(cl, cl), CLS = make_float2(cls, cls);
         const int fl = lane & 3;
-        for (int g = warp; g * 8 < n; g += NW) {
-            const int i = g * 8 + (lane >> 2);
-            float e[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (i < n) {
+        // a lane takes two points (one facet load for both: with one point the
+        // pass waits for shared memory) and two quarters at a time, four
+        // independent chains (3010 fits 168 -> 161 ms)
+        for (int g = warp; g * 16 < n; g += NW) {
+            float2 E1[2], E2[2], E3[2], F1[2], F2[2], F3[2];
 #pragma unroll
-                for (int c = 0; c < 6; c++) e[c] = rec[c * cap + i];
-            }
-            const float2 E1 = make_float2(e[0], e[0]), E2 = make_float2(e[1], e[1]), E3 = make_float2(e[2], e[2]);
-            const float2 F1 = make_float2(e[3], e[3]), F2 = make_float2(e[4], e[4]), F3 = make_float2(e[5], e[5]);
-            float2 br[4];
+            for (int k = 0; k < 2; k++) {
+                const int i = g * 16 + 8 * k + (lane >> 2);
+                float e[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                if (i < n) {
 #pragma unroll
-            for (int h = 0; h < 4; h++) br[h] = make_float2(0.f, 0.f);
-#pragma unroll 1
-            for (int kc = 0; kc < cq; kc++) {
-#pragma unroll
-                for (int h = 0; h < 4; h++) {
-                    const float4 *fp = s.fac + (h * cq + kc) * 8 + 2 * fl;
-                    const float4 fa = fp[0], fb = fp[1];
-                    const LitPair lp(fa, fb, E1, E2, E3, F1, F2, F3);
-                    // the product rounded by itself, as in facet_stage_tc
-                    // (which uses it twice): a paired product is fused into
-                    // the paired addition, scalar ones are not
-                    const float2 sv = lp.law(CL, CLS);
-                    br[h] = __fadd2_rn(br[h], make_float2(__fmul_rn(lp.ax.x, sv.x), __fmul_rn(lp.ax.y, sv.y)));
+                    for (int c = 0; c < 6; c++) e[c] = rec[c * cap + i];
                 }
+                E1[k] = make_float2(e[0], e[0]);
+                E2[k] = make_float2(e[1], e[1]);
+                E3[k] = make_float2(e[2], e[2]);
+                F1[k] = make_float2(e[3], e[3]);
+                F2[k] = make_float2(e[4], e[4]);
+                F3[k] = make_float2(e[5], e[5]);
             }
-            float t = 0.f;
+            float t[2] = {0.f, 0.f};
+#pragma unroll 1
+            for (int h0 = 0; h0 < 4; h0 += 2) {
+                float2 br[2][2];
 #pragma unroll
-            for (int h = 0; h < 4; h++) {
-                float v = br[h].x + br[h].y;
-                v += __shfl_xor_sync(0xffffffffu, v, 1);
-                v += __shfl_xor_sync(0xffffffffu, v, 2);
-                t += v;
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++) br[h][k] = make_float2(0.f, 0.f);
+#pragma unroll 1
+                for (int kc = 0; kc < cq; kc++) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const float4 *fp = s.fac + ((h0 + h) * cq + kc) * 8 + 2 * fl;
+                        const float4 fa = fp[0], fb = fp[1];
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            const LitPair lp(fa, fb, E1[k], E2[k], E3[k], F1[k], F2[k], F3[k]);
+                            // the product rounded by itself, as in
+                            // facet_stage_tc (which uses it twice): a paired
+                            // product is fused into the paired addition,
+                            // scalar ones are not
+                            const float2 sv = lp.law(CL, CLS);
+                            br[h][k] = __fadd2_rn(br[h][k],
+                                                  make_float2(__fmul_rn(lp.ax.x, sv.x), __fmul_rn(lp.ax.y, sv.y)));
+                        }
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        float v = br[h][k].x + br[h][k].y;
+                        v += __shfl_xor_sync(0xffffffffu, v, 1);
+                        v += __shfl_xor_sync(0xffffffffu, v, 2);
+                        t[k] += v;
+                    }
             }
-            if (fl == 0 && i < n) ym[i] = t * rec[6 * cap + i];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int i = g * 16 + 8 * k + (lane >> 2);
+                if (fl == 0 && i < n) ym[i] = t[k] * rec[6 * cap + i];
+            }
         }
         team_sync<NT>();
         // sums of the relative lightcurves' model values, a tile per warp
