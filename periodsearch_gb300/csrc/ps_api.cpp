@@ -727,7 +727,12 @@ ps_status upload_object(std::unique_ptr<ps_ctx> &c, ps_ctx **out)
            o_cgf = pk.add(o.cg_first), o_dsf = pk.add(dsph_f), o_alp = pk.add(alpha_pt), o_nxf = pk.add(nx_f),
            o_nyf = pk.add(ny_f), o_nzf = pk.add(nz_f), o_daf = pk.add(darea_f), o_s2i = pk.add(sig2i), o_geo = pk.add(geo_f);
     c->h2d_bytes = static_cast<int64_t>(pk.bytes.size());
-    PSG_CUDA(cp, cudaMalloc(&c->d_tables, pk.bytes.size()));
+    // the tensor-core paths' basis operand behind the tables, formed on the device
+    const bool narrow = psg::tensor_basis_ok(F, o.ncoef, o.mfit, 32);
+    const bool wide = !narrow && psg::tensor_wide_ok(F, o.ncoef, o.mfit, 32);
+    const size_t o_basis = (pk.bytes.size() + 255) & ~size_t(255);
+    const size_t basis_bytes = narrow || wide ? psg::basis_words(F, wide) * sizeof(uint32_t) : 0;
+    PSG_CUDA(cp, cudaMalloc(&c->d_tables, o_basis + basis_bytes));
     PSG_CUDA(cp, cudaMemcpyAsync(c->d_tables, pk.bytes.data(), pk.bytes.size(), cudaMemcpyHostToDevice, c->stream));
     char *b = c->d_tables;
     psg::DevObject &d = c->dob;
@@ -773,6 +778,15 @@ ps_status upload_object(std::unique_ptr<ps_ctx> &c, ps_ctx **out)
     d.darea_f = reinterpret_cast<const float *>(b + o_daf);
     d.sig2i = reinterpret_cast<const double *>(b + o_s2i);
     d.geo_f = reinterpret_cast<const float4 *>(b + o_geo);
+    if (basis_bytes > 0) {
+        double mx = 0;
+        for (double v : s.dsph) mx = std::max(mx, std::fabs(v));
+        d.basis_exp = (mx > 0.0 && mx < 1e300) ? 13 - std::ilogb(mx) : 0;
+        d.basis_tc = reinterpret_cast<const uint32_t *>(b + o_basis);
+        const int be = psg::launch_basis(d.dsph, F, o.ncoef, d.basis_exp, wide,
+                                         reinterpret_cast<uint32_t *>(b + o_basis), c->stream);
+        if (be != 0) return cuda_fail(cp, static_cast<cudaError_t>(be), "basis operand");
+    }
 
     ps_status pst = make_plan(cp, c->opt.form);
     if (pst != PS_OK) {

@@ -235,6 +235,48 @@ int launch_fits(int form, const DevObject &ob, const FitConfig &cfg, const FitWo
     return static_cast<int>(cudaGetLastError());
 }
 
+namespace {
+// The basis operand A of the contraction, one word (facets 2j, 2j + 1 as FP16
+// pair) per lane and Tensor Memory column.  Narrow path, column j: lane m < 64
+// holds coefficient m's high part, lane 64 + m what remains of it, the basis
+// scaled by 2^bexp (the largest magnitude just below 2^14, so that the low
+// parts stay normal FP16 numbers for elements down to 2^-3 of it).  Wide
+// path: R1 column j: lanes 0 .. C-1 the high parts, lanes C .. 127 the low
+// parts of the first 128 - C coefficients; R2 column j: the low parts of the
+// others, the first facet half in lanes 0 .., the second in lanes 64 ...
+__global__ void basis_kernel(const double *dsph, int F, int C, double bscale, int wide, uint32_t *words)
+{
+    const int m = threadIdx.x, Fp = tc_kpad(F);
+    int j = blockIdx.x, c, i;
+    bool low;
+    if (wide && j >= Fp / 2) {
+        j -= Fp / 2;
+        const int L1 = 128 - C, n2 = C - L1;
+        c = (m & 63) < n2 ? L1 + (m & 63) : -1;
+        i = (m >> 6) * (Fp / 2) + 2 * j;
+        low = true;
+    } else {
+        low = wide ? m >= C : m >= 64;
+        c = wide ? (low ? m - C : m) : m & 63;
+        i = 2 * j;
+    }
+    float v[2];
+    for (int u = 0; u < 2; u++) {
+        const double d = (c >= 0 && c < C && i + u < F) ? dsph[static_cast<size_t>(i + u) * C + c] * bscale : 0.0;
+        const float hi = tc::round_f16(static_cast<float>(d));
+        v[u] = low ? static_cast<float>(d - static_cast<double>(hi)) : hi;
+    }
+    words[static_cast<size_t>(blockIdx.x) * 128 + m] = tc::pack_f16x2(v[0], v[1]);
+}
+}  // namespace
+
+int launch_basis(const double *dsph, int nfac, int ncoef, int basis_exp, bool wide, uint32_t *words, void *stream)
+{
+    basis_kernel<<<static_cast<unsigned>(basis_words(nfac, wide) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+        dsph, nfac, ncoef, ldexp(1.0, basis_exp), wide ? 1 : 0, words);
+    return static_cast<int>(cudaGetLastError());
+}
+
 // As set_kernel_smem, for the kernel with two fits per CTA.
 int set_pair_smem(size_t smem)
 {

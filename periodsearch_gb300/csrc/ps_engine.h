@@ -34,6 +34,8 @@ struct DevObject {
     const int *free_list;                // [mfit]
     const double *cg_first;              // [ncoef]
     const float *dsph_f;                 // [nfac][ncoef] FP32 copy for the mixed form
+    const uint32_t *basis_tc;            // tensor-core paths: [columns][128 lanes] basis operand (launch_basis)
+    int basis_exp;                       // held scaled by 2^basis_exp
     const float4 *geo_f;                 // [ndata][2] FP32 (ee, alpha), (ee0, 0) for the mixed form
 };
 
@@ -282,6 +284,13 @@ PSG_HD inline int tc_arows(int mfit) { return (mfit + 1 + 7) & ~7; }
 // Launchers (ps_engine.cu).  All enqueue on `stream`; return cudaError_t as int.
 int launch_fits(int form, const DevObject &ob, const FitConfig &cfg, const FitWork &w, int grid,
                 int P, size_t smem, int dsph_smem, void *stream);
+// Forms the basis operand of an object's tensor-core path (wide: the path of
+// 65..96 coefficients) at `words`, basis_words(nfac, wide) FP16 pairs.
+int launch_basis(const double *dsph, int nfac, int ncoef, int basis_exp, bool wide, uint32_t *words, void *stream);
+inline size_t basis_words(int nfac, bool wide)
+{
+    return static_cast<size_t>(128) * (wide ? 3 * (tc_kpad(nfac) / 4) : tc_kpad(nfac) / 2);
+}
 // Mixed fits (tensor-core path), two side by side on each CTA: w.rel_rows,
 // w.scratch and w.alpha_g are those of kPairFits slots per CTA.
 int launch_fits_pair(const DevObject &ob, const FitConfig &cfg, const FitWork &w, int grid, size_t smem, void *stream);

@@ -917,37 +917,26 @@ __device__ inline void tc_alpha_wait(Smem<PS_FORM_MIXED> &s, TcState &t)
 }
 
 // Allocates the CTA's Tensor Memory (s0: the shared memory of its first
-// team), initialises the team's barriers, stages the team's facet constants (zero for the padding facets) and loads the basis into
-// Tensor Memory as A = [Dsph_hi^T; Dsph_lo^T]: lane m < 64 holds coefficient
-// m, lane 64 + m what remains of it, both FP16 and scaled by 2^basis_exp
-// (the largest magnitude just below 2^14, so that the low parts stay normal
-// FP16 numbers for elements down to 2^-3 of it); column j holds facets 2j
-// and 2j + 1.
+// team), initialises the team's barriers, stages the team's facet constants
+// (zero for the padding facets) and loads the basis operand into Tensor
+// Memory.  The operand is formed once per object (basis_words): formed here
+// from the FP64 basis, its conversions took about 45 us of every launch.
 template <int NT, bool WIDE = false>
 __device__ void tc_setup(const DevObject &ob, Smem<PS_FORM_MIXED> &s0, Smem<PS_FORM_MIXED> &s, TcState &t)
 {
-    constexpr int NC = threads_of<PS_FORM_MIXED>(), kTeams = NC / NT;   // the CTA's threads and teams
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int kTeams = kSlotThreads / NT;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const int ttid = team_thread<NT>(), team = tid / NT;
-    const int F = ob.nfac, C = ob.ncoef, Fp = tc_kpad(F);
+    const int F = ob.nfac, Fp = tc_kpad(F);
     if (warp == 0) tc::tmem_alloc(s0.tslot, tc_cols(F, ob.mfit, WIDE, kTeams));
     if (ttid == 0) {
         tc::mbar_init(s.mbar, 1);
         tc::mbar_init(s.mbar2, 1);
         *s.abort = 0;
     }
-    double mx = 0.0;
-    for (int e = tid; e < F * C; e += NC) mx = fmax(mx, fabs(ob.dsph[e]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) s0.red[warp] = mx;
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    mx = 0.0;
-    for (int w = 0; w < NC / 32; w++) mx = fmax(mx, s0.red[w]);
-    const int bexp = (mx > 0.0 && mx < 1e300) ? 13 - ilogb(mx) : 0;
-    const double bscale = ldexp(1.0, bexp);
     const uint32_t tbase = *s0.tslot;
     for (int i = ttid; i < Fp; i += NT) {
         fac_at(s.fac, i, 0) = i < F ? ob.nx_f[i] : 0.f;
@@ -956,56 +945,23 @@ __device__ void tc_setup(const DevObject &ob, Smem<PS_FORM_MIXED> &s0, Smem<PS_F
         fac_at(s.fac, i, 3) = 0.f;
     }
     for (int j = ttid; j < ob.mfit; j += NT) s.flist[j] = ob.free_list[j];
-    if (warp < 4) {
-        // lane m of R1: coefficient c, high part (low = false) or low part;
-        // lane m of R2 (wide path): low part of coefficient c2 for the
-        // facet half h2 (-1: unused lane)
-        const int m = warp * 32 + lane;
-        int c, c2 = -1, h2 = 0;
-        bool low;
-        if constexpr (WIDE) {
-            const int L1 = 128 - C, n2 = C - L1;
-            low = m >= C;
-            c = low ? m - C : m;
-            if ((m & 63) < n2) {
-                c2 = L1 + (m & 63);
-                h2 = m >> 6;
-            }
-        } else {
-            c = m & 63;
-            low = m >= 64;
-        }
-        const uint32_t row = tbase + (static_cast<uint32_t>(warp * 32) << 16);
-        auto part = [&](int cc, int i, bool lo) {
-            const double d = (cc >= 0 && cc < C && i < F) ? ob.dsph[static_cast<size_t>(i) * C + cc] * bscale : 0.0;
-            const float hi = tc::round_f16(static_cast<float>(d));
-            return lo ? static_cast<float>(d - static_cast<double>(hi)) : hi;
-        };
-        for (int j0 = 0; j0 < Fp / 2; j0 += 8) {
-            uint32_t v[8];
+    // lanes 32 (warp % 4) .. + 31, eight columns at a time, the warps of a
+    // lane quarter in turn
+    const uint32_t row = tbase + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const uint32_t *src = ob.basis_tc + (tid & 127);
+    const int cols = WIDE ? 3 * (Fp / 4) : Fp / 2;
+    for (int j0 = 8 * (warp >> 2); j0 < cols; j0 += kSlotThreads / 16) {
+        uint32_t v[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = tc::pack_f16x2(part(c, 2 * (j0 + j), low), part(c, 2 * (j0 + j) + 1, low));
-            tc::tmem_st8(row + static_cast<uint32_t>(j0), v);
-        }
-        if constexpr (WIDE) {
-            // R2 column j: facets 2j, 2j + 1 of the lane's facet half
-            for (int j0 = 0; j0 < Fp / 4; j0 += 8) {
-                uint32_t v[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int i = h2 * (Fp / 2) + 2 * (j0 + j);
-                    v[j] = tc::pack_f16x2(part(c2, i, true), part(c2, i + 1, true));
-                }
-                tc::tmem_st8(row + tc_r2col(F) + static_cast<uint32_t>(j0), v);
-            }
-        }
-        tc::tmem_wait_st();
+        for (int j = 0; j < 8; j++) v[j] = src[static_cast<size_t>(j0 + j) * 128];
+        tc::tmem_st8(row + static_cast<uint32_t>(j0), v);
     }
+    tc::tmem_wait_st();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     t.tbase = tbase;
-    t.basis_exp = bexp;
+    t.basis_exp = ob.basis_exp;
     t.wide = WIDE;
     t.dcol = tc_dcol(F, WIDE) + 64u * team;
     t.acol = tc_dcol(F) + 64u * kTeams + static_cast<uint32_t>(2 * tc_arows(ob.mfit) * team);
