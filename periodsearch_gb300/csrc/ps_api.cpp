@@ -57,6 +57,7 @@ struct ps_ctx {
     size_t list_cap = 0;
     int64_t launch_total = 0;   // fit-kernel launches since ps_prepare
     double *d_eval = nullptr;          // cg, alpha, beta, chisq, area of ps_eval
+    std::vector<double> h_eval;        // its results on the host
     double *d_state = nullptr;         // saved LM states of screened fits (learned scan)
     size_t state_cap = 0;              // fits
     int64_t *d_slot = nullptr;         // state rows of resumed fits
@@ -970,12 +971,16 @@ ps_status ps_eval(ps_ctx *c, double conw_r, const double *cg, double *alpha, dou
                    : psg::launch_eval(c->opt.form, c->dob, cfg, d_cg, d_al, d_be, d_c2, d_ar, c->d_scratch, c->P,
                                       c->smem, c->dsph_smem, c->rel_rows, c->stream);
     if (e != 0) return cuda_fail(c, static_cast<cudaError_t>(e), "eval kernel launch");
-    PSG_CUDA(c, cudaMemcpyAsync(alpha, d_al, static_cast<size_t>(mf) * mf * sizeof(double), cudaMemcpyDeviceToHost,
-                                c->stream));
-    PSG_CUDA(c, cudaMemcpyAsync(beta, d_be, mf * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    PSG_CUDA(c, cudaMemcpyAsync(chisq, d_c2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (area) PSG_CUDA(c, cudaMemcpyAsync(area, d_ar, F * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    // alpha, beta, chi^2 and the areas lie one after the other: one copy
+    const size_t n_al = static_cast<size_t>(mf) * mf, n_out = n_al + mf + 1 + (area ? F : 0);
+    c->h_eval.resize(n_out);
+    PSG_CUDA(c, cudaMemcpyAsync(c->h_eval.data(), d_al, n_out * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     PSG_CUDA(c, cudaStreamSynchronize(c->stream));
+    const double *h = c->h_eval.data();
+    std::copy(h, h + n_al, alpha);
+    std::copy(h + n_al, h + n_al + mf, beta);
+    *chisq = h[n_al + mf];
+    if (area) std::copy(h + n_al + mf + 1, h + n_out, area);
     return PS_OK;
 }
 
