@@ -2984,8 +2984,11 @@ __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
 // element and of the block's determinant) in one lane-parallel sequence.
 // The back substitution runs on warp 0 with b in registers and the rows of
 // L pre-scaled by their reciprocal diagonal.  Returns 2 when a pivot is not
-// positive.
-__device__ inline void chol_pivot_pair(double *A, double *b, int n, int j, double *col, double *flag, int lane)
+// positive (an integer flag: a comparison of doubles by every warp holds the
+// FP64 units for 256 cycles a step).  Bound by a pair's chain of dependent FP64
+// operations.  Measured (n = 55): the factorisation 74 -> 64 kcycles with the
+// flag, the selected loads and the pivot's factors formed by the helper itself.
+__device__ inline void chol_pivot_pair(double *A, double *b, int n, int j, double *col, int *flag, int lane)
 {
     const bool two = j + 1 < n;
     const double a = A[j * n + j];
@@ -3008,7 +3011,7 @@ __device__ inline void chol_pivot_pair(double *A, double *b, int n, int j, doubl
     const double i1 = __shfl_sync(0xffffffffu, v, 3);
     const bool ok = (okm & 1u) && (!two || (okm & 2u));
     if (lane == 0) {
-        *flag = ok ? 1.0 : 0.0;
+        *flag = ok ? 1 : 0;
         col[j] = i0;
         b[j] = y0;
         if (two) {
@@ -3032,16 +3035,22 @@ __device__ inline int helper_barrier()
 }
 
 // The 2 x 2 block [a bq; bq c] of pair (j, j + 1) and its rows bj, bj1 of
-// b, already updated, in registers of every lane of warp 0: stores 1/L_jj,
-// 1/L_j+1,j+1 (col) and L_j+1,j, arrives on the helper warp's named barrier
-// (the helper scales the columns below), then stores y (b).
+// b, already updated, in registers of every lane of warp 0: publishes the two
+// reciprocal square roots and arrives on the helper warp's named barrier (the
+// helper forms the pivot's factors itself, two dependent operations sooner, and
+// scales the columns below), then stores 1/L_jj, 1/L_j+1,j+1 (col), L_j+1,j and
+// y (b).
 template <int NT>
 __device__ inline void chol_pivot_block(double a, double bq, double c, double bj, double bj1, double *A, double *b,
-                                        int n, int j, bool two, double *col, double *flag, int lane)
+                                        int n, int j, bool two, double *col, double *pub, int *flag, int lane)
 {
     const double x = lane == 1 ? fma(a, c, -(bq * bq)) : a;
     const bool okx = x > 0.0;
+    if (lane >= 2 && lane < 4) pub[lane] = lane == 2 ? a : bq;
     const double r = okx ? rsqrt(x) : 0.0;
+    if (lane < 2) pub[lane] = r;
+    // the helper warp may scale the columns now
+    asm volatile("bar.arrive %0, 64;" ::"r"(helper_barrier<NT>()) : "memory");
     const unsigned okm = __ballot_sync(0xffffffffu, okx);
     const double i0 = __shfl_sync(0xffffffffu, r, 0);
     const double rd = __shfl_sync(0xffffffffu, r, 1);
@@ -3053,7 +3062,7 @@ __device__ inline void chol_pivot_block(double a, double bq, double c, double bj
     const double i1 = __shfl_sync(0xffffffffu, v, 3);
     const bool ok = (okm & 1u) && (!two || (okm & 2u));
     if (lane == 0) {
-        *flag = ok ? 1.0 : 0.0;
+        *flag = ok ? 1 : 0;
         col[j] = i0;
         b[j] = y0;
         if (two) {
@@ -3061,24 +3070,23 @@ __device__ inline void chol_pivot_block(double a, double bq, double c, double bj
             A[(j + 1) * n + j] = l10;
         }
     }
-    // the helper warp may scale the columns now
-    asm volatile("bar.arrive %0, 64;" ::"r"(helper_barrier<NT>()) : "memory");
     if (lane == 0 && two) b[j + 1] = (bj1 - l10 * y0) * i1;
 }
 
 template <int NT>
-__device__ int cholesky_solve(double *A, double *b, int n, double *col, double *flag)
+__device__ int cholesky_solve(double *A, double *b, int n, double *col, int *flag)
 {
     static_assert(NT % 128 == 0 && NT >= 256, "whole warps on every sub-partition");
     const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     // trailing-update workers: the warps of sub-partitions 1..3 but warp 1
     constexpr int kWorkers = (NT / 128 * 3 - 1) * 32;
     const bool worker = (warp & 3) != 0 && warp != 1;
+    double *pub = col + n;   // published for the helper: both reciprocal square roots, a, bq
     const int wtid = ((warp >> 2) * 3 + (warp & 3) - 2) * 32 + lane;
     team_sync<NT>();
     if (warp == 0) chol_pivot_pair(A, b, n, 0, col, flag, lane);
     team_sync<NT>();
-    if (*flag == 0.0) return 2;
+    if (*flag == 0) return 2;
     for (int j = 0; j + 2 < n; j += 2) {
         // pair (j, j + 1) is factored; b[j], b[j + 1] hold its y
         const bool two = j + 1 < n;
@@ -3090,20 +3098,23 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
         if (warp == 0) {
             // the next pair's 2 x 2 block and rows of b, one value per lane
             // (lane 0: a, 1: bq, 2: c, 3: b_jn, 4: b_jn+1), then its pivot
+            // (selected, not branched on)
             const double y0 = b[j], y1 = two ? b[j + 1] : 0.0;
-            double xv = 0.0, u1 = 0.0, v1 = 0.0, u2 = 0.0, v2 = 0.0;
-            if (lane == 0) { xv = A[jn * n + jn]; u1 = p0; v1 = p0; u2 = p1; v2 = p1; }
-            if (lane == 1 && twon) { xv = A[(jn + 1) * n + jn]; u1 = q0; v1 = p0; u2 = q1; v2 = p1; }
-            if (lane == 2) { xv = twon ? A[(jn + 1) * n + jn + 1] : 1.0; u1 = q0; v1 = q0; u2 = q1; v2 = q1; }
-            if (lane == 3) { xv = b[jn]; u1 = p0; v1 = y0; u2 = p1; v2 = y1; }
-            if (lane == 4 && twon) { xv = b[jn + 1]; u1 = q0; v1 = y0; u2 = q1; v2 = y1; }
+            const bool second = lane == 1 || lane == 2 || lane == 4;   // a value of row jn + 1
+            const bool isb = lane == 3 || lane == 4;
+            const int row = jn + (twon && second ? 1 : 0);
+            const double *at = isb ? b + row : A + row * n + jn + (lane == 2 && twon ? 1 : 0);
+            double xv = lane < 5 ? *at : 0.0;
+            if (second && !twon) xv = lane == 2 ? 1.0 : 0.0;
+            const double u1 = second ? q0 : p0, u2 = second ? q1 : p1;
+            const double v1 = isb ? y0 : lane == 2 ? q0 : p0, v2 = isb ? y1 : lane == 2 ? q1 : p1;
             const double xu = xv - u1 * v1 - u2 * v2;
             const double a = __shfl_sync(0xffffffffu, xu, 0);
             const double bq = __shfl_sync(0xffffffffu, xu, 1);
             const double cc = __shfl_sync(0xffffffffu, xu, 2);
             const double bj = __shfl_sync(0xffffffffu, xu, 3);
             const double bj1 = __shfl_sync(0xffffffffu, xu, 4);
-            chol_pivot_block<NT>(a, bq, cc, bj, bj1, A, b, n, jn, twon, col, flag, lane);
+            chol_pivot_block<NT>(a, bq, cc, bj, bj1, A, b, n, jn, twon, col, pub, flag, lane);
         } else if (warp == 1) {
             // the rest of the next pair's columns: update now, scale once
             // warp 0 has published the pivot
@@ -3120,8 +3131,9 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
                 if (twon) d1 = A[i2 * n + jn + 1] - li0 * q0 - li1 * q1;
             }
             asm volatile("bar.sync %0, 64;" ::"r"(helper_barrier<NT>()) : "memory");
-            const double i0 = col[jn];
-            const double i1 = twon ? col[jn + 1] : 0.0, l10 = twon ? A[(jn + 1) * n + jn] : 0.0;
+            // L_jn+1,jn and 1/L_jn+1,jn+1 as warp 0 forms them
+            const double i0 = pub[0];
+            const double i1 = twon ? pub[2] * i0 * pub[1] : 0.0, l10 = twon ? pub[3] * i0 : 0.0;
             if (i < n) {
                 const double a0 = c0 * i0;
                 A[i * n + jn] = a0;
@@ -3164,7 +3176,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, double *
             }
         }
         team_sync<NT>();
-        if (*flag == 0.0) return 2;
+        if (*flag == 0) return 2;
     }
     // L^T x = y: with the rows of L scaled, L'_jk = L_jk / L_jj (k < j),
     // x = col .* z where z_j = y_j - sum_{i > j} L'_ij z_i
@@ -3373,7 +3385,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
             // The damped normal matrix is symmetric positive definite: solve
             // it by Cholesky in FP64; if a pivot is not positive (rounding on
             // a nearly singular alpha), redo the step with Gauss-Jordan.
-            err = cholesky_solve<NT>(s.covar, s.da, mf, s.col, s.misc + M_PIV);
+            err = cholesky_solve<NT>(s.covar, s.da, mf, s.col, reinterpret_cast<int *>(s.misc + M_PIV));
             if (err) {
                 for (int e = tid; e < mf * mf; e += NT) {
                     const int j = e / mf, k = e - j * mf;
