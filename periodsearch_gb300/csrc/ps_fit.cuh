@@ -2898,12 +2898,12 @@ __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
         const int idx = __shfl_sync(0xffffffffu, bi, 0);
         if (idx < 0) return 1;
         const int irow = idx / n, icol = idx - irow * n;
-        const double piv = A[irow * n + icol];
-        if (piv == 0.0) return 2;
+        // (its bits: a comparison of doubles by every warp holds the FP64 units)
+        if (__shfl_sync(0xffffffffu, bv, 0) == 0) return 2;
         // the list without icol (the m - 1 columns still to be pivoted)
         int *cn = col[(step + 1) & 1];
         if (warp < 2) {
-            const double pivinv = 1.0 / piv;
+            const double pivinv = 1.0 / A[irow * n + icol];
             for (int c = tid; c <= m; c += 64) {
                 if (c < m) {
                     const int l = cl[c];
