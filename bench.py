@@ -34,12 +34,13 @@ e2e        the same steps through the C ABI with host buffers: ps_prepare
            host) and ps_destroy per step, wall clock;
 roofline   the kernel with the largest share of the step's device time:
            algorithmic FLOP of its launches over their time (mixed kernel:
-           the dense count 2 N F C + 60 N F + N m(m+1) + 9 F C per
-           evaluation and 2 m^3 per solve, against the measured dense BF16
-           rate, its contractions running on the tensor cores; FP64 kernel:
-           the reference's lit-facet work, flops_fp64, against the FP64 FMA
-           ceiling measured live, MEASURED_PEAKS.json having no FP64
-           figure); every kernel's share in kernels;
+           executed_mixed, from the dense count 2 N F C + 60 N F + N m(m+1)
+           + 9 F C per evaluation and 2 m^3 per solve, against the measured
+           dense BF16 rate, its contractions running on the tensor cores;
+           FP64 kernel: executed_fp64, from the reference's lit-facet work,
+           against the FP64 FMA ceiling measured live, MEASURED_PEAKS.json
+           having no FP64 figure; neither counts the derivatives of rejected
+           steps, which are not evaluated); every kernel's share in kernels;
 cpu_baseline  the reference's own CPU app (oracle/_ref/ps_ref, built from
            its sources) on all host cores, one process per core, each
            fitting one trial period of the window (10 fits) through the
@@ -133,6 +134,38 @@ def flops_fp64(info, evals: int, fits: int, lit: int) -> float:
     n, f, c, m = info.ndata, info.nfac, info.ncoef, info.mfit
     return ((70.0 + 2.0 * c) * lit + evals * (10.0 * n * f + n * m * (m + 1) + 9.0 * f * c) +
             (evals - fits) * 2.0 * m ** 3)
+
+
+# Share of an LM fit's steps that are accepted (24 to 26 of 50 on these
+# workloads).  The kernels decide a step on a chi^2 pass and evaluate the
+# derivatives of accepted steps only, so a rejected step's contraction and
+# normal matrix are not counted as work done.
+ACCEPTED = 0.5
+
+
+def executed_mixed(info, evals: int, fits: int) -> float:
+    """Work of the mixed form's kernels: every fit's first evaluation whole,
+    for each of the other evals a chi^2 pass (dense: 30 per pair, the
+    curvature), the rest of an evaluation for the accepted ones, and a solve."""
+    n, f, c, m = info.ndata, info.nfac, info.ncoef, info.mfit
+    whole = flops_per_eval(n, f, c, m)
+    chi2 = 30.0 * n * f + 9.0 * f * c
+    steps = max(evals - fits, 0)
+    return fits * whole + steps * (chi2 + ACCEPTED * (whole - 9.0 * f * c) + 2.0 * m ** 3)
+
+
+def executed_fp64(info, evals: int, fits: int, lit: int) -> float:
+    """The same of the FP64 kernels, from the reference's lit-facet work: the
+    chi^2 pass takes the dot products (10 per pair), the brightness of the
+    lit pairs (20) and the curvature."""
+    n, f, c, m = info.ndata, info.nfac, info.ncoef, info.mfit
+    if not evals:
+        return 0.0
+    one = lit / evals
+    whole = (70.0 + 2.0 * c) * one + 10.0 * n * f + n * m * (m + 1) + 9.0 * f * c
+    chi2 = 20.0 * one + 10.0 * n * f + 9.0 * f * c
+    steps = max(evals - fits, 0)
+    return fits * whole + steps * (chi2 + ACCEPTED * (whole - 9.0 * f * c) + 2.0 * m ** 3)
 
 
 def window_of(n_max: int, freq_start: float, freq_step: float, truth_h: float, width: int, rank: int = 0):
@@ -431,11 +464,11 @@ def c2_measurement(periods: int, local: int, peaks: dict) -> dict:
         eng.scan(conw_r, lo, lo + 9)      # warm-up
         rows_tc = eng.scan(conw_r, lo, hi)
         t = eng.timing()
-        fe = flops_per_eval(info.ndata, info.nfac, info.ncoef, info.mfit)
-        flop = t["evals"] * fe + (t["evals"] - t["fits"]) * 2.0 * info.mfit ** 3
+        flop = executed_mixed(info, t["evals"], t["fits"])
         ach = flop / (t["kernel_ms"] / 1e3) / 1e12
         bf16 = peaks.get("bf16_tflops")
-        shape = t["evals"] * 2.0 * info.ndata * info.nfac * info.ncoef / (t["kernel_ms"] / 1e3) / 1e12
+        derivs = t["fits"] + ACCEPTED * (t["evals"] - t["fits"])   # evaluations with a contraction
+        shape = derivs * 2.0 * info.ndata * info.nfac * info.ncoef / (t["kernel_ms"] / 1e3) / 1e12
         out.update({"tensor_cores": bool(info.tensor_cores), "ncoef": info.ncoef, "nfac": info.nfac,
                     "mfit": info.mfit, "window": [lo, hi], "fits": t["fits"],
                     "mixed_tensor_fits_per_s": t["fits"] / (t["kernel_ms"] / 1e3),
@@ -490,8 +523,8 @@ class Scanner:
     """One scan of [lo, hi] in the chosen form through the engine, with the
     device time and algorithmic FLOP of each kernel's launches."""
 
-    def __init__(self, form: str, eng, eng64, conw_r: float, fe: float, fs: float):
-        self.form, self.eng, self.eng64, self.conw_r, self.fe, self.fs = form, eng, eng64, conw_r, fe, fs
+    def __init__(self, form: str, eng, eng64, conw_r: float):
+        self.form, self.eng, self.eng64, self.conw_r = form, eng, eng64, conw_r
         self.info = eng.info
 
     def __call__(self, lo: int, hi: int):
@@ -518,9 +551,9 @@ class Scanner:
             st["fits_completed" if key == "complete" else "fits_refit"] = nfits
         screen_fits = nfits if st["evals_screen"] else 0
         mixed_ms = st["screen_ms"] + st["complete_ms"]
-        mixed_flop = ((st["evals_screen"] + st["evals_complete"]) * self.fe +
-                      (st["evals_screen"] - screen_fits + st["evals_complete"] - st["fits_completed"]) * self.fs)
-        fp64_flop = flops_fp64(self.info, st["evals_refit"], st["fits_refit"], lit)
+        mixed_flop = (executed_mixed(self.info, st["evals_screen"], screen_fits) +
+                      executed_mixed(self.info, st["evals_complete"], st["fits_completed"]))
+        fp64_flop = executed_fp64(self.info, st["evals_refit"], st["fits_refit"], lit)
         # the FP64 refit launches are the refit rounds; every other launch is the mixed kernel
         mixed_launches = st["launches"] - st["refit_rounds"]
         if self.form in ("mixed", "fp64"):
@@ -605,9 +638,7 @@ def run_engine_arm(args):
     info = eng.info
     n_max = int(info.n_max)
     conw_r, _ = eng.precalc_conw()
-    fe = flops_per_eval(info.ndata, info.nfac, info.ncoef, info.mfit)
-    fs = 2.0 * info.mfit ** 3
-    scan = Scanner(args.form, eng, eng64, conw_r, fe, fs)
+    scan = Scanner(args.form, eng, eng64, conw_r)
     lo, hi = window_of(n_max, info.freq_start, info.freq_step, truth["period_h"], args.window, rank)
     wfits = (hi - lo + 1) * 10
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=f"cuda:{local}")
@@ -647,7 +678,7 @@ def run_engine_arm(args):
         s0 = time.perf_counter()
         e_m = Engine(data, device=local, form=PS_FORM_MIXED)
         e_64 = Engine(data, device=local, form=PS_FORM_FP64) if args.form in ("fp64",) else None
-        Scanner(args.form, e_m, e_64, conw_r, fe, fs)(lo, hi)
+        Scanner(args.form, e_m, e_64, conw_r)(lo, hi)
         h2d = e_m.info.h2d_bytes + (e_64.info.h2d_bytes if e_64 else 0)
         e_m.close()
         if e_64:
@@ -678,7 +709,7 @@ def run_engine_arm(args):
             t64 = eng64.timing()
             b64 = lo + int(np.argmin(r64["rms"]))
             pv = wfits / (t64["kernel_ms"] / 1e3)
-            pflop = flops_fp64(info, t64["evals"], t64["fits"], t64["lit_facets"])
+            pflop = executed_fp64(info, t64["evals"], t64["fits"], t64["lit_facets"])
             pa = pflop / (t64["kernel_ms"] / 1e3) / 1e12
             fp64 = {"value": pv, "unit": "fits/s", "window": [lo, hi], "fits": wfits,
                     "seconds": t64["kernel_ms"] / 1e3, "best_index": b64,
@@ -686,7 +717,8 @@ def run_engine_arm(args):
                     "lit_fraction": t64["lit_facets"] / (t64["evals"] * info.ndata * info.nfac),
                     "roofline": {"bound": "fp64", "achieved": pa, "peak": p64.value, "unit": "TFLOP/s",
                                  "frac": pa / p64.value,
-                                 "count": "the reference's lit-facet work (flops_fp64)",
+                                 "count": "the reference's lit-facet work, a rejected step's derivatives left out "
+                                          "(executed_fp64)",
                                  "peak_source": "FP64 FMA ceiling measured live by ps_device_fma_peaks"}}
             rows_c = steps[-1][0]
             bc = best_steps[-1]
@@ -701,7 +733,7 @@ def run_engine_arm(args):
             for f in ("learned", "refined", "mixed"):
                 if f == args.form:
                     continue
-                rr, tt = Scanner(f, eng, eng64, conw_r, fe, fs)(lo, hi)
+                rr, tt = Scanner(f, eng, eng64, conw_r)(lo, hi)
                 bo = lo + int(np.argmin(rr["rms"]))
                 rel = np.abs(rr["rms"] - r64["rms"]) / r64["rms"]
                 others[f] = {"fits_per_s": wfits / (tt["device_ms"] / 1e3), "best_index": bo,
