@@ -1103,10 +1103,11 @@ struct LitPair {
 // of a point taking two adjacent facets of every 8 (lane % 4), so that one
 // warp store covers a whole 8-point x 8-facet core matrix of the MMA
 // operand [W_hi; W_lo] (FP16 pairs, W scaled by wscale = 2^k so that the
-// evaluation's largest W is just below 2^14).  The per-point sums (brightness, rotation and
-// scattering derivatives) are reduced over the four lanes and then over the
-// quarters into s.fpart[p * 9 + 0..5] (FP32: the J columns they feed are).  The tile's operand region must be free (previous
-// MMAs waited for).
+// evaluation's largest W is just below 2^14).  The per-point
+// sums (brightness, Lambert and scattering derivatives, U, V) are reduced over
+// the four lanes into s.fpart[(quarter * 32 + p) * 9 + 0..8], for
+// point_sums_tc.  The tile's operand region must be free (previous MMAs waited
+// for).
 template <int NT>
 __device__ void facet_stage_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int np, float cl, float cls,
                                float wscale)
@@ -1188,36 +1189,38 @@ __device__ void facet_stage_tc(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int 
             for (int k = 0; k < 9; k++) fp[k] = v[k];
         }
     }
-    team_sync<NT>();
-    if (tid < np) {
-        float t[9];
+}
+
+// The sums of point p of the tile from its four quarters' partials (FP32: the
+// J columns they feed are): brightness, the three rotation derivatives, the
+// Lambert and the scattering-weight derivatives.  Formed in the contraction
+// window by the warp that writes the J columns: at the end of the facet stage
+// they held all warps for a barrier and some 700 cycles a tile.
+__device__ inline void point_sums_tc(const Smem<PS_FORM_MIXED> &s, int p, float (&v)[6])
+{
+    float t[9];
 #pragma unroll
-        for (int k = 0; k < 9; k++) {
-            float a = 0.f;
+    for (int k = 0; k < 9; k++) {
+        float a = 0.f;
 #pragma unroll
-            for (int q = 0; q < 4; q++) a += s.fpart[(q * 32 + tid) * 9 + k];
-            t[k] = a;
-        }
-        // the point's sums in FP32 over its own quarter-0 partials (read
-        // above by this thread only): brightness, the three rotation
-        // derivatives, the Lambert and the scattering-weight derivatives
-        // D_k . U with D_k = fm u_k (k: beta, lambda) is u_k . fm^T U; the
-        // omega derivative is D_2 = t (e_y, -e_x, 0), e = fm u_0
-        const float *pt = s.pt + tid * kPointStride;
-        const float cf = pt[28], sf = pt[29], tt = pt[30];
-        const float Ux = cf * t[3] - sf * t[4], Uy = sf * t[3] + cf * t[4], Uz = t[5];
-        const float Vx = cf * t[6] - sf * t[7], Vy = sf * t[6] + cf * t[7], Vz = t[8];
-        float *rf = s.fpart + tid * 9;
-        rf[0] = t[0];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const float *ue = pt + 6 * (k + 1), *us = ue + 3;
-            rf[1 + k] = ue[0] * Ux + ue[1] * Uy + ue[2] * Uz + us[0] * Vx + us[1] * Vy + us[2] * Vz;
-        }
-        rf[3] = tt * (pt[1] * Ux - pt[0] * Uy + pt[4] * Vx - pt[3] * Vy);
-        rf[4] = t[1];
-        rf[5] = t[2];
+        for (int q = 0; q < 4; q++) a += s.fpart[(q * 32 + p) * 9 + k];
+        t[k] = a;
     }
+    // D_k . U with D_k = fm u_k (k: beta, lambda) is u_k . fm^T U; the
+    // omega derivative is D_2 = t (e_y, -e_x, 0), e = fm u_0
+    const float *pt = s.pt + p * kPointStride;
+    const float cf = pt[28], sf = pt[29], tt = pt[30];
+    const float Ux = cf * t[3] - sf * t[4], Uy = sf * t[3] + cf * t[4], Uz = t[5];
+    const float Vx = cf * t[6] - sf * t[7], Vy = sf * t[6] + cf * t[7], Vz = t[8];
+    v[0] = t[0];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float *ue = pt + 6 * (k + 1), *us = ue + 3;
+        v[1 + k] = ue[0] * Ux + ue[1] * Uy + ue[2] * Uz + us[0] * Vx + us[1] * Vy + us[2] * Vz;
+    }
+    v[3] = tt * (pt[1] * Ux - pt[0] * Uy + pt[4] * Vx - pt[3] * Vy);
+    v[4] = t[1];
+    v[5] = t[2];
 }
 
 // Convexity rows (conv.c:12-29) on the tensor-core path: rows 0..2 of the
@@ -1770,8 +1773,7 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 if (!conv) {
                     R v[6];
                     if constexpr (kPipe) {
-#pragma unroll
-                        for (int k = 0; k < 6; k++) v[k] = s.fpart[p * 9 + k];
+                        point_sums_tc(s, p, v);
                     } else {
 #pragma unroll
                         for (int k = 0; k < 6; k++) v[k] = R(rd[k]);
@@ -1818,9 +1820,13 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                     if (lane < np) {
                         const int q = start + t0 + lane;
                         const double *pa = reinterpret_cast<const double *>(s.pref + kPrefAcc) + 3 * lane;
+                        float br = 0.f;
+                        if (!conv) {
+#pragma unroll
+                            for (int h = 0; h < 4; h++) br += s.fpart[(h * 32 + lane) * 9];
+                        }
                         const double ymv = conv ? s.red[lane * kRedStride]
-                                                : static_cast<double>(s.fpart[lane * 9] *
-                                                                      s.pt[lane * kPointStride + 24]);
+                                                : static_cast<double>(br * s.pt[lane * kPointStride + 24]);
                         const double sig2i = conv ? 1 / (conv_sig * conv_sig) : pa[0];
                         const double wg = conv ? ob.weight[q] : pa[1];
                         const double dy = (conv ? 0.0 : pa[2]) - ymv;
