@@ -393,7 +393,7 @@ __device__ inline int list_lit_fp64(const DevObject &ob, double e1, double e2, d
     int n = 0;
     // Three rounds of 32 facets at a time, their loads ahead of the ballots
     // (one by one, the loads' latency made the list 5.6 of a point's 22 kcycles
-    // in the chi^2 pass; ten periods in FP64 38.8 -> 37.5 ms, 760 fits 515 ->
+    // in the chi^2 pass; ten periods in FP64 38.8 -> 37.5 ms, 400 fits 515 ->
     // 475 ms).
     constexpr int kRounds = 3;
     for (int i0 = 0; i0 < F; i0 += 32 * kRounds) {
