@@ -2539,7 +2539,17 @@ __device__ void chi2_fp64(const DevObject &ob, const FitConfig &cfg, const SlotL
             for (int c = 0; c < 6; c++) rec[c * cap + i] = e[c];
             rec[6 * cap + i] = sc;
         }
-        __syncthreads();
+        // A cluster's CTAs store into each other's ym below.  Buffer buf was
+        // last read two chunks ago, before the cluster barrier of the chunk in
+        // between; in a call's first chunk it may be the one that the call
+        // before ended on, which a CTA reads (residuals, the last chain) after
+        // that call's last cluster barrier: one more barrier here.
+        bool first = false;
+        if constexpr (SPLIT) {
+            first = q0 == 0;
+            if (first) cgr::this_cluster().sync();
+        }
+        if (!first) __syncthreads();
         if (warp == NW - 1 && lane == 0) chain(cp.ym + static_cast<size_t>(buf ^ 1) * cap, prev_q, prev_n);
         // brightness, a warp per pair of points
         int lit = 0;

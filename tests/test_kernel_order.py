@@ -1,0 +1,54 @@
+"""Order of the fit kernels' shared-memory accesses, on the CPU: the barriers
+and accesses are read from the kernels' source in textual order and replayed
+on a model of the threads that share the memory.  Two accesses of one place by
+different threads are ordered when a barrier of both lies between them; the
+model counts the barriers passed."""
+from __future__ import annotations
+
+import re
+from pathlib import Path
+
+import pytest
+
+SOURCE = (Path(__file__).resolve().parent.parent / "periodsearch_gb300" / "csrc" / "ps_fit.cuh").read_text()
+
+
+def body(name: str) -> str:
+    """The text of function `name`, comments removed."""
+    text = re.sub(r"//[^\n]*", "", SOURCE)
+    at = re.search(r"\b" + name + r"\([^;{}]*\)\s*\{", text).end()
+    depth, end = 1, at
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[end], 0)
+        end += 1
+    return text[at:end]
+
+
+@pytest.mark.parametrize("chunks", [1, 2, 3, 4])
+def test_cluster_chi2_buffers(chunks):
+    """chi2_fp64 of a cluster, called again and again (rejected steps): a CTA's
+    stores into another CTA's model values lie a cluster barrier after that
+    CTA's reads of the same buffer."""
+    text = body("chi2_fp64")
+    loop, tail = text.split("while (q0 < N)")[1], text.rsplit("buf ^= 1;", 1)[1]
+    kinds = {"first": r"if \(first\) cgr::this_cluster\(\)\.sync\(\)",
+             "every": r"if constexpr \(SPLIT\) cgr::this_cluster\(\)\.sync\(\)",
+             "store": r"map_shared_rank\(ym", "read": r"double \*y = ym"}
+    order = [k for _, k in sorted((m.start(), k) for k, pat in kinds.items() for m in re.finditer(pat, loop))]
+    assert [order.count(k) for k in ("every", "store", "read")] == [1, 1, 1] and "chain(" in loop and "chain(" in tail
+    passed = 0                  # cluster barriers
+    last_read = {0: -1, 1: -1}  # barriers passed before the latest read of a buffer
+    for _ in range(3):          # calls
+        buf = 0
+        for c in range(chunks):
+            for e in order:
+                if e == "store":
+                    assert last_read[buf] < passed, f"chunk {c}: a store may meet the reads of buffer {buf}"
+                elif e == "read":
+                    last_read[buf] = passed
+                elif e == "every" or c == 0:
+                    if c and e == "every":
+                        last_read[buf ^ 1] = passed   # the chain over the chunk before
+                    passed += 1
+            buf ^= 1
+        last_read[buf ^ 1] = passed   # the last chain
