@@ -3676,6 +3676,7 @@ __global__ void __launch_bounds__(threads_of<PS_FORM_FP64>(), 1)
                              : w.scratch + static_cast<size_t>(blockIdx.x) * w.scratch_stride;
     if (threadIdx.x == 0) *lit_counter(s.misc) = 0;
     __shared__ long long next;
+    cl.sync();   // every CTA of the cluster runs: its shared memory may be written
     for (;;) {
         if (rank == 0 && threadIdx.x == 0) {
             const long long f = static_cast<long long>(atomicAdd(w.queue, 1ULL));

@@ -52,3 +52,11 @@ def test_cluster_chi2_buffers(chunks):
                     passed += 1
             buf ^= 1
         last_read[buf ^ 1] = passed   # the last chain
+
+
+def test_cluster_started_before_remote_access():
+    """A CTA's shared memory may be reached by the others of its cluster once
+    it has started: a cluster barrier comes before the first remote access (of
+    an evaluation: the barrier of its first round of tiles)."""
+    for text in (body("fit_kernel_split"), body("evaluate_fp64").split("auto flush_round")[1]):
+        assert 0 <= text.find(".sync()") < text.index("map_shared_rank")
