@@ -3017,7 +3017,7 @@ __device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
 // The back substitution runs on warp 0 with b in registers and the rows of
 // L pre-scaled by their reciprocal diagonal.  Returns 2 when a pivot is not
 // positive (an integer flag: a comparison of doubles by every warp holds the
-// FP64 units for 256 cycles a step).  Bound by a pair's chain of dependent FP64
+// FP64 units for 256 cycles a step; two of them in turn, see pivot_flag).  Bound by a pair's chain of dependent FP64
 // operations.  Measured (n = 55): the factorisation 74 -> 64 kcycles with the
 // flag, the selected loads and the pivot's factors formed by the helper itself.
 __device__ inline void chol_pivot_pair(double *A, double *b, int n, int j, double *col, int *flag, int lane)
@@ -3105,8 +3105,14 @@ __device__ inline void chol_pivot_block(double a, double bq, double c, double bj
     if (lane == 0 && two) b[j + 1] = (bj1 - l10 * y0) * i1;
 }
 
+// The flag of the pair (j, j + 1), one of two: warp 0 stores the next pair's
+// while the other warps may still have this pair's to read; the barrier that
+// ends the next pair's step comes before this one's place is stored again.
+__device__ inline int *pivot_flag(int *flags, int j) { return flags + ((j >> 1) & 1); }
+
+// flags: two ints (pivot_flag).
 template <int NT>
-__device__ int cholesky_solve(double *A, double *b, int n, double *col, int *flag)
+__device__ int cholesky_solve(double *A, double *b, int n, double *col, int *flags)
 {
     static_assert(NT % 128 == 0 && NT >= 256, "whole warps on every sub-partition");
     const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
@@ -3116,9 +3122,9 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, int *fla
     double *pub = col + n;   // published for the helper: both reciprocal square roots, a, bq
     const int wtid = ((warp >> 2) * 3 + (warp & 3) - 2) * 32 + lane;
     team_sync<NT>();
-    if (warp == 0) chol_pivot_pair(A, b, n, 0, col, flag, lane);
+    if (warp == 0) chol_pivot_pair(A, b, n, 0, col, pivot_flag(flags, 0), lane);
     team_sync<NT>();
-    if (*flag == 0) return 2;
+    if (*pivot_flag(flags, 0) == 0) return 2;
     for (int j = 0; j + 2 < n; j += 2) {
         // pair (j, j + 1) is factored; b[j], b[j + 1] hold its y
         const bool two = j + 1 < n;
@@ -3146,7 +3152,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, int *fla
             const double cc = __shfl_sync(0xffffffffu, xu, 2);
             const double bj = __shfl_sync(0xffffffffu, xu, 3);
             const double bj1 = __shfl_sync(0xffffffffu, xu, 4);
-            chol_pivot_block<NT>(a, bq, cc, bj, bj1, A, b, n, jn, twon, col, pub, flag, lane);
+            chol_pivot_block<NT>(a, bq, cc, bj, bj1, A, b, n, jn, twon, col, pub, pivot_flag(flags, jn), lane);
         } else if (warp == 1) {
             // the rest of the next pair's columns: update now, scale once
             // warp 0 has published the pivot
@@ -3208,7 +3214,7 @@ __device__ int cholesky_solve(double *A, double *b, int n, double *col, int *fla
             }
         }
         team_sync<NT>();
-        if (*flag == 0) return 2;
+        if (*pivot_flag(flags, jn) == 0) return 2;
     }
     // L^T x = y: with the rows of L scaled, L'_jk = L_jk / L_jj (k < j),
     // x = col .* z where z_j = y_j - sum_{i > j} L'_ij z_i

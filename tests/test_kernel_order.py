@@ -60,3 +60,23 @@ def test_cluster_started_before_remote_access():
     an evaluation: the barrier of its first round of tiles)."""
     for text in (body("fit_kernel_split"), body("evaluate_fp64").split("auto flush_round")[1]):
         assert 0 <= text.find(".sync()") < text.index("map_shared_rank")
+
+
+def test_pivot_flags_of_the_solve():
+    """cholesky_solve: a step's pivot flag is read behind the barrier that ends
+    the step, when warp 0 may already store the next step's: not in its place,
+    and in no place before another barrier has passed."""
+    loop = body("cholesky_solve").split("for (int j = 0; j + 2 < n; j += 2)")[1]
+    store = re.search(r"chol_pivot_block<NT>\(([^;]*)\);", loop).group(1).split(", ", 12)[12].rsplit(",", 1)[0]
+    barrier = loop.index("team_sync<NT>()")
+    read = re.search(r"if \(\*(.*) == 0\) return 2;", loop[barrier:]).group(1)
+    rule = re.search(r"int \*pivot_flag\(int \*flags, int j\) \{ return (.*); \}", SOURCE)
+
+    def place(expr, jn):
+        return eval(rule.group(1), {"flags": 0, "j": jn}) if rule and expr == "pivot_flag(flags, jn)" else 0
+
+    reads = {}
+    for step, jn in enumerate(range(2, 40, 2)):
+        reads[step] = place(read, jn)
+        assert place(store, jn) == reads[step]
+        assert step == 0 or place(store, jn) != reads[step - 1]
