@@ -3293,19 +3293,21 @@ __device__ float mlp_predict_warp(const float *W, const float *f, float *sh)
 // ---------------------------------------------------------------------------
 // One fit (period_search_BOINC.cpp:817-921 with mrqmin.c:11-110).
 // ---------------------------------------------------------------------------
-template <int FORM, int KU, int NT = threads_of<FORM>()>
-__device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<FORM> &s,
-                        typename RealOf<FORM>::T *scratch, int64_t n, int pole, ps_fit *out, const FitWork &w,
-                        long long fidx, TcState &tcs, bool split = false)
+// SPLIT: by the CTAs of a cluster (FP64 form).  Inlined, so that the launch's
+// structs stay kernel parameters: a call passes them by address, through local
+// memory of 1.5 KB a thread, for which the runtime takes 140 MB of device
+// memory at the first launch.
+template <int FORM, int KU, int NT = threads_of<FORM>(), bool SPLIT = false>
+__device__ __forceinline__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<FORM> &s,
+                                        typename RealOf<FORM>::T *scratch, int64_t n, int pole, ps_fit *out,
+                                        const FitWork &w, long long fidx, TcState &tcs)
 {
     constexpr bool kTensor = FORM == PS_FORM_MIXED && (KU == 0 || KU == 3);
-    // one model evaluation; with split (FP64 form, cluster launch) spread
-    // over the cluster's CTAs.  fresh = false: chi2 has just
-    // run at the same parameters.
+    // one model evaluation; fresh = false: chi2 has just run at the same
+    // parameters
     auto eval = [&](const double *a, double *M, double *bv, bool fresh) {
         if constexpr (FORM == PS_FORM_FP64) {
-            if (split) evaluate_fp64<true>(ob, cfg, L, s, a, M, bv, scratch, fresh);
-            else evaluate_fp64<false>(ob, cfg, L, s, a, M, bv, scratch, fresh);
+            evaluate_fp64<SPLIT>(ob, cfg, L, s, a, M, bv, scratch, fresh);
         } else {
             evaluate_mixed<KU, NT>(ob, cfg, L, s, a, M, bv, scratch, tcs, fresh);
         }
@@ -3317,8 +3319,7 @@ __device__ void run_fit(const DevObject &ob, const FitConfig &cfg, const SlotLay
     else lazy = kTensor;
     auto chi2 = [&](const double *a) {
         if constexpr (FORM == PS_FORM_FP64) {
-            if (split) chi2_fp64<true>(ob, cfg, L, s, a);
-            else chi2_fp64<false>(ob, cfg, L, s, a);
+            chi2_fp64<SPLIT>(ob, cfg, L, s, a);
         } else if constexpr (kTensor) {
             chi2_mixed<KU, NT>(ob, cfg, L, s, a);
         }
@@ -3701,7 +3702,8 @@ __global__ void __launch_bounds__(threads_of<PS_FORM_FP64>(), 1)
             n = w.n_lo + f / PS_N_POLES;
             pole = static_cast<int>(f % PS_N_POLES) + 1;
         }
-        run_fit<PS_FORM_FP64, 1>(ob, cfg, L, s, scratch, n, pole, rank == 0 ? w.out + f : nullptr, w, f, tcs, true);
+        run_fit<PS_FORM_FP64, 1, threads_of<PS_FORM_FP64>(), true>(ob, cfg, L, s, scratch, n, pole,
+                                                                   rank == 0 ? w.out + f : nullptr, w, f, tcs);
     }
     if (threadIdx.x == 0 && w.lit) atomicAdd(w.lit, *lit_counter(s.misc));
 }
