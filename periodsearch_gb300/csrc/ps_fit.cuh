@@ -480,8 +480,7 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
 // Accumulates the rows J[0..np) (model values in ym) of one tile into the
 // normal matrix M (lower triangle), bv and chi^2 (mrqcof.c:106-136) on the
 // SIMT pipes of the mixed form: FP32 partial sums, every element over the
-// points in data order, kept in registers and added to the FP64 totals every
-// few tiles.  A warp takes units of 4 rows by 32 columns of the matrix (a
+// points in data order, added to the FP64 totals every few tiles.  A warp takes units of 4 rows by 32 columns of the matrix (a
 // lane one column, four rows from one 16-byte broadcast of the weighted
 // rows): two loads for four products, where an element per thread takes two
 // each and waits for shared memory.  Unit u is unit u of the list of row
@@ -497,6 +496,14 @@ constexpr int kTilesPerFlush = 8;
 // 80 with up to 128 coefficients (KU 2).
 template <int KU>
 constexpr int kAlphaUnits = KU == 2 ? 5 : 3;
+// The wide tensor-core path keeps its partial sums in registers.  The SIMT
+// contraction needs those for its loads in flight: there the loops over the
+// units are not unrolled, which puts the sums in local memory (80 bytes a
+// thread, read and written once a tile).  Held in registers through the
+// contraction they made it wait for its loads: 304 fits of 20 steps (980
+// points, 512 facets, 81 coefficients) 168.6 ms, against 134.9 so.
+template <int KU>
+constexpr int kAlphaUnroll = KU == 3 ? kAlphaUnits<KU> : 1;
 
 // Unit u: its first row (a group of four rows has the panels of 32 columns
 // that reach its last row's diagonal) and, in the upper half, its first
@@ -519,7 +526,7 @@ __device__ inline void flush_partials(double *M, double *bv, int mf, const int (
                                       float4 (&accA)[kAlphaUnits<KU>], float &accB)
 {
     const int tid = threadIdx.x, lane = tid & 31;
-#pragma unroll
+#pragma unroll kAlphaUnroll<KU>
     for (int q = 0; q < kAlphaUnits<KU>; q++) {
         if (unit[q] >= 0) {
             const int r0 = unit[q] & 0xffff, k = (unit[q] >> 16) + lane;
@@ -569,7 +576,7 @@ __device__ void accumulate_tile(const DevObject &ob, Smem<PS_FORM_MIXED> &s, int
         wt[e] = j < mf ? s.J[p * ma + ob.free_list[j]] * wtp[p] : 0.f;
     }
     __syncthreads();
-#pragma unroll
+#pragma unroll kAlphaUnroll<KU>
     for (int q = 0; q < kAlphaUnits<KU>; q++) {
         if (unit[q] < 0) continue;
         const float *jc = s.J + ob.free_list[min((unit[q] >> 16) + lane, mf - 1)];
@@ -614,10 +621,17 @@ __device__ inline float load_basis(const float *d, int idx)
 // of one tile, FP32 on the SIMT pipes.  Register tile: warp w owns points
 // (w % 8) + 8 r (r < 4) and coefficients lane + 32 ((w / 8) + 2 u) (u < KU);
 // W is read four facets at a time (float4 broadcast), Dsph one coalesced row
-// per facet.
+// per facet.  Bound by the latency of those loads, so by what the compiler
+// keeps in flight: a function of its own (contract_mixed_call) has all
+// registers for it.  304 fits of 20 steps with 81 coefficients and 512 facets
+// 134.9 -> 84.8 ms, with 49 coefficients and 288 facets 35.8 -> 30.1; one
+// coefficient per lane with the basis in L2 is better inlined (49 coefficients,
+// 648 facets: 72.0 ms, 119 as a call).  Unrolled by four facet groups with the
+// basis in shared memory, by two else (four: 91.5 ms in the first case, none
+// 95.3).
 template <int NT, int KU, bool SMEM_D>
-__device__ void contract_mixed(Smem<PS_FORM_MIXED> &s, const float *dsph, int np, int F, int C, int ma, int wcols,
-                               bool conv)
+__device__ __forceinline__ void contract_mixed(const float *Wf, const float *pt, float *J, const float *dsph, int np,
+                                               int F, int C, int ma, int wcols, bool conv)
 {
     static_assert(NT == 512, "the register tile assumes 16 warps");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -638,8 +652,8 @@ __device__ void contract_mixed(Smem<PS_FORM_MIXED> &s, const float *dsph, int np
     bool any = false;
 #pragma unroll
     for (int u = 0; u < KU; u++) any |= kv[u];
-    const float *Wf = s.W;
     if (any) {
+#pragma unroll (SMEM_D ? 4 : 2)
         for (int i = 0; i < F; i += 4) {
             float4 w4[kPW];
 #pragma unroll
@@ -666,12 +680,19 @@ __device__ void contract_mixed(Smem<PS_FORM_MIXED> &s, const float *dsph, int np
     for (int r = 0; r < kPW; r++) {
         const int p = g + 8 * r;
         if (p < np) {
-            const float sc = conv ? 1.f : s.pt[p * kPointStride + 24];
+            const float sc = conv ? 1.f : pt[p * kPointStride + 24];
 #pragma unroll
             for (int u = 0; u < KU; u++)
-                if (kv[u]) s.J[p * ma + kk[u]] = sc * acc[r][u];
+                if (kv[u]) J[p * ma + kk[u]] = sc * acc[r][u];
         }
     }
+}
+
+template <int NT, int KU, bool SMEM_D>
+__device__ __noinline__ void contract_mixed_call(const float *Wf, const float *pt, float *J, const float *dsph, int np,
+                                                 int F, int C, int ma, int wcols, bool conv)
+{
+    contract_mixed<NT, KU, SMEM_D>(Wf, pt, J, dsph, np, F, C, ma, wcols, conv);
 }
 
 // Mixed-form point set-up in three parts (bright.c:27-57, phasec.c,
@@ -1775,9 +1796,11 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
                 contract_tc_issue<NT, kWide>(s, F, tcs);   // the work below overlaps the MMAs
             } else {
                 if (s.dsph)
-                    contract_mixed<NT, KU, true>(s, dsphF, np, F, C, ma, wcols, conv);
+                    contract_mixed_call<NT, KU, true>(s.W, s.pt, s.J, dsphF, np, F, C, ma, wcols, conv);
+                else if constexpr (KU == 2)
+                    contract_mixed_call<NT, KU, false>(s.W, s.pt, s.J, dsphF, np, F, C, ma, wcols, conv);
                 else
-                    contract_mixed<NT, KU, false>(s, dsphF, np, F, C, ma, wcols, conv);
+                    contract_mixed<NT, KU, false>(s.W, s.pt, s.J, dsphF, np, F, C, ma, wcols, conv);
             }
             // remaining columns of J: one thread per point (not thread 0 on the
             // tensor-core path: it issues the MMAs)
