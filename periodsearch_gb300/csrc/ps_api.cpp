@@ -270,14 +270,13 @@ int64_t tiles_of(const ps_ctx *c, int P)
 }
 
 // CTAs per fit for a launch: FP64 fits without trajectories, saved states
-// or an iteration limit, at most half as many as the fit slots, are each
-// spread over a thread-block cluster, of as many CTAs (up to 16, and not more
-// than the object has tiles or, where the slots hold them, 4) as leave every
+// or an iteration limit, fewer than the fit slots, are each spread over a
+// thread-block cluster: of 2 or 4 CTAs where the slots hold them, and of as
+// many (up to 16, not more than the object has tiles) as still leave every
 // fit a cluster that is resident at once.  A cluster lies within one GPC, so
 // there are fewer than slots / cs of the larger ones (36 of 4, 13 of 10, 7 of
 // 16 CTAs on 152 SMs), and a second round of fits costs more than a larger
-// cluster gains (38 fits of 130 points, 16 coefficients: two rounds of 4 CTAs
-// 2.42 ms, one of 3 1.46).  Measured on 980 points, 288 facets (32 tiles), one launch in ms
+// cluster gains.  Measured on 980 points, 288 facets (32 tiles), one launch in ms
 // by CTAs per fit: 175 (1), 105 (2), 76 (3), 62 (4), 54 (5), 49 (6), 39 (9 and
 // 10), 35 (12), 31 (16); 200 points (7 tiles): 40 (1), 27 (2), 20 (4), 17 (6),
 // 16 (7).
@@ -285,12 +284,12 @@ int split_size(ps_ctx *c, const psg::FitWork &w, int form)
 {
     if (form != PS_FORM_FP64 || w.traj || w.state || w.iter_limit > 0 || w.nfits < 1) return 1;
     FormPlan &pl = c->plan[form];
-    if (w.nfits * 2 > pl.slots) return 1;
-    const int64_t least = w.nfits * 4 <= pl.slots ? 4 : 2;
-    // (a CTA takes a slot's scratch)
-    int k = static_cast<int>(std::min<int64_t>(psg::kMaxClusterCtas, std::max(least, tiles_of(c, pl.P))));
-    while (k > 1 && (w.nfits * k > c->scratch_slots || clusters_of(pl, k) < w.nfits)) k--;
-    return k;
+    const int64_t slots = pl.slots;
+    int cs = w.nfits * 4 <= slots ? 4 : w.nfits * 2 <= slots ? 2 : 1;
+    const int most = static_cast<int>(std::min<int64_t>(psg::kMaxClusterCtas, tiles_of(c, pl.P)));
+    for (int k = most; k > cs && cs > 1; k--)
+        if (clusters_of(pl, k) >= w.nfits) cs = k;
+    return cs;
 }
 
 // Launches the fits described by w in the given form (queue and outputs
@@ -345,7 +344,8 @@ ps_status run_fits(ps_ctx *c, double conw_r, psg::FitWork w, int form)
     PSG_CUDA(c, cudaEventRecord(c->ev[0], c->stream));
     int e;
     if (cs > 1) {
-        e = psg::launch_fits_split(c->dob, cfg, w, static_cast<int>(w.nfits), cs, pl.P, pl.smem, c->stream);
+        const int clusters = static_cast<int>(std::min<int64_t>(std::max(clusters_of(pl, cs), 1), w.nfits));
+        e = psg::launch_fits_split(c->dob, cfg, w, clusters, cs, pl.P, pl.smem, c->stream);
     } else if (pair) {
         e = psg::launch_fits_pair(c->dob, cfg, w, grid, pl.pair_smem, c->stream);
     } else {
@@ -963,7 +963,7 @@ ps_status ps_eval(ps_ctx *c, double conw_r, const double *cg, double *alpha, dou
     int cs = 1;
     if (c->opt.form == PS_FORM_FP64) {
         FormPlan &pl = c->plan[PS_FORM_FP64];
-        cs = static_cast<int>(std::min<int64_t>(std::min(psg::kMaxClusterCtas, c->scratch_slots), tiles_of(c, pl.P)));
+        cs = static_cast<int>(std::min<int64_t>(psg::kMaxClusterCtas, tiles_of(c, pl.P)));
         while (cs > 1 && clusters_of(pl, cs) < 1) cs--;
     }
     int e = cs > 1 ? psg::launch_eval_split(c->dob, cfg, d_cg, d_al, d_be, d_c2, d_ar, c->d_scratch,
