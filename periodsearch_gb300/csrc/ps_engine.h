@@ -121,7 +121,8 @@ struct SlotLayout {
     size_t rels;            // relative-lightcurve rows in shared memory, or 0 (global scratch)
     size_t pref;            // tensor-core path: per-point data prefetched for the contraction window
     size_t flist;           // tensor-core path: the free parameters' columns
-    size_t phase, resid;    // FP64 form: first set-up part of the next tiles; residuals and point orders
+    size_t phase;           // FP64 form: first set-up part of the next phase_tiles tiles (1: in the points' records)
+    int phase_tiles;
     size_t lit;             // FP64 form: per point of a tile, its lit-facet count, then its lit facets
     size_t bytes;
 };
@@ -139,7 +140,11 @@ PSG_HD constexpr int threads_of()
 // Threads of a team of the kernel that runs two mixed fits per CTA.
 constexpr int kTeamThreads = 256, kPairFits = 2;
 constexpr int kPointStride = 33;   // reals of per-point set-up (odd: a warp with one point per lane hits 32 banks)
-constexpr int kRedStride = 9;      // doubles of per-point facet sums
+constexpr int kRedStride = 8;      // doubles of per-point facet sums
+// FP64 form, spare places of a point's record: the first set-up part while no
+// other place holds it (four), then its byte of every warp's point order; the
+// ninth facet sum.
+constexpr int kPtPhase = 28, kPtOrder = 28, kPtSum = 32;
 constexpr int kMisc = 40;
 // Prefetch area of the tensor-core path, for a 32-point tile: times (32
 // doubles), two copies of the FP32 geometry (32 x 2 float4 each) and sig^-2,
@@ -164,6 +169,10 @@ PSG_HD constexpr int rel_row_stride(int ma) { return ma + 3; }
 // multiple of the 16 facets of one FP16 MMA).
 PSG_HD constexpr int tc_kpad(int nfac) { return (nfac + 31) & ~31; }
 
+
+// Dynamic shared memory that a layout fills up with what is better larger: the
+// 227 KB of a CTA less the kernels' own static shared memory.
+constexpr size_t kSmemFill = 227 * 1024 - 1024;
 
 // Workspace of the Gauss-Jordan solve of n equations: the scaled pivot row,
 // the pivot column, the right-hand side's entry and a candidate's bits per
@@ -218,10 +227,13 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     L.pt = take(static_cast<size_t>(P) * kPointStride * rs);
     L.ym = take(P * d);
     L.red = take(static_cast<size_t>(P) * kRedStride * d);
+    // the solvers' workspace over the tiles' (of W, J, pt, ym and red nothing
+    // is needed from an evaluation to the next)
+    const size_t tiles_end = o, work = gj_doubles(mfit) * d + gj_ints(mfit) * sizeof(int);
     L.dave = take(ma * d);
-    L.col = take(gj_doubles(mfit) * d);
+    L.col = tiles_end - L.W >= work ? L.W : take(work);
+    L.ipiv = L.col + gj_doubles(mfit) * d;
     L.misc = take(kMisc * d);
-    L.ipiv = take(sizeof(int) * gj_ints(mfit));
     L.dsph = dsph_smem == kBasisSmem ? take(static_cast<size_t>(nfac) * ncoef * sizeof(float)) : 0;
     if (basis_on_tensor(dsph_smem)) {
         const bool wide = dsph_smem == kBasisTensorWide;
@@ -264,10 +276,18 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     L.bmat = take(32 * rs);
     L.rels = rel_rows > 0 ? take(static_cast<size_t>(rel_rows) * rel_row_stride(ma) * rs) : 0;
     // FP64 form: P counts (int) and P x wcols facet indices (uint16_t)
-    const int warps64 = threads_of<PS_FORM_FP64>() / 32;
-    L.phase = form == PS_FORM_FP64 ? take(static_cast<size_t>(4 * warps64) * P * d) : 0;
-    L.resid = form == PS_FORM_FP64 ? take(64 * d + static_cast<size_t>(32) * warps64) : 0;
     L.lit = form == PS_FORM_FP64 ? take(static_cast<size_t>(P) * (4 + 2 * L.wcols)) : 0;
+    // a tile per warp where that fits, else as many as do (they give way to
+    // the tile size and to parked rows)
+    L.phase_tiles = 1;
+    if (form == PS_FORM_FP64) {
+        const size_t tile = 4 * static_cast<size_t>(P) * d, fit = o < kSmemFill ? (kSmemFill - o) / tile : 0;
+        const size_t most = threads_of<PS_FORM_FP64>() / 32;
+        if (fit > 1) {
+            L.phase_tiles = static_cast<int>(fit < most ? fit : most);
+            L.phase = take(tile * L.phase_tiles);
+        }
+    }
     L.bytes = (o + 127) & ~size_t(127);
     return L;
 }

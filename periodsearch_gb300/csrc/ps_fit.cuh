@@ -99,9 +99,7 @@ struct Smem {
     // facets in increasing order ([P][wcols], the W row holds their values)
     int *nlit;
     uint16_t *lidx;
-    double *phase;          // FP64 form: [4][warps * P] first set-up part of the CTA's next tiles
-    double *resid;          // FP64 form: [2][32] a tile's residuals and their weighted squares
-    unsigned char *order;   // FP64 form: [warps][32] points of the tile by lit count
+    double *phase;          // FP64 form: [4][phase_tiles * P] first set-up part of the CTA's next tiles
     uint32_t *tslot;
     int *abort;
 };
@@ -138,8 +136,6 @@ __device__ inline Smem<FORM> carve(char *base, const SlotLayout &L)
     s.lidx = L.form == PS_FORM_FP64 ? reinterpret_cast<uint16_t *>(base + L.lit + 4 * static_cast<size_t>(L.P))
                                      : nullptr;
     s.phase = L.form == PS_FORM_FP64 ? reinterpret_cast<double *>(base + L.phase) : nullptr;
-    s.resid = L.form == PS_FORM_FP64 ? reinterpret_cast<double *>(base + L.resid) : nullptr;
-    s.order = L.form == PS_FORM_FP64 ? reinterpret_cast<unsigned char *>(base + L.resid + 64 * sizeof(double)) : nullptr;
     s.dsph = L.dsph_smem == kBasisSmem ? reinterpret_cast<float *>(base + L.dsph) : nullptr;
     if (basis_on_tensor(L.dsph_smem)) {
         s.bhi = reinterpret_cast<unsigned char *>(base + L.bhi);
@@ -341,11 +337,12 @@ __device__ inline double fold_pair(double a, double c, int ia, int ic, int m, in
     return keep + __shfl_xor_sync(0xffffffffu, give, m);
 }
 
-// Sums nine FP64 values over the warp and stores sum k at out[k]: every
+// Sums nine FP64 values over the warp and stores sum k at out[k] (the last at
+// out8): every
 // level pairs the same lanes as warp_sum, so each sum is warp_sum's bit for
 // bit, in 12 shuffles and 12 additions instead of 45.  Each sum ends in the
 // lanes that kept it; they store it (the same value).
-__device__ inline void warp_sum9(const double (&v)[9], double *out, int lane)
+__device__ inline void warp_sum9(const double (&v)[9], double *out, double *out8, int lane)
 {
     double w[5];
     int iw[5];
@@ -366,7 +363,7 @@ __device__ inline void warp_sum9(const double (&v)[9], double *out, int lane)
     iy[1] = ix[2];
     int iz;
     const double z = fold_pair(y[0], y[1], iy[0], iy[1], 2, lane, iz);
-    out[iz] = z + __shfl_xor_sync(0xffffffffu, z, 1);
+    *(iz < 8 ? out + iz : out8) = z + __shfl_xor_sync(0xffffffffu, z, 1);
 }
 
 // Lists the lit facets of a point with Earth and Sun directions e, f in
@@ -431,14 +428,15 @@ __device__ inline int list_lit_fp64(const DevObject &ob, double e1, double e2, d
 // lane busy (an FP64 instruction holds its sub-partition's FP64 unit for
 // the whole warp, however few lanes are active), lane l taking the list's
 // entries l, l + 32, ...  W is left in the W row at the list positions.
-// The facet sums go to s.red[p * kRedStride + 0..8]: brightness, U, V, the
-// Lambert and the scattering-weight derivatives.
+// The facet sums go to s.red[p * kRedStride + 0..7], brightness, U, V and the
+// Lambert derivative, and the scattering-weight derivative to the point's
+// record.
 // count: add the point's lit facets to the CTA's counter.
 __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> &s, int p, int wcols, double cl,
                                         double cls, bool count)
 {
     const int lane = threadIdx.x & 31;
-    const double *pt = s.pt + p * kPointStride;
+    double *pt = s.pt + p * kPointStride;
     const double e1 = pt[0], e2 = pt[1], e3 = pt[2];
     const double f1 = pt[3], f2 = pt[4], f3 = pt[5];
     uint16_t *idx = s.lidx + static_cast<size_t>(p) * wcols;
@@ -470,7 +468,7 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
         dcls = dcls + ar * lt.dcls_w;
     }
     const double v9[9] = {br, ux, uy, uz, vx, vy, vz, dcl, dcls};
-    warp_sum9(v9, s.red + p * kRedStride, lane);
+    warp_sum9(v9, s.red + p * kRedStride, pt + kPtSum, lane);
     if (lane == 0) {
         s.nlit[p] = n;
         if (count) atomicAdd(lit_counter(s.misc), static_cast<unsigned long long>(n));
@@ -2070,34 +2068,47 @@ __device__ void evaluate_mixed(const DevObject &ob, const FitConfig &cfg, const 
 constexpr int kMaxSplit = 16;
 constexpr int kWarpsFp64 = threads_of<PS_FORM_FP64>() / 32;
 
-// First part of the set-up (setup_phase_fp64) of the CTA's next kWarpsFp64
-// tiles, warp w the w-th, a point per lane: with one tile at a time the
-// set-up ran on 8 lanes of 4 warps (28 of a tile's 320 kcycles; 7 now, with
-// the second part).  (lc, t0): the first of these tiles; step: tiles from one
+// Where the first set-up part of point `lane` of the group's tile `slot` lies:
+// the four values' distance in stride.
+__device__ inline double *phase_at(const SlotLayout &L, const Smem<PS_FORM_FP64> &s, int slot, int lane, int &stride)
+{
+    const bool own = L.phase_tiles > 1;
+    stride = own ? L.phase_tiles * L.P : 1;
+    return own ? s.phase + slot * L.P + lane : s.pt + lane * kPointStride + kPtPhase;
+}
+
+// First part of the set-up (setup_phase_fp64) of the CTA's next
+// L.phase_tiles tiles, warp w the w-th, a point per lane: with one tile at a
+// time the set-up ran on 8 lanes of 4 warps (28 of a tile's 320 kcycles; 7 now,
+// with the second part).  (lc, t0): the first of these tiles; step: tiles from one
 // of the CTA's tiles to its next.
 __device__ inline void setup_group_fp64(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L,
                                         Smem<PS_FORM_FP64> &s, int lc, int t0, int step, double omg)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int skip = warp * step;
-    while (lc < ob.n_lc - 1) {
-        const int nt = (ob.lc_npts[lc] - t0 + L.P - 1) / L.P;
-        if (skip < nt) break;
-        skip -= nt;
-        lc++;
-        t0 = 0;
-    }
-    if (lc < ob.n_lc - 1) {
-        t0 += skip * L.P;
-        if (lane < min(L.P, ob.lc_npts[lc] - t0))
-            setup_phase_fp64(ob, cfg, ob.lc_start[lc] + t0 + lane, omg, s.bmat, s.phase + warp * L.P + lane,
-                             kWarpsFp64 * L.P);
+    if (warp < L.phase_tiles) {
+        int skip = warp * step;
+        while (lc < ob.n_lc - 1) {
+            const int nt = (ob.lc_npts[lc] - t0 + L.P - 1) / L.P;
+            if (skip < nt) break;
+            skip -= nt;
+            lc++;
+            t0 = 0;
+        }
+        if (lc < ob.n_lc - 1) {
+            t0 += skip * L.P;
+            if (lane < min(L.P, ob.lc_npts[lc] - t0)) {
+                int stride;
+                double *ph = phase_at(L, s, warp, lane, stride);
+                setup_phase_fp64(ob, cfg, ob.lc_start[lc] + t0 + lane, omg, s.bmat, ph, stride);
+            }
+        }
     }
     __syncthreads();
 }
 
 // Model rows of one tile of np points from q0 on into s.J / s.ym
-// (bright.c:14-126), its first set-up part in slot `slot` of s.phase; conv:
+// (bright.c:14-126), its first set-up part in the group's slot `slot`; conv:
 // the convexity rows (conv.c:12-29).  Leaves with a barrier.
 __device__ void tile_rows_fp64(const DevObject &ob, const SlotLayout &L, Smem<PS_FORM_FP64> &s, int q0, int np,
                                bool conv, int slot, bool count)
@@ -2111,14 +2122,15 @@ __device__ void tile_rows_fp64(const DevObject &ob, const SlotLayout &L, Smem<PS
         static_assert(NW == 12, "twelve set-up parts");
         const int part = warp & 3, i = warp >> 2;
         if (lane < np) {
-            const double *ph = s.phase + slot * L.P + lane;
+            int stride;
+            const double *ph = phase_at(L, s, slot, lane, stride);
             double *pt = s.pt + lane * kPointStride;
-            setup_row_fp64(ob, q0 + lane, part, i, s.bmat, ph, NW * L.P, pt);
+            setup_row_fp64(ob, q0 + lane, part, i, s.bmat, ph, stride, pt);
             if (part == 3 && i == 2) {
-                const double alpha = ob.alpha_pt[q0 + lane], ex = ph[2 * NW * L.P];
+                const double alpha = ob.alpha_pt[q0 + lane], ex = ph[2 * stride];
                 pt[24] = phase_scale_fp64(s.bmat[27], s.bmat[29], ex, alpha);
                 pt[25] = ex;
-                pt[26] = ph[3 * NW * L.P];
+                pt[26] = ph[3 * stride];
                 pt[27] = alpha;
             }
         }
@@ -2141,8 +2153,11 @@ __device__ void tile_rows_fp64(const DevObject &ob, const SlotLayout &L, Smem<PS
     // Contraction: outputs (point, coefficient) in units of 32 lanes.  A lane
     // runs as long as its point's lit list, a unit as long as its longest, so
     // the points are taken in order of their counts (each warp orders them
-    // itself): a unit's points then have nearly the same count.
-    unsigned char *ord = s.order + warp * 32;
+    // itself, into its byte of the points' records): a unit's points then have
+    // nearly the same count.
+    auto ord = [&](int r) -> unsigned char & {
+        return reinterpret_cast<unsigned char *>(s.pt + r * kPointStride + kPtOrder)[warp];
+    };
     {
         const int n = lane < np ? (conv ? F : s.nlit[lane]) : -1;
         int r = 0;
@@ -2151,11 +2166,11 @@ __device__ void tile_rows_fp64(const DevObject &ob, const SlotLayout &L, Smem<PS
             const int m = __shfl_sync(0xffffffffu, n, o);
             r += (m > n || (m == n && o < lane)) ? 1 : 0;
         }
-        ord[r] = static_cast<unsigned char>(lane);
+        if (lane < np) ord(r) = static_cast<unsigned char>(lane);
         __syncwarp();
     }
     for (int o = tid; o < np * C; o += NW * 32) {
-        const int r = o / C, k = o - r * C, p = ord[r];
+        const int r = o / C, k = o - r * C, p = ord(r);
         const double acc = contract_fp64(s, ob.dsph + k, p, C, F, wcols, conv);
         s.J[p * ma + k] = conv ? acc : s.pt[p * kPointStride + 24] * acc;
     }
@@ -2183,7 +2198,7 @@ __device__ void tile_rows_fp64(const DevObject &ob, const SlotLayout &L, Smem<PS
             Jp[C + 4] = br * pt[26];
             Jp[C + 5] = br * pt[27];
             Jp[C + 6] = scale * rd[7] * cl;
-            Jp[C + 7] = scale * rd[8];
+            Jp[C + 7] = scale * pt[kPtSum];
             s.ym[p] = br * scale;
         } else {
             for (int k = C; k < ma; k++) Jp[k] = 0;
@@ -2219,7 +2234,7 @@ __device__ void accumulate_tile_fp64(const DevObject &ob, Smem<PS_FORM_FP64> &s,
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ma = ob.ma, mf = ob.mfit;
     double *wt = s.W;   // [np][mf], reuses the facet-weight tile
-    double *dyv = s.resid, *tv = dyv + 32;
+    double *dyv = s.pt, *tv = dyv + 32;   // (the points' records have served)
     const double conv_s2 = conv ? 1 / (conv_sig * conv_sig) : 0.0;
     if (warp == kWarpsFp64 - 1 && lane < np) {
         const double dy = (conv ? 0.0 : ob.bright[q0 + lane]) - ymv[lane];
@@ -2366,7 +2381,7 @@ __device__ void evaluate_fp64(const DevObject &ob, const FitConfig &cfg, const S
 
     // rounds of cs tiles over the real lightcurves, in data order
     int rlc[SPLIT ? kMaxSplit : 1], rt0[SPLIT ? kMaxSplit : 1], rnp[SPLIT ? kMaxSplit : 1];
-    int nround = 0, slot = NW;
+    int nround = 0, slot = L.phase_tiles;
     auto flush_round = [&]() {
         if constexpr (SPLIT) cgr::this_cluster().sync();   // every CTA's tile of the round is in its shared memory
         for (int k = 0; k < nround; k++) {
@@ -2397,7 +2412,7 @@ __device__ void evaluate_fp64(const DevObject &ob, const FitConfig &cfg, const S
             rt0[nround] = t0;
             rnp[nround] = np;
             if (nround == rank) {
-                if (slot == NW) {
+                if (slot == L.phase_tiles) {
                     setup_group_fp64(ob, cfg, L, s, lc, t0, cs, omg);
                     slot = 0;
                 }
