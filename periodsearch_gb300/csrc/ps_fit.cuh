@@ -2692,11 +2692,15 @@ __device__ void chi2_fp64(const DevObject &ob, const FitConfig &cfg, const SlotL
 // Each value by evaluate's operations in their order (a point's brightness:
 // facet_stage_tc's four lanes and four facet quarters; chi^2: tile sums in
 // tile order), so chi^2 is evaluate's bit for bit.
-// Buffers in the operand region (at least 1040 points: any relative
-// lightcurve fits).
+// Buffers in the operand region, eight floats a point: at least kChi2Points, so
+// that any relative lightcurve fits (one that did not would never be passed).
 // Measured: 3010 fits of 980 points, 288 facets 290 -> 219 ms; 1010 fits with
 // 81 coefficients, 512 facets 247 -> 171 ms.
 // ---------------------------------------------------------------------------
+constexpr int kChi2Bytes = 128 * 65 * sizeof(float);   // of the operand region, at least (make_layout)
+constexpr int kChi2Points = kChi2Bytes / 32 & ~31;
+static_assert(kChi2Points >= PS_POINTS_MAX, "a relative lightcurve is summed in one chunk");
+
 template <int KU, int NT>
 __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const SlotLayout &L, Smem<PS_FORM_MIXED> &s,
                            const double *a)
@@ -2706,7 +2710,7 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
     const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
     const int F = ob.nfac, C = ob.ncoef, nreal = ob.n_lc - 1, N = ob.ndata;
     shape_prologue<PS_FORM_MIXED, KU, NT>(ob, s, a);
-    const int cap = static_cast<int>(2 * (L.blo - L.bhi) > 33280 ? 2 * (L.blo - L.bhi) : 33280) / 32 & ~31;
+    const int cap = max(static_cast<int>(2 * (L.blo - L.bhi)), kChi2Bytes) / 32 & ~31;
     float *rec = reinterpret_cast<float *>(s.bhi);   // [7][cap] directions, phase function
     float *ym = rec + 7 * cap;                       // [cap] model values
     double *tsum = s.red, *c2sum = s.red + kTiles;

@@ -80,3 +80,18 @@ def test_pivot_flags_of_the_solve():
         reads[step] = place(read, jn)
         assert place(store, jn) == reads[step]
         assert step == 0 or place(store, jn) != reads[step - 1]
+
+
+def test_chunks_of_the_mixed_chi2_pass():
+    """chi2_mixed takes a relative lightcurve whole, and its chunk loop passes
+    one that does not fit never: the smallest operand region of any layout, and
+    the sums of a chunk's tiles, hold the longest lightcurve that is accepted."""
+    header = (Path(__file__).resolve().parent.parent / "include" / "ps_gb300.h").read_text()
+    longest = int(re.search(r"#define PS_POINTS_MAX (\d+)", header).group(1))
+    engine = (Path(__file__).resolve().parent.parent / "periodsearch_gb300" / "csrc" / "ps_engine.h").read_text()
+    region = re.search(r"size_t readback = (.*) \* sizeof\(float\);", engine).group(1)
+    assert re.search(r"kChi2Bytes = (.*) \* sizeof\(float\);", SOURCE).group(1) == region
+    assert "static_assert(kChi2Points >= PS_POINTS_MAX" in SOURCE
+    assert (eval(region) * 4 // 32 & ~31) >= longest
+    tiles = 16 * int(re.search(r"kRedStride = (\d+);", engine).group(1))
+    assert tiles * 32 >= longest
