@@ -151,7 +151,8 @@ ps_status build_plan(ps_ctx *c, int form, int dsph_smem, int P, int per_sm_cap, 
     const int F = o.shape.nfac;
     cudaDeviceProp prop;
     PSG_CUDA(c, cudaGetDeviceProperties(&prop, c->opt.device));
-    const size_t smem_max = static_cast<size_t>(prop.sharedMemPerBlockOptin);
+    constexpr size_t kStatic = 64;   // the fit kernels' own static shared memory
+    const size_t smem_max = static_cast<size_t>(prop.sharedMemPerBlockOptin) - kStatic;
     if (dsph_smem == psg::kBasisTensor && !psg::tensor_basis_ok(F, o.ncoef, o.mfit, P)) return PS_ERR_LIMIT;
     if (dsph_smem == psg::kBasisTensorWide && !psg::tensor_wide_ok(F, o.ncoef, o.mfit, P)) return PS_ERR_LIMIT;
     const psg::SlotLayout L = psg::make_layout(form, o.ma, o.mfit, F, o.ncoef, P, dsph_smem);
@@ -202,11 +203,10 @@ ps_status build_plan(ps_ctx *c, int form, int dsph_smem, int P, int per_sm_cap, 
     // (not when the caller asked for one slot per SM)
     out->pair_smem = 0;
     if (dsph_smem == psg::kBasisTensor && per_sm_cap != 1 && psg::tensor_pair_ok(F, o.mfit)) {
-        constexpr size_t kStatic = 64;   // the kernel's own static shared memory
         for (int rows : {o.max_rel_points, 0}) {
             const size_t need =
                 psg::kPairFits * psg::make_layout(form, o.ma, o.mfit, F, o.ncoef, P, dsph_smem, rows, true).bytes;
-            if (need + kStatic > smem_max) continue;
+            if (need > smem_max) continue;
             e = psg::set_pair_smem(std::max(need, floor_tc));
             if (e != 0) return cuda_fail(c, static_cast<cudaError_t>(e), "cudaFuncSetAttribute");
             out->pair_smem = std::max(need, floor_tc);
@@ -1441,8 +1441,20 @@ ps_status ps_pack_create(ps_ctx *const *ctxs, int32_t n, int32_t form, ps_pack *
     const FormPlan &pl = c0->plan[form];
     k->P = pl.P;
     k->dsph_smem = pl.dsph_smem;
-    k->smem = pl.smem;
     k->slots = pl.slots;
+    // Shared memory: no parked rows, and a fit's object in static shared
+    // memory.  (The FP64 form's results do not depend on the tile size.)
+    int smem_max = 0, smem_sm = 0;
+    PSG_PACK_CUDA(k.get(), cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, k->device));
+    PSG_PACK_CUDA(k.get(), cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, k->device));
+    const size_t room = static_cast<size_t>(smem_max), fixed = sizeof(psg::DevObject) + sizeof(psg::FitConfig) + 64;
+    const size_t floor_tc = psg::basis_on_tensor(k->dsph_smem) ? static_cast<size_t>(smem_sm) / 2 + 1024 : 0;
+    auto slot_bytes = [&](bool pair) {
+        const psg::HostObject &o = c0->obj;
+        return psg::make_layout(form, o.ma, o.mfit, o.shape.nfac, o.ncoef, k->P, k->dsph_smem, 0, pair).bytes;
+    };
+    while (form == PS_FORM_FP64 && k->P > 2 && slot_bytes(false) + fixed > room) k->P /= 2;
+    k->smem = std::max(slot_bytes(false), floor_tc);
     int e = psg::set_pack_smem(form, k->smem, c0->obj.ncoef, k->dsph_smem);
     if (e != 0) return pack_fail(k.get(), static_cast<cudaError_t>(e), "cudaFuncSetAttribute");
     for (ps_ctx *c : k->ctx) k->scratch_stride = std::max(k->scratch_stride, c->scratch_stride);
@@ -1451,16 +1463,10 @@ ps_status ps_pack_create(ps_ctx *const *ctxs, int32_t n, int32_t form, ps_pack *
     PSG_PACK_CUDA(k.get(), cudaEventCreate(&k->ev[1]));
     PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_objs, sizeof(psg::DevObject) * n));
     PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_cfgs, sizeof(psg::FitConfig) * n));
-    if (pl.pair_smem > 0) {
-        const psg::HostObject &o = c0->obj;
-        k->pair_smem = std::max(psg::kPairFits * psg::make_layout(form, o.ma, o.mfit, o.shape.nfac, o.ncoef, k->P,
-                                                                  k->dsph_smem, 0, true).bytes,
-                                k->smem);
-        // (the packed kernel's static shared memory may leave no room)
-        if (psg::set_pack_pair_smem(k->pair_smem) != 0) {
-            cudaGetLastError();
-            k->pair_smem = 0;
-        }
+    if (pl.pair_smem > 0 && psg::kPairFits * (slot_bytes(true) + fixed) <= room) {
+        k->pair_smem = std::max(psg::kPairFits * slot_bytes(true), floor_tc);
+        e = psg::set_pack_pair_smem(k->pair_smem);
+        if (e != 0) return pack_fail(k.get(), static_cast<cudaError_t>(e), "cudaFuncSetAttribute");
     }
     const int fit_slots = k->slots * (k->pair_smem > 0 ? psg::kPairFits : 1);
     PSG_PACK_CUDA(k.get(), cudaMalloc(&k->d_scratch, k->scratch_stride * fit_slots * sizeof(double)));
