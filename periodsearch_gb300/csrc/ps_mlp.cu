@@ -552,11 +552,11 @@ int mlp_train(float *h_P, const float *h_x, const float *h_y, int n, int epochs,
     if (e != cudaSuccess) return static_cast<int>(e);
     DevMem d;
     e = cudaMalloc(&d.p, (nx + n + 3 * kMlpFloats + act_floats(B) + total) * sizeof(float) +
-                             2 * static_cast<size_t>(n) * sizeof(int) + total * sizeof(float2) + 20 * 256);
+                             static_cast<size_t>(n) * sizeof(int) + total * sizeof(float2) + 20 * 256);
     if (e != cudaSuccess) return static_cast<int>(e);
     float *dx = d.take<float>(nx), *dy = d.take<float>(n), *dP = d.take<float>(kMlpFloats),
           *dm = d.take<float>(kMlpFloats), *dv = d.take<float>(kMlpFloats), *dl = d.take<float>(total);
-    int *didx[2] = {d.take<int>(n), d.take<int>(n)};
+    int *di = d.take<int>(n);
     float2 *dcc = d.take<float2>(total);
     const Acts a = take_acts(d, B);
     std::vector<float2> cc(total);
@@ -574,12 +574,11 @@ int mlp_train(float *h_P, const float *h_x, const float *h_y, int n, int epochs,
     std::mt19937_64 rng(seed);
     std::vector<int> perm(n);
     std::iota(perm.begin(), perm.end(), 0);
-    // The next epoch's order is shuffled and copied (into the other buffer,
-    // which the epoch before has finished with) while an epoch runs.
+    // The next epoch's order is shuffled while an epoch runs; its copy, in the
+    // same stream, follows that epoch.
     for (int ep = 0; ep < epochs && e == cudaSuccess; ep++) {
         std::shuffle(perm.begin(), perm.end(), rng);
-        int *di = didx[ep & 1];
-        e = cudaMemcpyAsync(di, perm.data(), n * sizeof(int), cudaMemcpyHostToDevice, nullptr);
+        e = cudaMemcpy(di, perm.data(), n * sizeof(int), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) break;
         const size_t at = static_cast<size_t>(ep) * steps;
         e = cudaLaunchKernelEx(&lc, train_kernel_of, static_cast<const float *>(dx), static_cast<const float *>(dy),
