@@ -110,7 +110,7 @@ PSG_HD inline bool basis_on_tensor(int mode) { return mode == kBasisTensor || mo
 
 struct SlotLayout {
     int form, ma, mfit, nfac, ncoef, P, wcols, dsph_smem;
-    size_t cg, atry, beta, da, alpha, covar, area, gv, areaR, gvR, W, J, pt, ym, red, dave, col, misc, ipiv, dsph;
+    size_t cg, atry, beta, da, alpha, covar, area, gv, areaR, gvR, W, J, pt, ym, red, dave, col, misc, dsph;
     size_t bhi, blo, tcm;   // tensor-core operand tiles (TF32 high/low parts) and barrier/TMEM slot
     size_t pt2;             // second point set-up buffer (tensor-core path: next tile's set-up)
     size_t fac, fpart;      // tensor-core path: facet normals and per-evaluation areas, facet-sum partials
@@ -232,7 +232,6 @@ PSG_HD inline SlotLayout make_layout(int form, int ma, int mfit, int nfac, int n
     const size_t tiles_end = o, work = gj_doubles(mfit) * d + gj_ints(mfit) * sizeof(int);
     L.dave = take(ma * d);
     L.col = tiles_end - L.W >= work ? L.W : take(work);
-    L.ipiv = L.col + gj_doubles(mfit) * d;
     L.misc = take(kMisc * d);
     L.dsph = dsph_smem == kBasisSmem ? take(static_cast<size_t>(nfac) * ncoef * sizeof(float)) : 0;
     if (basis_on_tensor(dsph_smem)) {

@@ -84,7 +84,6 @@ struct Smem {
     float *davef; // mixed form: FP32 copy of a relative lightcurve's derivative sums
     R *bmat;      // [27] rotation matrix and its beta/lambda derivatives, [27..29] phase
                   // function a, d, k, [30] Lommel-Seeliger and [31] Lambert weight
-    int *ipiv;
     float *dsph;  // FP32 basis in shared memory (mixed form), or nullptr
     // tensor-core contraction: operand tiles, MMA-completion barrier, Tensor
     // Memory address slot and the abort flag set when a wait gives up
@@ -131,7 +130,6 @@ __device__ inline Smem<FORM> carve(char *base, const SlotLayout &L)
     s.dave = reinterpret_cast<double *>(base + L.dave);
     s.col = reinterpret_cast<double *>(base + L.col);
     s.misc = reinterpret_cast<double *>(base + L.misc);
-    s.ipiv = reinterpret_cast<int *>(base + L.ipiv);
     s.nlit = L.form == PS_FORM_FP64 ? reinterpret_cast<int *>(base + L.lit) : nullptr;
     s.lidx = L.form == PS_FORM_FP64 ? reinterpret_cast<uint16_t *>(base + L.lit + 4 * static_cast<size_t>(L.P))
                                      : nullptr;
@@ -2912,12 +2910,13 @@ __device__ void chi2_mixed(const DevObject &ob, const FitConfig &cfg, const Slot
 // the last element in row-major order (the reference's >=).  The bits of |a|
 // order as its values do (NaN patterns, above +inf's, skipped as v >= 0 skips
 // them), so the search compares 64-bit integers, off the FP64 unit.
-// wd, wi: gj_doubles(n) doubles and gj_ints(n) ints of workspace.
+// wd: gj_doubles(n) doubles and then gj_ints(n) ints of workspace.
 // Measured (n = 55, 980 points): ten fits on 4-CTA clusters 68.8 -> 62.8 ms, 400
 // fits on one CTA each 548 -> 523 ms.
 template <int NT>
-__device__ int gauss_jordan(double *A, double *b, int n, double *wd, int *wi)
+__device__ int gauss_jordan(double *A, double *b, int n, double *wd)
 {
+    int *wi = reinterpret_cast<int *>(wd + gj_doubles(n));
     constexpr int NW = NT / 32;
     constexpr long long kInfBits = 0x7ff0000000000000LL;
     const int tid = team_thread<NT>(), lane = tid & 31, warp = tid >> 5;
@@ -3461,7 +3460,7 @@ __device__ __forceinline__ void run_fit(const DevObject &ob, const FitConfig &cf
         team_sync<NT>();
         int err;
         if constexpr (FORM == PS_FORM_FP64) {
-            err = gauss_jordan<NT>(s.covar, s.da, mf, s.col, s.ipiv);
+            err = gauss_jordan<NT>(s.covar, s.da, mf, s.col);
         } else {
             // The damped normal matrix is symmetric positive definite: solve
             // it by Cholesky in FP64; if a pivot is not positive (rounding on
@@ -3474,7 +3473,7 @@ __device__ __forceinline__ void run_fit(const DevObject &ob, const FitConfig &cf
                 }
                 for (int j = tid; j < mf; j += NT) s.da[j] = s.beta[j];
                 team_sync<NT>();
-                err = gauss_jordan<NT>(s.covar, s.da, mf, s.col, s.ipiv);
+                err = gauss_jordan<NT>(s.covar, s.da, mf, s.col);
             }
         }
         team_sync<NT>();

@@ -24,7 +24,7 @@ int main(int, char **v)
     for (int k = 0; k < 6; k++) a[k] = std::atoi(v[k + 1]);
     const int C = (a[1] + 1) * (a[1] + 1);
     const psg::SlotLayout L = psg::make_layout(a[0], C + 8, C + 6, 8 * a[2] * a[2], C, a[3], a[4], a[5]);
-    std::printf("%zu %zu %zu %zu %zu %zu %d\\n", L.bytes, L.col, L.ipiv + sizeof(int) * psg::gj_ints(C + 6), L.W, L.dave,
+    std::printf("%zu %zu %zu %zu %zu %zu %d\\n", L.bytes, L.col, L.col + sizeof(double) * psg::gj_doubles(C + 6) + sizeof(int) * psg::gj_ints(C + 6), L.W, L.dave,
                 L.phase, L.phase_tiles);
 }
 """
