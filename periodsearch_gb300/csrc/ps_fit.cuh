@@ -336,10 +336,9 @@ __device__ inline double fold_pair(double a, double c, int ia, int ic, int m, in
 }
 
 // Sums nine FP64 values over the warp and stores sum k at out[k] (the last at
-// out8): every
-// level pairs the same lanes as warp_sum, so each sum is warp_sum's bit for
-// bit, in 12 shuffles and 12 additions instead of 45.  Each sum ends in the
-// lanes that kept it; they store it (the same value).
+// out8): every level pairs the same lanes as warp_sum, so each sum is
+// warp_sum's bit for bit, in 12 shuffles and 12 additions instead of 45.  Each
+// sum ends in the lanes that kept it; they store it (the same value).
 __device__ inline void warp_sum9(const double (&v)[9], double *out, double *out8, int lane)
 {
     double w[5];
@@ -388,8 +387,8 @@ __device__ inline int list_lit_fp64(const DevObject &ob, double e1, double e2, d
     int n = 0;
     // Three rounds of 32 facets at a time, their loads ahead of the ballots
     // (one by one, the loads' latency made the list 5.6 of a point's 22 kcycles
-    // in the chi^2 pass; ten periods in FP64 38.8 -> 37.5 ms, 400 fits 515 ->
-    // 475 ms).
+    // in the chi^2 pass; one period's ten FP64 fits 38.8 -> 37.5 ms, 400 fits 515
+    // -> 475 ms).
     constexpr int kRounds = 3;
     for (int i0 = 0; i0 < F; i0 += 32 * kRounds) {
         float nxf[kRounds], nyf[kRounds], nzf[kRounds];
@@ -476,30 +475,31 @@ __device__ inline void facet_point_fp64(const DevObject &ob, Smem<PS_FORM_FP64> 
 // Accumulates the rows J[0..np) (model values in ym) of one tile into the
 // normal matrix M (lower triangle), bv and chi^2 (mrqcof.c:106-136) on the
 // SIMT pipes of the mixed form: FP32 partial sums, every element over the
-// points in data order, added to the FP64 totals every few tiles.  A warp takes units of 4 rows by 32 columns of the matrix (a
-// lane one column, four rows from one 16-byte broadcast of the weighted
-// rows): two loads for four products, where an element per thread takes two
-// each and waits for shared memory.  Unit u is unit u of the list of row
-// groups' column panels (alpha_unit); warp w takes w, w + 16, ...
-// Measured (87 free parameters): an evaluation's accumulation of 33 tiles 566 -> 280
-// kcycles, 1010 fits 165 -> 148 ms.
+// points in data order, added to the FP64 totals every few tiles.  A warp
+// takes units of 4 rows by 32 columns of the matrix (a lane one column, four
+// rows from one 16-byte broadcast of the weighted rows): two loads for four
+// products, where an element per thread takes two each and waits for shared
+// memory.  Unit u is unit u of the list of row groups' column panels
+// (alpha_unit); warp w takes w, w + 16, ...
+// Measured (87 free parameters): an evaluation's accumulation of 33 tiles 566
+// -> 280 kcycles, 1010 fits 165 -> 148 ms.
+constexpr int kTilesPerFlush = 8;
 // The tensor-core path's FP32 alpha accumulator in Tensor Memory (products
 // of TF32 high/low parts) is added to the FP64 normal matrix every 16 tiles.
 constexpr int kTcTilesPerFlush = 16;
 
-constexpr int kTilesPerFlush = 8;
 // Units of a warp by kernel variant: at most 45 units (90 free parameters), or
 // 80 with up to 128 coefficients (KU 2).
 template <int KU>
 constexpr int kAlphaUnits = KU == 2 ? 5 : 3;
-// The wide tensor-core path keeps its partial sums in registers.  The SIMT
-// contraction needs those for its loads in flight: there the loops over the
-// units are not unrolled, which puts the sums in local memory (80 bytes a
-// thread, read and written once a tile).  Held in registers through the
-// contraction they made it wait for its loads: 304 fits of 20 steps (980
-// points, 512 facets, 81 coefficients) 168.6 ms, against 134.9 so.
+// The SIMT contraction of one coefficient per lane (KU 1) needs the registers
+// of the partial sums for its loads in flight: there the loops over the units
+// are not unrolled, which puts the sums in local memory (48 bytes a thread,
+// read and written once a tile; 304 fits of 20 steps with 16 coefficients 22.0
+// -> 21.0 ms).  With two per lane the contraction is a call, which saves them anyhow, and the
+// packed kernel is slower without the unrolling (28.2 against 21.9 ms).
 template <int KU>
-constexpr int kAlphaUnroll = KU == 3 ? kAlphaUnits<KU> : 1;
+constexpr int kAlphaUnroll = KU == 1 ? 1 : kAlphaUnits<KU>;
 
 // Unit u: its first row (a group of four rows has the panels of 32 columns
 // that reach its last row's diagonal) and, in the upper half, its first
@@ -619,12 +619,13 @@ __device__ inline float load_basis(const float *d, int idx)
 // W is read four facets at a time (float4 broadcast), Dsph one coalesced row
 // per facet.  Bound by the latency of those loads, so by what the compiler
 // keeps in flight: a function of its own (contract_mixed_call) has all
-// registers for it.  304 fits of 20 steps with 81 coefficients and 512 facets
-// 134.9 -> 84.8 ms, with 49 coefficients and 288 facets 35.8 -> 30.1; one
-// coefficient per lane with the basis in L2 is better inlined (49 coefficients,
-// 648 facets: 72.0 ms, 119 as a call).  Unrolled by four facet groups with the
-// basis in shared memory, by two else (four: 91.5 ms in the first case, none
-// 95.3).
+// registers for it, also those of the partial sums of the normal matrix, which
+// inlined it shares them with.  304 fits of 20 steps with 81 coefficients and
+// 512 facets 168.3 -> 90.4 ms, with 49 coefficients and 288 facets 36.4 -> 29.9;
+// one coefficient per lane with the basis in L2 is better inlined (49
+// coefficients, 648 facets: 72.0 ms, 119 as a call).  Unrolled by four facet
+// groups with the basis in shared memory, by two else (81 coefficients: four
+// 91.5 ms, none 95.3, two 86.6).
 template <int NT, int KU, bool SMEM_D>
 __device__ __forceinline__ void contract_mixed(const float *Wf, const float *pt, float *J, const float *dsph, int np,
                                                int F, int C, int ma, int wcols, bool conv)
@@ -853,7 +854,7 @@ __device__ inline void setup_row_fp64(const DevObject &ob, int q, int part, int 
 
 // The part of the FP64 form's set-up that the model value needs: the rotated
 // Earth and Sun directions into e[0..5] and the phase function (returned),
-// by setup_point's operations.
+// by the operations of setup_phase_fp64 and setup_row_fp64.
 __device__ inline double setup_point_light(const DevObject &ob, const FitConfig &cfg, int q, double omg,
                                            const double *bm, double (&e)[6])
 {
