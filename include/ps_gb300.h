@@ -160,13 +160,15 @@ typedef struct ps_timing {
     double kernel_ms;      /* fit kernel(s) */
     double total_ms;       /* kernels + result copy */
     int64_t fits;          /* fits computed */
-    int64_t evals;         /* model evaluations (mrqcof calls) */
+    int64_t evals;         /* evaluations of the model's chi^2: LM steps plus one per fit (the reference's
+                              mrqcof calls; the engine forms the derivatives for accepted steps only) */
     int32_t launches;      /* kernel launches */
     int32_t cluster_size;  /* CTAs per fit of the last launch: 1, or 2..16 when FP64 fits were each spread over a
                               thread-block cluster (fewer fits than fit slots; bit-identical results) */
-    int64_t lit_facets;    /* FP64 form: (point, facet) pairs on the lit side over all evaluations, the work of
-                              the facet law and of the shape contraction (bright.c runs both on lit facets
-                              only); 0 for the mixed form, whose tensor-core contraction is dense */
+    int64_t lit_facets;    /* FP64 form: (point, facet) pairs on the lit side over these evaluations, each counted
+                              once: the work of the reference's facet law and shape contraction (bright.c
+                              runs both on lit facets only; the engine runs the contraction for accepted steps,
+                              with the law once more); 0 for the mixed form, whose contraction is dense */
 } ps_timing;
 
 typedef struct ps_ctx ps_ctx;
@@ -268,7 +270,7 @@ typedef struct ps_learned_stats {
     int64_t fits_completed;    /* run to the end in the mixed form, resumed from their screening
                                   state (stages 2 and 3) */
     int64_t fits_refit;        /* refitted in full in the FP64 form (stage 4) */
-    int64_t evals;             /* model evaluations of all stages */
+    int64_t evals;             /* model evaluations of all stages (as ps_timing.evals) */
     double screen_ms, complete_ms, refit_ms;   /* kernel time of the stages */
     int64_t best_index;        /* period index of the best row */
     int64_t region_periods;    /* periods whose fits were completed (stages 2 and 3) */
@@ -327,8 +329,9 @@ typedef struct ps_learned_opts {
                                  best row after the completion, */
     int32_t refit_halfwidth;  /* and refit_halfwidth periods on each side of the best */
     int32_t fill_refit_waves; /* 1: top every FP64 refit launch up with the next-lowest rows (whole
-                                 periods) until its last wave of fit slots is full -- no extra time, fewer
-                                 refit rounds (ps_scan_refined always does); 0: refit exactly the set */
+                                 periods) until its last wave is full (a wave of few fits is a quarter or
+                                 half of the slots: a longer launch than the set alone) -- fewer refit
+                                 rounds (ps_scan_refined always does); 0: refit exactly the set */
 } ps_learned_opts;
 
 /* Period scan with the learned early stop, a cascade in which only the fits

@@ -276,10 +276,11 @@ int64_t tiles_of(const ps_ctx *c, int P)
 // fit a cluster that is resident at once.  A cluster lies within one GPC, so
 // there are fewer than slots / cs of the larger ones (36 of 4, 13 of 10, 7 of
 // 16 CTAs on 152 SMs), and a second round of fits costs more than a larger
-// cluster gains.  Measured on 980 points, 288 facets (32 tiles), one launch in ms
-// by CTAs per fit: 175 (1), 105 (2), 76 (3), 62 (4), 54 (5), 49 (6), 39 (9 and
-// 10), 35 (12), 31 (16); 200 points (7 tiles): 40 (1), 27 (2), 20 (4), 17 (6),
-// 16 (7).
+// cluster gains.  (The slots' 2 and 4 are kept without asking: 37 and 38 fits
+// on 152 slots run a second round on clusters of 4.)  Measured on 980 points,
+// 288 facets (32 tiles), one launch in ms by CTAs per fit: 157 (1), 91 (2), 67
+// (3), 54 (4), 48 (5), 44 (6), 35 (9 and 10), 32 (12), 28 (16); 200 points (7
+// tiles): 37 (1), 25 (2), 20 (3), 19 (4), 16 (6), 15 (7).
 int split_size(ps_ctx *c, const psg::FitWork &w, int form)
 {
     if (form != PS_FORM_FP64 || w.traj || w.state || w.iter_limit > 0 || w.nfits < 1) return 1;
@@ -477,11 +478,13 @@ struct ScanFits {
 // rel (relative) of the best row or within halfwidth periods of it, and
 // repeats with the new rows until the set is closed: the best row and its
 // neighbourhood then carry FP64 values, and no row outside the set comes
-// within rel of it.  A refit launch takes one FP64 fit's time whether it
-// fills the device's fit slots or not, so each launch is topped up with the
-// next-lowest rows (whole periods) until its last wave of slots is full:
-// periods that a later round would likely have needed come at no extra
-// time, and fewer rounds run.
+// within rel of it.  Each launch is topped up with the next-lowest rows
+// (whole periods) until its last wave is full: periods that a later round
+// would likely have needed, for less than that round would take.  Between
+// half of the slots and all of them, and in further waves, the added fits
+// take no time at all; a smaller launch gives up larger clusters for them (10
+// fits 35 ms, the 30 that they are topped up to 54, of 980 points; see
+// split_size).
 ps_status refit_minimum(ps_ctx *c, double conw_r, ScanFits &sf, double rel, int32_t halfwidth, bool fill,
                         double *ms, int64_t *nrefit, int64_t *evals, int32_t *rounds, int64_t *lit)
 {
@@ -508,9 +511,9 @@ ps_status refit_minimum(ps_ctx *c, double conw_r, ScanFits &sf, double rel, int3
             picked[static_cast<size_t>(n)] = 1;
         }
         if (per.empty()) return PS_OK;
-        // top up the last wave with the lowest remaining rows; a set that
-        // leaves half (a quarter) of the slots free runs its fits over 2 (4)
-        // CTAs each, so its wave holds slots / 2 (slots / 4) fits
+        // top up the last wave with the lowest remaining rows; the wave of a
+        // set that leaves half (a quarter) of the slots free is slots / 2
+        // (slots / 4) fits, over at least 2 (4) CTAs each
         const int64_t need = static_cast<int64_t>(per.size()) * PS_N_POLES;
         const int64_t wave = need * 4 <= slots ? slots / 4 : need * 2 <= slots ? slots / 2 : slots;
         const int64_t cap = (need + wave - 1) / wave * wave;
