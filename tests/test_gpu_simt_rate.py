@@ -1,7 +1,7 @@
 """The mixed form off the tensor cores (more than 64 coefficients, basis in
 L2): its shape contraction, which takes most of such a fit, at no less than 5 %
-of the device's FP32 rate over the whole launch (4 % with the partial sums of
-the normal matrix held in registers through it, 8 % without)."""
+of the device's FP32 rate over the whole launch (4 % inlined, sharing its
+registers with the partial sums of the normal matrix, 7.5 % as a function)."""
 from __future__ import annotations
 
 import ctypes as C
